@@ -140,33 +140,32 @@ cudaError_t copy2d(double* dst, size_t dpitch, const double* src, size_t spitch,
   return cudaMemcpy2DAsync(dst, dpitch * 8, src, spitch * 8, width * 8, rows, kind, s);
 }
 
-// a taumol hand-over buffer of at least `bytes` (grown on demand)
-int ensure_buffer(gb_lw_context* ctx, float** buf, size_t* have, size_t bytes) {
-  if (*buf && *have >= bytes) return 0;
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
+// a gas-optics hand-over buffer of about `bytes` (grown on demand).  A buffer of
+// at least `least` bytes also does, with more passes per call: it is kept
+// under stream capture, where nothing can be allocated, and taken in place of
+// a larger one that does not fit on the device.
+int ensure_buffer(gb_lw_context* ctx, float** buf, size_t* have, size_t bytes, size_t least, cudaStream_t stream) {
+  if (*buf && (*have >= bytes || (*have >= least && capturing(stream)))) return 0;
   cudaFree(*buf);
   *buf = nullptr;
   *have = 0;
-  if (cudaMalloc(buf, bytes) != cudaSuccess) {
+  for (size_t n = bytes;; n = std::max(n / 2, least)) {
+    if (cudaMalloc(buf, n) == cudaSuccess) {
+      *have = n;
+      return 0;
+    }
     cudaGetLastError();
     *buf = nullptr;
-    ctx->last_error = "device allocation of the gas-optics hand-over planes failed";
-    return GB_LW_E_NOMEM;
+    if (n <= least) break;
   }
-  *have = bytes;
-  return 0;
+  ctx->last_error = "device allocation of the gas-optics hand-over planes failed";
+  return GB_LW_E_NOMEM;
 }
-
-// points a descriptor at a hand-over buffer of `bytes` (slots of nsmax layers)
-void attach_gas(LwBatch& b, float* buf, size_t bytes) {
-  b.gstride = (long long)b.nsmax * GB_NGPT;
-  b.gslots = (long long)(bytes / (3 * sizeof(float) * (size_t)b.gstride));
-  b.gtau = buf;
-  b.gfrac = buf + (size_t)b.gslots * b.gstride;
-  b.gcld = buf + (size_t)2 * b.gslots * b.gstride;
-}
-
-// hand-over bytes a batch of `ncols` columns at `nlay` layers is solved with
-size_t gas_need(int nlay, long long ncols) { return gb_lw_gas_bytes(nlay, gb_lw_gas_slots(nlay, ncols)); }
 
 bool flags_ok(int idrv, int inflglw, int iceflglw, int liqflglw) {
   return (idrv == 0 || idrv == 1) && inflglw >= 0 && inflglw <= 2 && iceflglw >= 0 && iceflglw <= 3 &&
@@ -227,9 +226,10 @@ int launch_one(gb_lw_context* ctx, const LwArgs& a, int k, cudaStream_t stream) 
   b.col0[0] = 0;
   b.col0[1] = a.ncol;
   b.g[0] = a;
-  int rc = ensure_buffer(ctx, &ctx->d_gas[k], &ctx->gas_bytes[k], gas_need(a.nlay, a.ncol));
+  int rc = ensure_buffer(ctx, &ctx->d_gas[k], &ctx->gas_bytes[k], gb_lw_gas_bytes(a.nlay, a.ncol, false),
+                         gb_lw_gas_min_bytes(a.nlay), stream);
   if (rc) return rc;
-  attach_gas(b, ctx->d_gas[k], ctx->gas_bytes[k]);
+  gb_lw_attach_gas(b, ctx->d_gas[k], ctx->gas_bytes[k]);
   const gb_lw_tuning t = tuning_for(ctx, a.nlay, batch_kind(b));
   cudaError_t e = gb_lw_launch_batch(b, ctx->d_tables, t.variant, t.blocks, stream);
   return e == cudaSuccess ? GB_LW_OK : gb_ctx_fail(ctx, e, "column kernels");
@@ -328,10 +328,12 @@ int gb_ctx_make_batch(gb_lw_context* ctx, int ngrid, const gb_lw_grid* grids, do
 }
 
 // hand-over planes for a descriptor's columns from the context's batch buffer
-static int attach_batch_gas(gb_lw_context* ctx, LwBatch& b) {
-  int rc = ensure_buffer(ctx, &ctx->d_bgas, &ctx->bgas_bytes, gas_need(b.nsmax, b.col0[b.ngrid]));
+static int attach_batch_gas(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
+  int rc = ensure_buffer(ctx, &ctx->d_bgas, &ctx->bgas_bytes,
+                         gb_lw_gas_bytes(b.nsmax, b.col0[b.ngrid], batch_kind(b) & GB_LW_KIND_LEARNED),
+                         gb_lw_gas_min_bytes(b.nsmax), stream);
   if (rc) return rc;
-  attach_gas(b, ctx->d_bgas, ctx->bgas_bytes);
+  gb_lw_attach_gas(b, ctx->d_bgas, ctx->bgas_bytes);
   return 0;
 }
 
@@ -360,7 +362,7 @@ int gb_ctx_launch_batch(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
   if (b.col0[b.ngrid] == 0) return GB_LW_OK;
   cudaSetDevice(ctx->device);
   const gb_lw_tuning t = tuning_for(ctx, b.nsmax, batch_kind(b));
-  int rc = attach_batch_gas(ctx, b);
+  int rc = attach_batch_gas(ctx, b, stream);
   if (rc) return rc;
   const size_t nd = gb_ctx_fused_draws(b);
   if (nd > ctx->fdraws_elems) {
@@ -1120,7 +1122,7 @@ int gb_rrtmg_lw_autotune(gb_lw_context* ctx, void* stream, int ngrid, const gb_l
   }
   if (cands.empty()) return GB_LW_E_ARGS;
   (void)max_blocks;
-  if ((rc = attach_batch_gas(ctx, b)) != 0) return rc;
+  if ((rc = attach_batch_gas(ctx, b, st)) != 0) return rc;
   if ((rc = attach_fall(ctx, b)) != 0) return rc;
   // the fused-cloud draws are made once: every candidate times the column kernel alone
   const size_t nd = gb_ctx_fused_draws(b);
@@ -1196,13 +1198,14 @@ int gb_rrtmg_lw_batch_graph_create(gb_lw_context* ctx, int ngrid, const gb_lw_gr
   const gb_lw_tuning t = tuning_for(ctx, b.nsmax, batch_kind(b));
   gb_lw_graph* g = new gb_lw_graph();
   g->ctx = ctx;
-  const size_t gbytes = gas_need(b.nsmax, b.col0[ngrid]);
-  if (cudaMalloc(&g->gas, gbytes) != cudaSuccess) {
-    cudaGetLastError();
+  size_t gbytes = 0;
+  if ((rc = ensure_buffer(ctx, &g->gas, &gbytes,
+                          gb_lw_gas_bytes(b.nsmax, b.col0[ngrid], batch_kind(b) & GB_LW_KIND_LEARNED),
+                          gb_lw_gas_min_bytes(b.nsmax), nullptr)) != 0) {
     delete g;
-    return GB_LW_E_NOMEM;
+    return rc;
   }
-  attach_gas(b, g->gas, gbytes);
+  gb_lw_attach_gas(b, g->gas, gbytes);
   const size_t nd = gb_ctx_fused_draws(b);
   if (nd && cudaMalloc(&g->draws, nd * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();

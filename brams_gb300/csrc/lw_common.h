@@ -10,15 +10,22 @@
 #define GB_NG_LIST {10, 12, 16, 14, 16, 8, 12, 8, 12, 6, 8, 8, 4, 2, 2, 2}
 #define GB_NGS0_LIST {0, 10, 22, 38, 52, 68, 76, 88, 96, 108, 114, 122, 130, 134, 136, 138}
 
+// floats of one row of a band's tables: its g-points rounded up to whole
+// 16-byte vectors (two g-points stay two floats)
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int gb_pitch(int ng) { return ng <= 2 ? ng : (ng + 3) / 4 * 4; }
+
 // Offsets (in floats) of every band table inside the device table blob.
-// Layouts are g-fastest so that lanes holding consecutive g-points of one
-// band read consecutive words:
-//   ka  [65*nspa rows][ng]     (row = the reference's absa first index)
-//   kb  [235*max(nspb,1) rows][ng]
-//   sr  [10][ng]  fo [4][ng]
-//   fa  [neta_a + 1][ng], fb [neta_b + 1][ng]   (one padding row)
-//   m*  minor tables [19][neta][ng] (neta = 1 for temperature-only minors)
-//   x*  per-g scalars [ng]
+// Layouts are g-fastest, rows of p = gb_pitch(ng) floats, every table on a
+// 16-byte boundary, so that a row's g-points are read by vector loads:
+//   ka  [65*nspa rows][p]     (row = the reference's absa first index)
+//   kb  [235*max(nspb,1) rows][p]
+//   sr  [10][p]  fo [4][p]
+//   fa  [neta_a + 1][p], fb [neta_b + 1][p]   (one padding row)
+//   m*  minor tables [19][neta][p] (neta = 1 for temperature-only minors)
+//   x*  per-g scalars [p]
 struct GbBandTab {
   int ng, g0;
   int ka, kb, fa, fb, sr, fo;

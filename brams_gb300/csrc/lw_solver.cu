@@ -6,13 +6,19 @@
 // t (the last warp has 12 live lanes), and persistent blocks walk the columns
 // of a batch of grids.  Nothing per cell goes to global scratch:
 //
-//   taumol (gas_column) -- setcoef (rrtmg_lw_setcoef.f90:275-430) with one
-//     thread per layer, then band by band a prologue per layer builds the
-//     layer's term list (lw_gasoptics.cuh) and one thread per (layer, g) cell
-//     gathers taug = sum w * table[row + g] and interpolates the Planck
-//     fraction.  taug (without aerosol) and the fractions go to fp32 planes in
-//     a slot owned by the block, which stays in L2 until the transfer of the
-//     same column reads it.
+//   taumol -- of a batch, by kernels of its own (lw_taumol.cu), into a plane
+//     per column that the transfer reads; the batch goes through in passes of
+//     as many columns as the planes hold.  It was part of the column's block
+//     before (setcoef by 45 of 160 threads, two barriers per band, a shared-
+//     memory read and a 4-byte gather per multiply-add) and took 42% of its
+//     time: 24.1 ms for 108,000 columns of 45 layers with caller sub-columns,
+//     17.0 ms since, and 17.9 to 8.3 ms for 67,909 columns with in-kernel
+//     clouds.  The in-block form (gas_column) is still the way where a block
+//     finds its columns on the device only (lw_list_kernel), and for single
+//     outputs per (layer, g-point) (lw_gas_kernel): setcoef
+//     with one thread per layer, then band by band a prologue per layer builds
+//     the layer's term list (lw_gasoptics.cuh) and one thread per (layer, g)
+//     cell gathers taug = sum w * table[row + g].
 //
 //   transfer (rt_column) -- inatm's column amounts, the laytrop and value
 //     checks, Planck interpolation per (layer, band) and the surface source,
@@ -31,11 +37,11 @@
 //     are added error-free (two-sum) into fp64, and the net fluxes and heating
 //     rates heatfac*dF/dp are fp64 (rtrnmc.f90:566-592).
 //
-// Kernels: lw_full_kernel (taumol then the transfer; for batches without a
-// network, and for the columns a network batch hands over), lw_rt_kernel (the
-// transfer on the network's fp16 taug and Planck fractions; columns with a
-// layer off the network are handed over), lw_gas_kernel (taumol alone, for
-// the network's training samples and the gas-optics diagnostics).
+// Kernels: lw_rt_kernel (the transfer, on taumol's planes or on the network's
+// fp16 taug and Planck fractions; there, columns with a layer off the network
+// are handed over), lw_list_kernel (taumol and the transfer of the columns
+// handed over), lw_gas_kernel (taumol alone, for the network's training
+// samples and the gas-optics diagnostics).
 //
 // Precision: gas optics and transfer in fp32, flux sums across warps
 // error-free into fp64, net fluxes and the heating-rate step in fp64.
@@ -72,18 +78,6 @@ __constant__ float c_a2[16] = {0.f, -12.0f, -11.7f, 0.f, -0.72f, -0.243f, 0.19f,
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
 // ------------------------------------------------------------------ helpers
-__device__ __forceinline__ double in2(const double* __restrict__ a, long long ld, long long icol, int k) {
-  return __ldg(a + icol + ld * k);
-}
-
-// setcoef's regime switch (plog <= 4.56 is the upper atmosphere,
-// rrtmg_lw_setcoef.f90:312), decided in fp64 near the switch
-__device__ __forceinline__ bool lower_atmosphere(double pd, float plog) {
-  bool lower = plog > 4.56f;
-  if (fabsf(plog - 4.56f) < 1.0e-4f) lower = log(pd) > 4.56;
-  return lower;
-}
-
 // Warp sums of two values per lane at once: lane i returns the sum over the
 // 32 lanes of v(i & 1) (one exchange, then four xor steps).
 __device__ __forceinline__ float reduce2(float v0, float v1, int lane) {
@@ -209,13 +203,11 @@ struct GasSmem {
   int* iv;         // [NI][nl]
   float2* terms;   // [TGROUP][nl] gas-optics terms of the current band, term-major
   FracRec* frec;   // [nl] Planck-fraction records of the current band
-  double* d;       // [ND][nl] fp64 column amounts of the binary species
   int* iscal;      // [4]: laytrop
 };
 
 __host__ __device__ inline size_t gas_smem_bytes(int nl) {
-  return align16((size_t)(NF + NI) * nl * 4) + align16((size_t)nl * TGROUP * 8) + align16((size_t)nl * sizeof(FracRec)) +
-         align16((size_t)ND * nl * 8) + 16;
+  return align16((size_t)(NF + NI) * nl * 4) + align16((size_t)nl * TGROUP * 8) + align16((size_t)nl * sizeof(FracRec)) + 16;
 }
 
 __device__ inline GasSmem gas_carve(char* p, int nl) {
@@ -227,8 +219,6 @@ __device__ inline GasSmem gas_carve(char* p, int nl) {
   p += align16((size_t)nl * TGROUP * 8);
   s.frec = (FracRec*)p;
   p += align16((size_t)nl * sizeof(FracRec));
-  s.d = (double*)p;
-  p += align16((size_t)ND * nl * 8);
   s.iscal = (int*)p;
   return s;
 }
@@ -236,10 +226,11 @@ __device__ inline GasSmem gas_carve(char* p, int nl) {
 // Prologue of band b for one layer: the band-specific per-layer code
 // (lw_gasoptics.cuh) writing the layer's terms and Planck-fraction record.
 template <int b>
-__device__ __forceinline__ void band_prologue(const GasSmem& s, int nl, int lay, bool lower, const float* T) {
-  Cell c{s.f, s.iv, nl, lay, T, s.d};
+__device__ __forceinline__ void band_prologue(const GasSmem& s, int nl, int lay, bool lower, const float* T,
+                                              const LwArgs& a, long long icol) {
+  Cell c{s.f, s.iv, nl, lay, T, &a, icol};
   Terms t{s.terms + lay, nl, 0};
-  FracRec r = prologue<b>(c, lower, t);
+  FracRec r = Band<b>::prologue(c, lower, t);
   t.pad(maxt(b), c_T.band[b - 1].sr);
   s.frec[lay] = r;
 }
@@ -249,11 +240,11 @@ __device__ __forceinline__ void band_prologue(const GasSmem& s, int nl, int lay,
 // (the band's term count and g-points are compile-time constants, so the
 // gather loop is unrolled) and interpolating the Planck fraction.  Ends with
 // a barrier.
-template <int b, int NT>
-__device__ __forceinline__ void gas_band(const GasSmem& s, int nl, int laytrop, const float* __restrict__ T,
-                                         float* gt, float* gf) {
-  constexpr int NG = ngb_const(b), G0 = g0_const(b), M = maxt(b);
-  for (int lay = threadIdx.x; lay < nl; lay += NT) band_prologue<b>(s, nl, lay, lay < laytrop, T);
+template <int b, int NT, class Out>
+__device__ __forceinline__ void gas_band(const LwArgs& a, long long icol, const GasSmem& s, int nl, int laytrop,
+                                         const float* __restrict__ T, const Out& out) {
+  constexpr int NG = ngb_const(b), M = maxt(b);
+  for (int lay = threadIdx.x; lay < nl; lay += NT) band_prologue<b>(s, nl, lay, lay < laytrop, T, a, icol);
   __syncthreads();
   for (int cell = threadIdx.x; cell < nl * NG; cell += NT) {
     const int lay = cell / NG, gi = cell - lay * NG;
@@ -269,156 +260,45 @@ __device__ __forceinline__ void gas_band(const GasSmem& s, int nl, int laytrop, 
     const FracRec fr = s.frec[lay];
     const float* fp = T + fr.off + gi;
     const float f0 = __ldg(fp);
-    gt[lay * GB_NGPT + G0 + gi] = acc;
-    gf[lay * GB_NGPT + G0 + gi] = fmaf(fr.fpl, __ldg(fp + NG) - f0, f0);
+    out.put(b, lay, gi, acc, fmaf(fr.fpl, __ldg(fp + pitch_const(b)) - f0, f0));
   }
   __syncthreads();
 }
 
-// taumol of one column by the whole block: taug and Planck fractions of every
-// (layer, g) cell into the planes gt/gf ([nl][140] each).  Ends with a barrier.
-template <int NT>
-__device__ void gas_column(const LwArgs& a, long long icol, const GasSmem& s, float* gt, float* gf,
+// taumol of one column by the whole block: taug and Planck fraction of every
+// (layer, g) cell through out.put.  Ends with a barrier.
+template <int NT, class Out>
+__device__ void gas_column(const LwArgs& a, long long icol, const GasSmem& s, const Out& out,
                            const float* __restrict__ T) {
   const int nl = a.nlay, tid = threadIdx.x;
   if (tid == 0) s.iscal[0] = 0;
   __syncthreads();
-  // setcoef (rrtmg_lw_setcoef.f90:275-430) after inatm's column amounts
-  // (rrtmg_lw_rad.f90:807-867), one thread per layer
-  const float stpfac = 296.0f / 1013.0f;
-  const float amd = 28.9660f, amw = 18.0160f;
   for (int lay = tid; lay < nl; lay += NT) {
-    const double pd = in2(a.play, a.ld, icol, lay);
-    const float pavel = (float)pd;
-    const float tavel = (float)in2(a.tlay, a.ld, icol, lay);
-    const double dpz = in2(a.plev, a.ld, icol, lay) - in2(a.plev, a.ld, icol, lay + 1);
-    const float w1 = (float)in2(a.h2ovmr, a.ld, icol, lay);
-    const float w2 = (float)in2(a.co2vmr, a.ld, icol, lay);
-    const float w3 = (float)in2(a.o3vmr, a.ld, icol, lay);
-    const float w4 = (float)in2(a.n2ovmr, a.ld, icol, lay);
-    const float w6 = (float)in2(a.ch4vmr, a.ld, icol, lay);
-    const float w7 = (float)in2(a.o2vmr, a.ld, icol, lay);
-    const float amm = (1.0f - w1) * amd + w1 * amw;
-    const float coldry = (float)dpz * 1.e3f * (float)c_T.avogad / (1.e2f * (float)c_T.grav * amm * (1.0f + w1));
-    const float summol = w2 + w3 + w4 + 0.0f + w6 + w7;
-    const float wbrodl = coldry * (1.0f - summol);
-    const float wk1 = coldry * w1, wk2 = coldry * w2, wk3 = coldry * w3, wk4 = coldry * w4, wk6 = coldry * w6,
-                wk7 = coldry * w7;
-    float* F = s.f;
-    auto put = [&](int k, float v) { F[k * nl + lay] = v; };
-    put(F_COLDRY, coldry);
-    put(F_PAVEL, pavel);
-    put(F_WX1, coldry * (float)in2(a.ccl4vmr, a.ld, icol, lay) * 1.e-20f);
-    put(F_WX2, coldry * (float)in2(a.cfc11vmr, a.ld, icol, lay) * 1.e-20f);
-    put(F_WX3, coldry * (float)in2(a.cfc12vmr, a.ld, icol, lay) * 1.e-20f);
-    put(F_WX4, coldry * (float)in2(a.cfc22vmr, a.ld, icol, lay) * 1.e-20f);
-    const float plog = __logf(pavel);
-    const bool lower = lower_atmosphere(pd, plog);
-    // The truncations jp, jt, jt1 (setcoef.f90:276-306) are taken in fp32 and
-    // re-taken in fp64, as the reference computes them, where the fp32 value
-    // lies near an integer.
-    const double td = in2(a.tlay, a.ld, icol, lay);
-    const float xjp = 36.0f - 5.0f * (plog + 0.04f);
-    int jp = (int)xjp;
-    if (fabsf(xjp - rintf(xjp)) < 2.0e-3f) jp = (int)(36.0 - 5 * (log(pd) + 0.04));
-    jp = clampi(jp, 1, 58);
-    jp = lower ? (jp > 12 ? 12 : jp) : (jp < 13 ? 13 : jp);
-    const float fp = 5.0f * (__ldg(T + c_T.ref_preflog + jp - 1) - plog);
-    const float dt0 = (tavel - __ldg(T + c_T.ref_tref + jp - 1)) / 15.0f;
-    int jt = (int)(3.0f + dt0);
-    if (fabsf(3.0f + dt0 - rintf(3.0f + dt0)) < 1.0e-4f) jt = (int)(3.0 + (td - c_T.tref64[jp - 1]) / 15.0);
-    jt = clampi(jt, 1, 4);
-    const float ft = dt0 - (float)(jt - 3);
-    const float dt1 = (tavel - __ldg(T + c_T.ref_tref + jp)) / 15.0f;
-    int jt1 = (int)(3.0f + dt1);
-    if (fabsf(3.0f + dt1 - rintf(3.0f + dt1)) < 1.0e-4f) jt1 = (int)(3.0 + (td - c_T.tref64[jp]) / 15.0);
-    jt1 = clampi(jt1, 1, 4);
-    const float ft1 = dt1 - (float)(jt1 - 3);
-    // fp64 column amounts of the binary species (inatm :807-867, setcoef.f90:349-362)
-    {
-      const double amd64 = 28.9660, amw64 = 18.0160;
-      const double h = in2(a.h2ovmr, a.ld, icol, lay);
-      const double amm64 = (1.0 - h) * amd64 + h * amw64;
-      const double cd = dpz * 1.e3 * c_T.avogad / (1.e2 * c_T.grav * amm64 * (1.0 + h));
-      auto col = [&](const double* v) {
-        const double x = 1.e-20 * (cd * in2(v, a.ld, icol, lay));
-        return x == 0.0 ? 1.e-32 * cd : x;
-      };
-      s.d[D_H2O * nl + lay] = 1.e-20 * (cd * h);
-      s.d[D_CO2 * nl + lay] = col(a.co2vmr);
-      s.d[D_O3 * nl + lay] = col(a.o3vmr);
-      s.d[D_N2O * nl + lay] = col(a.n2ovmr);
-      s.d[D_CH4 * nl + lay] = col(a.ch4vmr);
-    }
-    const float water = wk1 / coldry;
-    const float scalefac = pavel * stpfac / tavel;
-    const float forfac = scalefac / (1.0f + water);
-    float forfrac, selffrac = 0.0f;
-    int indfor, indself = 1;
-    // truncations of temperature factors, re-taken in fp64 near an integer
-    auto trunc_t = [&](float f32, double num64, double den) {
-      return fabsf(f32 - rintf(f32)) < 1.0e-4f ? (int)(num64 / den) : (int)f32;
-    };
-    if (lower) {
-      float factor = (332.0f - tavel) / 36.0f;
-      indfor = min(2, max(1, trunc_t(factor, 332.0 - td, 36.0)));
-      forfrac = factor - (float)indfor;
-      factor = (tavel - 188.0f) / 7.2f;
-      indself = min(9, max(1, trunc_t(factor, td - 188.0, 7.2) - 7));
-      selffrac = factor - (float)(indself + 7);
-    } else {
-      const float factor = (tavel - 188.0f) / 36.0f;
-      indfor = 3;
-      forfrac = factor - 1.0f;
-    }
-    const float selffac = water * forfac;
-    const float scaleminor = pavel / tavel;
-    const float scaleminorn2 = scaleminor * (wbrodl / (coldry + wk1));
-    const float factor = (tavel - 180.8f) / 7.2f;
-    const int indminor = min(18, max(1, trunc_t(factor, td - 180.8, 7.2)));
-    const float minorfrac = factor - (float)indminor;
-    const float colh2o = 1.e-20f * wk1;
-    float colco2 = 1.e-20f * wk2, colo3 = 1.e-20f * wk3, coln2o = 1.e-20f * wk4, colco = 0.0f;
-    float colch4 = 1.e-20f * wk6;
-    const float colo2 = 1.e-20f * wk7;
-    if (colco2 == 0.0f) colco2 = 1.e-32f * coldry;
-    if (colo3 == 0.0f) colo3 = 1.e-32f * coldry;
-    if (coln2o == 0.0f) coln2o = 1.e-32f * coldry;
-    if (colco == 0.0f) colco = 1.e-32f * coldry;
-    if (colch4 == 0.0f) colch4 = 1.e-32f * coldry;
-    const float compfp = 1.0f - fp;
-    put(F_FAC10, compfp * ft);
-    put(F_FAC00, compfp * (1.0f - ft));
-    put(F_FAC11, fp * ft1);
-    put(F_FAC01, fp * (1.0f - ft1));
-    put(F_COLH2O, colh2o); put(F_COLCO2, colco2); put(F_COLO3, colo3); put(F_COLN2O, coln2o);
-    put(F_COLCO, colco); put(F_COLCH4, colch4); put(F_COLO2, colo2); put(F_COLBRD, 1.e-20f * wbrodl);
-    put(F_SELFFAC, colh2o * selffac); put(F_SELFFRAC, selffrac);
-    put(F_FORFAC, colh2o * forfac); put(F_FORFRAC, forfrac);
-    put(F_MINORFRAC, minorfrac); put(F_SCALEMINOR, scaleminor); put(F_SCALEMINORN2, scaleminorn2);
+    LayerInts ix;
+    const bool lower = setcoef_layer(a, icol, lay, T, ix, [&](int k, float v) { s.f[k * nl + lay] = v; });
     int* IV = s.iv;
-    IV[I_JP * nl + lay] = jp; IV[I_JT * nl + lay] = jt; IV[I_JT1 * nl + lay] = jt1;
-    IV[I_INDSELF * nl + lay] = indself; IV[I_INDFOR * nl + lay] = indfor; IV[I_INDMINOR * nl + lay] = indminor;
+    IV[I_JP * nl + lay] = ix.jp; IV[I_JT * nl + lay] = ix.jt; IV[I_JT1 * nl + lay] = ix.jt1;
+    IV[I_INDSELF * nl + lay] = ix.indself; IV[I_INDFOR * nl + lay] = ix.indfor; IV[I_INDMINOR * nl + lay] = ix.indminor;
     if (lower) atomicAdd(&s.iscal[0], 1);  // laytrop (the transfer checks that these form a prefix)
   }
   __syncthreads();
   const int laytrop = s.iscal[0];
-  gas_band<1, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<2, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<3, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<4, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<5, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<6, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<7, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<8, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<9, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<10, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<11, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<12, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<13, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<14, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<15, NT>(s, nl, laytrop, T, gt, gf);
-  gas_band<16, NT>(s, nl, laytrop, T, gt, gf);
+  gas_band<1, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<2, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<3, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<4, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<5, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<6, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<7, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<8, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<9, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<10, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<11, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<12, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<13, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<14, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<15, NT>(a, icol, s, nl, laytrop, T, out);
+  gas_band<16, NT>(a, icol, s, nl, laytrop, T, out);
 }
 
 // ================================================================== transfer
@@ -486,8 +366,7 @@ __device__ inline RtSmem rt_carve(char* p, int nl) {
 
 // Where taug and the Planck fractions of a column come from.
 struct GasSrc {
-  const float* gt;            // fp32 planes [nl][140] (taumol), or NULL
-  const float* gf;
+  const float* plane;         // taumol's plane of the column (rows of GB_LW_PROW floats), or NULL
   float* gc;                  // caller sub-columns: the cells' cloud plane [nl][140], or NULL
   const __half* nt;           // fp16 rows [nl][140] (network), or NULL
   const __half* nf;
@@ -502,15 +381,20 @@ __device__ __forceinline__ bool layer_on_net(const GasSrc& src, int lay) {
   return src.flag[lay] != 0;
 }
 
+// g-point gi of band b (1..16) in a plane row: its taug, and its Planck fraction two floats on
+__host__ __device__ constexpr int plane_pos(int b, int gi) { return 4 * (gb_pair0(b) + gi / 2) + gi % 2; }
+
+// po: the g-point's position in a plane row
 template <int MODE>
-__device__ __forceinline__ void gas_at(const GasSrc& src, bool net, int lay, int g, float& tg, float& pf) {
-  const int o = lay * GB_NGPT + g;
+__device__ __forceinline__ void gas_at(const GasSrc& src, bool net, int lay, int g, int po, float& tg, float& pf) {
   if (MODE != RT_GAS && net) {
+    const int o = lay * GB_NGPT + g;
     tg = __half2float(__ldg(src.nt + o));
     pf = __half2float(__ldg(src.nf + o));
   } else {
-    tg = src.gt[o];  // plain loads: taumol wrote these planes in the same launch
-    pf = src.gf[o];
+    const float* p = src.plane + lay * GB_LW_PROW + po;  // plain loads: the hand-over kernel's taumol
+    tg = p[0];                                           // wrote its planes in the same launch
+    pf = p[2];
   }
 }
 
@@ -837,6 +721,7 @@ __device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, cons
   const int g = live ? tid : GB_NGPT - 1;
   const int band = __float_as_int(__ldg(T + c_T.gpt_band + g));
   const float wgt = live ? __ldg(T + c_T.gpt_wgt + g) : 0.0f;
+  const int po = plane_pos(band + 1, g - c_T.band[band].g0);
   __syncthreads();
 
   // ---------------- per layer: inatm's column amounts (pwvcm), value checks, laytrop, Planck rows
@@ -1098,12 +983,12 @@ __device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, cons
   const float* gcp = !BAND && clouds && !fused ? src.gc : nullptr;  // the cells' cloud values, if handed over
   float cvn = 0.0f;
   bool pend = false;  // a layer's weighted radiances wait in p0, p1 (the same in every lane)
-  gas_at<MODE>(src, layer_on_net<MODE>(src, nl - 1), nl - 1, g, tgn, pfn);
+  gas_at<MODE>(src, layer_on_net<MODE>(src, nl - 1), nl - 1, g, po, tgn, pfn);
   if (gcp) cvn = gcp[(nl - 1) * GB_NGPT + g];
   for (int lay = nl - 1; lay >= 0; --lay) {
     const float tg = tgn, pf = pfn, cv = cvn;
     if (lay > 0) {  // in flight meanwhile
-      gas_at<MODE>(src, layer_on_net<MODE>(src, lay - 1), lay - 1, g, tgn, pfn);
+      gas_at<MODE>(src, layer_on_net<MODE>(src, lay - 1), lay - 1, g, po, tgn, pfn);
       if (gcp) cvn = gcp[(lay - 1) * GB_NGPT + g];
     }
     const float4 r = S.L[lay].rec[band];
@@ -1187,12 +1072,12 @@ __device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, cons
   // ---------------- upward pass (rtrnmc.f90:486-529): level lay+1 above layer lay
   float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f, q3 = 0.0f;
   pend = false;  // a layer's weighted values wait in q0..q3
-  gas_at<MODE>(src, layer_on_net<MODE>(src, 0), 0, g, tgn, pfn);
+  gas_at<MODE>(src, layer_on_net<MODE>(src, 0), 0, g, po, tgn, pfn);
   if (gcp) cvn = gcp[g];
   for (int lay = 0; lay < nl; ++lay) {
     const float tg = tgn, pf = pfn, cv = cvn;
     if (lay + 1 < nl) {
-      gas_at<MODE>(src, layer_on_net<MODE>(src, lay + 1), lay + 1, g, tgn, pfn);
+      gas_at<MODE>(src, layer_on_net<MODE>(src, lay + 1), lay + 1, g, po, tgn, pfn);
       if (gcp) cvn = gcp[(lay + 1) * GB_NGPT + g];
     }
     const float4 r = S.L[lay].rec[band];
@@ -1342,7 +1227,26 @@ __device__ __forceinline__ const LwArgs& stage_args(const LwArgs& a, char* smem)
   return *reinterpret_cast<const LwArgs*>(smem);
 }
 
-// taumol over batch columns [c0, c1): column c0 + k into slot k.
+// taumol's outputs as [layer][140] planes
+struct SampleOut {
+  float *gt, *gf;
+  __device__ __forceinline__ void put(int b, int lay, int gi, float tau, float frac) const {
+    const int o = lay * GB_NGPT + g0_const(b) + gi;
+    gt[o] = tau;
+    gf[o] = frac;
+  }
+};
+// taumol's outputs as the transfer's plane of a column
+struct PlaneOut {
+  float* plane;
+  __device__ __forceinline__ void put(int b, int lay, int gi, float tau, float frac) const {
+    float* p = plane + lay * GB_LW_PROW + plane_pos(b, gi);
+    p[0] = tau;
+    p[2] = frac;
+  }
+};
+
+// taumol alone over batch columns [c0, c1): column c0 + k into slot k of gtau and gfrac.
 template <int NT>
 __global__ void __launch_bounds__(NT) lw_gas_kernel(const __grid_constant__ LwBatch B, const float* __restrict__ T,
                                                     long long c0, long long c1) {
@@ -1353,14 +1257,15 @@ __global__ void __launch_bounds__(NT) lw_gas_kernel(const __grid_constant__ LwBa
     gi = grid_of(B, i, gi);
     const LwArgs& a = stage_args(B.g[gi], smem_raw);
     const long long slot = i - c0;
-    gas_column<NT>(a, i - B.col0[gi], s, B.gtau + slot * B.gstride, B.gfrac + slot * B.gstride, T);
+    gas_column<NT>(a, i - B.col0[gi], s, SampleOut{B.gtau + slot * B.gstride, B.gfrac + slot * B.gstride}, T);
   }
 }
 
-// The transfer on the network's gas optics over batch columns [c0, c1), one
-// block per column; a column with a layer off the network is appended to
-// B.fall instead.
-template <int MINB>
+// The transfer over batch columns [c0, c1), one block per column.  RT_GAS: on
+// taumol's planes, column c0 + k in slot k (BAND: the non-McICA driver's band
+// clouds).  RT_NET: on the network's gas optics; a column with a layer off the
+// network is appended to B.fall instead.
+template <int MINB, int MODE, bool BAND>
 __global__ void __launch_bounds__(RT_NT, MINB) lw_rt_kernel(const __grid_constant__ LwBatch B,
                                                              const float* __restrict__ T, long long c0, long long c1) {
   extern __shared__ __align__(16) char smem_raw[];
@@ -1371,40 +1276,41 @@ __global__ void __launch_bounds__(RT_NT, MINB) lw_rt_kernel(const __grid_constan
     const LwArgs& a = stage_args(B.g[gi], smem_raw);
     const long long icol = i - B.col0[gi];
     GasSrc src{};
-    const long long row = icol * a.nlay * GB_NGPT;
-    src.nt = a.sur_tau ? a.sur_tau + row : nullptr;
-    src.nf = a.sur_frac ? a.sur_frac + row : nullptr;
-    src.flag = a.sur_flag ? a.sur_flag + icol * a.nlay : nullptr;
-    const bool done = rt_column<RT_NET>(a, icol, S, src, T);
-    if (!done && threadIdx.x == 0) B.fall[atomicAdd(B.nfall, 1u)] = i;
+    if (MODE == RT_GAS) {
+      src.plane = B.plane + (i - c0) * B.nsmax * GB_LW_PROW;
+      src.gc = !BAND && B.gcld ? B.gcld + (long long)blockIdx.x * B.nsmax * GB_NGPT : nullptr;
+    } else {
+      const long long row = icol * a.nlay * GB_NGPT;
+      src.nt = a.sur_tau ? a.sur_tau + row : nullptr;
+      src.nf = a.sur_frac ? a.sur_frac + row : nullptr;
+      src.flag = a.sur_flag ? a.sur_flag + icol * a.nlay : nullptr;
+    }
+    const bool done = rt_column<MODE, BAND>(a, icol, S, src, T);
+    if (MODE == RT_NET && !done && threadIdx.x == 0) B.fall[atomicAdd(B.nfall, 1u)] = i;
   }
 }
 
-// taumol and the transfer of a column in one block, taumol's planes in the
-// block's own slot (which stays in L2).  LIST: the columns handed over by the
-// network's transfer kernel (B.fall), each layer's gas optics from the
-// network or from taumol; else batch columns [c0, c1).
-template <int MINB, bool LIST>
-__global__ void __launch_bounds__(RT_NT, MINB) lw_full_kernel(const __grid_constant__ LwBatch B,
-                                                               const float* __restrict__ T, long long c0, long long c1) {
+// The columns handed over by the network's transfer kernel (B.fall): taumol
+// into the block's plane slot, then the transfer with each layer's gas optics
+// from the network or from taumol.
+template <int MINB>
+__global__ void __launch_bounds__(RT_NT, MINB) lw_list_kernel(const __grid_constant__ LwBatch B,
+                                                               const float* __restrict__ T) {
   extern __shared__ __align__(16) char smem_raw[];
   const GasSmem gs = gas_carve(smem_raw + ARGS_BYTES, B.nsmax);
   const RtSmem S = rt_carve(smem_raw + ARGS_BYTES, B.nsmax);  // used after taumol is done with the same memory
-  float* gt = B.gtau + (long long)blockIdx.x * B.gstride;
-  float* gf = B.gfrac + (long long)blockIdx.x * B.gstride;
-  const long long n = LIST ? (long long)*B.nfall : c1;
-  int gi = 0;
-  for (long long i = (LIST ? 0 : c0) + blockIdx.x; i < n; i += gridDim.x) {
-    const long long gc = LIST ? B.fall[i] : i;
-    gi = grid_of(B, gc, LIST ? 0 : gi);  // the list is in no particular order
+  float* plane = B.plane + (long long)blockIdx.x * B.nsmax * GB_LW_PROW;
+  const long long n = (long long)*B.nfall;
+  for (long long i = blockIdx.x; i < n; i += gridDim.x) {
+    const long long gc = B.fall[i];
+    const int gi = grid_of(B, gc, 0);  // the list is in no particular order
     const LwArgs& a = stage_args(B.g[gi], smem_raw);
     const long long icol = gc - B.col0[gi];
-    gas_column<RT_NT>(a, icol, gs, gt, gf, T);
+    gas_column<RT_NT>(a, icol, gs, PlaneOut{plane}, T);
     GasSrc src{};
-    src.gt = gt;
-    src.gf = gf;
-    src.gc = B.gcld ? B.gcld + (long long)blockIdx.x * B.gstride : nullptr;
-    if (LIST && a.sur_flag) {
+    src.plane = plane;
+    src.gc = B.gcld ? B.gcld + (long long)blockIdx.x * B.nsmax * GB_NGPT : nullptr;
+    if (a.sur_flag) {
       const long long row = icol * a.nlay * GB_NGPT;
       src.nt = a.sur_tau + row;
       src.nf = a.sur_frac + row;
@@ -1413,29 +1319,6 @@ __global__ void __launch_bounds__(RT_NT, MINB) lw_full_kernel(const __grid_const
     } else {
       rt_column<RT_GAS>(a, icol, S, src, T);
     }
-  }
-}
-
-// The fused taumol and transfer kernel for the non-McICA driver's band
-// clouds (batch columns [c0, c1), block k in slot k).
-template <int MINB>
-__global__ void __launch_bounds__(RT_NT, MINB) lw_band_kernel(const __grid_constant__ LwBatch B,
-                                                               const float* __restrict__ T, long long c0, long long c1) {
-  extern __shared__ __align__(16) char smem_raw[];
-  const GasSmem gs = gas_carve(smem_raw + ARGS_BYTES, B.nsmax);
-  const RtSmem S = rt_carve(smem_raw + ARGS_BYTES, B.nsmax);
-  float* gt = B.gtau + (long long)blockIdx.x * B.gstride;
-  float* gf = B.gfrac + (long long)blockIdx.x * B.gstride;
-  int gi = 0;
-  for (long long i = c0 + blockIdx.x; i < c1; i += gridDim.x) {
-    gi = grid_of(B, i, gi);
-    const LwArgs& a = stage_args(B.g[gi], smem_raw);
-    const long long icol = i - B.col0[gi];
-    gas_column<RT_NT>(a, icol, gs, gt, gf, T);
-    GasSrc src{};
-    src.gt = gt;
-    src.gf = gf;
-    rt_column<RT_GAS, true>(a, icol, S, src, T);
   }
 }
 
@@ -1459,24 +1342,17 @@ struct VariantInfo {
   cudaError_t (*launch)(const LwBatch&, const float*, long long, long long, int, size_t, cudaStream_t);
 };
 
-template <int MINB>
-cudaError_t launch_full(const LwBatch& b, const float* T, long long c0, long long c1, int nblocks, size_t smem,
-                        cudaStream_t st) {
-  gb::lw_full_kernel<MINB, false><<<nblocks, gb::RT_NT, smem, st>>>(b, T, c0, c1);
-  return cudaGetLastError();
-}
-template <int MINB>
-cudaError_t launch_net(const LwBatch& b, const float* T, long long c0, long long c1, int nblocks, size_t smem,
-                       cudaStream_t st) {
-  gb::lw_rt_kernel<MINB><<<nblocks, gb::RT_NT, smem, st>>>(b, T, c0, c1);
+template <int MINB, int MODE>
+cudaError_t launch_rt(const LwBatch& b, const float* T, long long c0, long long c1, int nblocks, size_t smem,
+                      cudaStream_t st) {
+  gb::lw_rt_kernel<MINB, MODE, false><<<nblocks, gb::RT_NT, smem, st>>>(b, T, c0, c1);
   return cudaGetLastError();
 }
 
-// batches without a network: the fused taumol + transfer kernel; with a
-// network: the transfer kernel on the network's outputs
-#define GB_LW_FULL_ENTRY(i, mb) {mb, (const void*)gb::lw_full_kernel<mb, false>, launch_full<mb>},
-#define GB_LW_NET_ENTRY(i, mb) {mb, (const void*)gb::lw_rt_kernel<mb>, launch_net<mb>},
-const VariantInfo kVariants[] = {GB_LW_VARIANTS(GB_LW_FULL_ENTRY)};
+// the transfer kernel on taumol's planes, and on the network's outputs
+#define GB_LW_GAS_ENTRY(i, mb) {mb, (const void*)gb::lw_rt_kernel<mb, gb::RT_GAS, false>, launch_rt<mb, gb::RT_GAS>},
+#define GB_LW_NET_ENTRY(i, mb) {mb, (const void*)gb::lw_rt_kernel<mb, gb::RT_NET, false>, launch_rt<mb, gb::RT_NET>},
+const VariantInfo kVariants[] = {GB_LW_VARIANTS(GB_LW_GAS_ENTRY)};
 const VariantInfo kLean[] = {GB_LW_VARIANTS(GB_LW_NET_ENTRY)};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 constexpr int kMaxPerSm = 16;  // most resident column blocks per SM any shape launches
@@ -1490,11 +1366,9 @@ int device_sms() {
   return nsm;
 }
 
-// shared memory of a block of the fused kernel (taumol or transfer area) or of the transfer kernel
-size_t block_smem(int nlay, bool lean) {
-  return gb::ARGS_BYTES +
-         (lean ? gb::rt_smem_bytes(nlay) : std::max(gb::rt_smem_bytes(nlay), gb::gas_smem_bytes(nlay)));
-}
+// shared memory of a block of the transfer kernel, and of the hand-over kernel (taumol or transfer area)
+size_t block_smem(int nlay) { return gb::ARGS_BYTES + gb::rt_smem_bytes(nlay); }
+size_t list_smem(int nlay) { return gb::ARGS_BYTES + std::max(gb::rt_smem_bytes(nlay), gb::gas_smem_bytes(nlay)); }
 
 // Shared-memory carve-out for `per` resident blocks of `smem` bytes: just what
 // they need, so that the rest of the SM's memory stays L1 for the table
@@ -1556,25 +1430,52 @@ LwVariant gb_lw_variant(int v, bool lean) {
   return LwVariant{gb::RT_NT, info(v, lean).min_blocks};
 }
 
-size_t gb_lw_smem_bytes(int nlay) { return block_smem(nlay, false); }
+size_t gb_lw_smem_bytes(int nlay) { return list_smem(nlay); }
 
-cudaError_t gb_lw_set_tables(const GbTables& T) { return cudaMemcpyToSymbol(gb::c_T, &T, sizeof(GbTables)); }
+cudaError_t gb_lw_set_tables(const GbTables& T) {
+  const cudaError_t e = cudaMemcpyToSymbol(gb::c_T, &T, sizeof(GbTables));
+  return e == cudaSuccess ? gb_lw_taumol_set_tables(T) : e;
+}
 
 int gb_lw_slots(int nlay, int variant, bool lean) {
   if (variant < 0 || variant >= kNumVariants) variant = 0;
   const VariantInfo& v = info(variant, lean);
   int per = 0;
-  if (occupancy(v.fn, gb::RT_NT, block_smem(nlay, lean), &per) != cudaSuccess || per < 1) per = 1;
+  if (occupancy(v.fn, gb::RT_NT, block_smem(nlay), &per) != cudaSuccess || per < 1) per = 1;
   return device_sms() * std::min(per, kMaxPerSm);
 }
 
-long long gb_lw_gas_slots(int nlay, long long ncols) {
-  (void)nlay;
-  (void)ncols;
-  return (long long)device_sms() * kMaxPerSm;  // one per resident block of the fused or hand-over kernel
+namespace {
+// plane bytes of one column slot: its rows, setcoef's words, laytrop
+size_t slot_bytes(int nlay) { return (size_t)nlay * (GB_LW_PROW + GB_LW_COEF_WORDS) * 4 + sizeof(int); }
+// cloud planes of the resident columns
+size_t cloud_slots() { return (size_t)device_sms() * kMaxPerSm; }
+size_t cloud_bytes(int nlay) { return cloud_slots() * (size_t)nlay * GB_NGPT * sizeof(float); }
+size_t round_slots(size_t n) { return (n + 31) & ~size_t(31); }
+// a pass's planes: enough columns that the tail of a pass is small beside it
+// (a wave of the transfer is about 900 columns), few enough that the buffer
+// stays small beside the batch's own arrays
+constexpr size_t kPlaneBytes = size_t(1536) << 20;
+}  // namespace
+
+size_t gb_lw_gas_bytes(int nlay, long long ncols, bool learned) {
+  const size_t room = std::max<size_t>(kPlaneBytes / slot_bytes(nlay) & ~size_t(31), 32);
+  const size_t want = learned ? 0 : round_slots((size_t)ncols + GB_LW_MAX_GRIDS);
+  const size_t slots = std::max(std::min(want, room), round_slots((size_t)gb_lw_list_slots()));
+  return cloud_bytes(nlay) + slots * slot_bytes(nlay);
 }
 
-size_t gb_lw_gas_bytes(int nlay, long long slots) { return (size_t)slots * 3 * nlay * GB_NGPT * sizeof(float); }
+size_t gb_lw_gas_min_bytes(int nlay) { return gb_lw_gas_bytes(nlay, 0, true); }
+
+void gb_lw_attach_gas(LwBatch& b, void* buf, size_t bytes) {
+  const size_t cloud = cloud_bytes(b.nsmax);
+  b.cslots = (long long)cloud_slots();
+  b.pslots = bytes > cloud ? (long long)((bytes - cloud) / slot_bytes(b.nsmax) & ~size_t(31)) : 0;
+  b.plane = static_cast<float*>(buf);  // the rows first: each on a 32-byte boundary
+  b.coef = b.plane + (size_t)b.pslots * b.nsmax * GB_LW_PROW;
+  b.gcld = b.coef + (size_t)b.pslots * b.nsmax * GB_LW_COEF_WORDS;
+  b.laytrop = reinterpret_cast<int*>(b.gcld + (size_t)b.cslots * b.nsmax * GB_NGPT);
+}
 
 long long gb_lw_list_slots() { return (long long)device_sms() * gb::LIST_PER_SM; }
 
@@ -1585,12 +1486,15 @@ cudaError_t gb_lw_launch_gas(const LwBatch& b, const float* d_tables, long long 
   return launch_gas_range(b, d_tables, c0, c1, stream);
 }
 
-cudaError_t gb_lw_launch_batch(const LwBatch& b, const float* d_tables, int variant, int nblocks,
+cudaError_t gb_lw_launch_batch(const LwBatch& bin, const float* d_tables, int variant, int nblocks,
                                cudaStream_t stream) {
+  LwBatch b = bin;
   if (variant < 0 || variant >= kNumVariants || b.ngrid < 1 || b.ngrid > GB_LW_MAX_GRIDS) return cudaErrorInvalidValue;
   const long long n = b.col0[b.ngrid];
   if (n <= 0 || nblocks <= 0) return cudaSuccess;
-  if (!b.gtau || !b.gfrac || b.gslots < 1 || b.gstride < (long long)b.nsmax * GB_NGPT) return cudaErrorInvalidValue;
+  if (!b.plane || b.pslots < 32) return cudaErrorInvalidValue;
+  b.cpb = 1;
+  for (int i = 0; i <= b.ngrid; ++i) b.unit0[i] = b.col0[i];
   for (int i = 0; i < b.ngrid; ++i)  // fused-cloud grids come with their McICA draws
     if (b.g[i].cloud_mode == LW_CLOUD_FUSED && b.g[i].icld >= 1 && b.g[i].ncol > 0 && !b.g[i].draws)
       return cudaErrorInvalidValue;
@@ -1602,39 +1506,40 @@ cudaError_t gb_lw_launch_batch(const LwBatch& b, const float* d_tables, int vari
     if (g.icld >= 1 && g.ncol > 0 && (!g.ncbands || !g.cldfrac || !g.tauc)) return cudaErrorInvalidValue;
   }
   if ((long long)nblocks > n) nblocks = (int)n;
-  if (nband) {
-    // band clouds: every grid in that mode, taumol gas optics
-    if (nband != b.ngrid || b.fall) return cudaErrorInvalidValue;
-    if ((long long)nblocks > b.gslots) nblocks = (int)b.gslots;
-    const void* fn = (const void*)gb::lw_band_kernel<gb::BAND_MINB>;
-    const size_t smem = block_smem(b.nsmax, false);
-    return launch_resident(fn, gb::RT_NT, smem, nblocks, [&](int nb) {
-      gb::lw_band_kernel<gb::BAND_MINB><<<nb, gb::RT_NT, smem, stream>>>(b, d_tables, 0, n);
-      return cudaGetLastError();
-    });
-  }
+  if ((long long)nblocks > b.cslots) nblocks = (int)b.cslots;
+  const size_t smem = block_smem(b.nsmax);
   if (!b.fall || !b.nfall) {
-    // taumol and the transfer, one block per column, taumol's planes in the block's slot
-    if ((long long)nblocks > b.gslots) nblocks = (int)b.gslots;
+    // pass by pass: taumol into the planes, then the transfer
+    if (nband && nband != b.ngrid) return cudaErrorInvalidValue;  // band clouds: every grid in that mode
     const VariantInfo& v = info(variant, false);
-    const size_t smem = block_smem(b.nsmax, false);
-    return launch_resident(v.fn, gb::RT_NT, smem, nblocks,
-                           [&](int nb) { return v.launch(b, d_tables, 0, n, nb, smem, stream); });
+    const void* fn = nband ? (const void*)gb::lw_rt_kernel<gb::BAND_MINB, gb::RT_GAS, true> : v.fn;
+    const long long passes = (n + b.pslots - 1) / b.pslots, step = (n + passes - 1) / passes;
+    for (long long c0 = 0; c0 < n; c0 += step) {
+      const long long c1 = std::min(c0 + step, n);
+      cudaError_t e = gb_lw_launch_taumol(b, d_tables, c0, c1, stream);
+      if (e != cudaSuccess) return e;
+      e = launch_resident(fn, gb::RT_NT, smem, (int)std::min<long long>(nblocks, c1 - c0), [&](int nb) {
+        if (!nband) return v.launch(b, d_tables, c0, c1, nb, smem, stream);
+        gb::lw_rt_kernel<gb::BAND_MINB, gb::RT_GAS, true><<<nb, gb::RT_NT, smem, stream>>>(b, d_tables, c0, c1);
+        return cudaGetLastError();
+      });
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
   }
   // learned gas optics: the transfer kernel on the network's outputs, then the
   // hand-over kernel over the columns it passed on (its blocks find an empty
   // list and return when every column was on the network)
-  if (b.gslots < gb_lw_list_slots()) return cudaErrorInvalidValue;
+  if (nband || b.pslots < gb_lw_list_slots()) return cudaErrorInvalidValue;
   cudaError_t e = cudaMemsetAsync(b.nfall, 0, sizeof(unsigned), stream);
   if (e != cudaSuccess) return e;
   const VariantInfo& v = info(variant, true);
-  const size_t smem = block_smem(b.nsmax, true);
   e = launch_resident(v.fn, gb::RT_NT, smem, nblocks, [&](int nb) { return v.launch(b, d_tables, 0, n, nb, smem, stream); });
   if (e != cudaSuccess) return e;
-  const void* fn = (const void*)gb::lw_full_kernel<gb::LIST_MINB, true>;
-  const size_t lsmem = block_smem(b.nsmax, false);
+  const void* fn = (const void*)gb::lw_list_kernel<gb::LIST_MINB>;
+  const size_t lsmem = list_smem(b.nsmax);
   return launch_resident(fn, gb::RT_NT, lsmem, (int)gb_lw_list_slots(), [&](int nb) {
-    gb::lw_full_kernel<gb::LIST_MINB, true><<<nb, gb::RT_NT, lsmem, stream>>>(b, d_tables, 0, 0);
+    gb::lw_list_kernel<gb::LIST_MINB><<<nb, gb::RT_NT, lsmem, stream>>>(b, d_tables);
     return cudaGetLastError();
   });
 }

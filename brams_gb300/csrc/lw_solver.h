@@ -52,24 +52,49 @@ struct LwArgs {
 // no device-side descriptor and can be captured in a CUDA graph as is.
 #define GB_LW_MAX_GRIDS 32
 //
-// Gas optics hand-over: taumol writes, per slot, taug (without aerosol) and
-// the Planck fractions as fp32 [nlay][140] planes at gtau + slot * gstride and
-// gfrac + slot * gstride; the transfer reads them.  The fused taumol and
-// transfer kernel uses one slot per block (so that the planes stay in L2).
+// Gas optics hand-over.  A batch is solved in units of cpb neighbouring
+// columns of one grid; unit0[i] is grid i's first unit (a grid of an odd
+// number of columns leaves a column of its last unit empty).  For the units
+// [u0, u1) of one pass, taumol (gb_lw_launch_taumol) fills a plane per column
+// slot, slot (u - u0) * cpb + c:
+//   plane + (slot * nsmax + layer) * GB_LW_PROW   the layer's row: per pair of
+//     neighbouring g-points of a band (tau, tau, fraction, fraction) as fp32
+//     (taug without aerosol, Planck fractions), bands on 32-byte boundaries
+//     (gb_pair0), so that the transfer reads a pair in one 16-byte load.
+// coef and laytrop hold setcoef's words between taumol's two kernels.  A pass
+// takes as many units as the planes have room for.
 //
 // Batches with learned gas optics (fall and nfall set) run in two launches:
 // the transfer kernel solves every column whose layers are all on the network
 // and hands the others (batch numbering) over in fall[0 .. *nfall), then the
-// hand-over kernel runs taumol and the transfer for those, mixing per layer
-// the network's values and taumol's.  fall holds at least col0[ngrid] entries.
+// hand-over kernel runs taumol and the transfer for those in its blocks (block
+// k in plane slot k), mixing per layer the network's values and taumol's.
+// fall holds at least col0[ngrid] entries.
+//
+// gtau and gfrac ([slot][layer][140] planes, gstride floats per slot) are the
+// outputs of the taumol-only launch (training samples, diagnostics).
+constexpr int GB_LW_PROW = 304;        // floats per plane row: 76 pair positions
+constexpr int GB_LW_COEF_WORDS = 26;   // setcoef words per column and layer
+// first pair position of band b (1..16) in a plane row
+__host__ __device__ constexpr int gb_pair0(int b) {
+  constexpr int m[17] = {0, 0, 6, 12, 20, 28, 36, 40, 46, 50, 56, 60, 64, 68, 70, 72, 74};
+  return m[b];
+}
 struct LwBatch {
   int ngrid;
   int nsmax;                              // largest nlay (stride of the shared-memory areas)
   long long col0[GB_LW_MAX_GRIDS + 1];
-  float* gtau = nullptr;                  // gas-optics hand-over (see above)
+  int cpb = 1;                            // columns per unit (see above)
+  long long unit0[GB_LW_MAX_GRIDS + 1];
+  float* plane = nullptr;                 // gas-optics planes
+  float* coef = nullptr;                  // setcoef's words
+  int* laytrop = nullptr;                 // per slot
+  long long pslots = 0;                   // plane slots available (a multiple of 32)
+  float* gcld = nullptr;                  // caller sub-columns: each cloudy cell's optical depth (or
+                                          // fractional cldfmcl), [nsmax][140] per resident column
+  long long cslots = 0;                   // such slots available
+  float* gtau = nullptr;                  // taumol-only launch (see above)
   float* gfrac = nullptr;
-  float* gcld = nullptr;                  // caller sub-columns: each cloudy cell's optical depth
-                                          // (or fractional cldfmcl), same slots; may be NULL
   long long gstride = 0;                  // floats per slot (>= nsmax * 140)
   long long gslots = 0;                   // slots available
   long long* fall = nullptr;              // columns handed over off the network
@@ -92,20 +117,26 @@ LwVariant gb_lw_variant(int v, bool lean = false);
 size_t gb_lw_smem_bytes(int nlay);
 // column blocks of `variant` resident on the device at once for this nlay
 int gb_lw_slots(int nlay, int variant = 0, bool lean = false);
-// hand-over slots a batch is solved with (one per resident block)
-long long gb_lw_gas_slots(int nlay, long long ncols);
-// bytes of a hand-over buffer of `slots` slots (taug, fractions and cell clouds, fp32)
-size_t gb_lw_gas_bytes(int nlay, long long slots);
-// hand-over slots the hand-over kernel of a learned batch uses (one per block)
+// bytes of the hand-over buffer a batch of `ncols` columns is solved with
+// (learned: only the hand-over kernel's planes), and the least it runs with
+size_t gb_lw_gas_bytes(int nlay, long long ncols, bool learned);
+size_t gb_lw_gas_min_bytes(int nlay);
+// points a descriptor at a hand-over buffer of `bytes`
+void gb_lw_attach_gas(LwBatch& b, void* buf, size_t bytes);
+// column blocks of the hand-over kernel of a learned batch
 long long gb_lw_list_slots();
 cudaError_t gb_lw_set_tables(const GbTables& T);
 // All grids of `b` with `variant` at `nblocks` persistent blocks: taumol
-// batches through the fused taumol + transfer kernel (block k in slot k);
-// with b.fall set the learned-gas-optics transfer kernel, then the hand-over
+// batches through taumol's kernels and the transfer kernel, pass by pass; with
+// b.fall set the learned-gas-optics transfer kernel, then the hand-over
 // kernel.  Batches of LW_CLOUD_BAND grids (all grids in that mode, taumol
-// only) run the band-cloud flavour of the fused kernel.
+// only) run the band-cloud flavour of the transfer kernel.
 cudaError_t gb_lw_launch_batch(const LwBatch& b, const float* d_tables, int variant, int nblocks,
                                cudaStream_t stream);
 // The taumol kernel alone over batch columns [c0, c1) into slots 0 .. c1-c0-1.
 cudaError_t gb_lw_launch_gas(const LwBatch& b, const float* d_tables, long long c0, long long c1,
                              cudaStream_t stream);
+// taumol of units [u0, u1) into plane slots 0 .. (lw_taumol.cu).
+cudaError_t gb_lw_launch_taumol(const LwBatch& b, const float* d_tables, long long u0, long long u1,
+                                cudaStream_t stream);
+cudaError_t gb_lw_taumol_set_tables(const GbTables& T);

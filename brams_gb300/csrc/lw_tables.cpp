@@ -79,10 +79,11 @@ bool gb_build_tables(const char* ref_path, const char* k_path, double cpdair, Gb
   };
   std::memset(&T, 0, sizeof(T));
   blob.clear();
+  // every table starts on a 16-byte boundary (the taumol kernel's vector loads)
   auto push = [&](size_t n) {
-    int off = (int)blob.size();
-    blob.resize(blob.size() + n, 0.0f);
-    return off;
+    const size_t off = (blob.size() + 3) & ~size_t(3);
+    blob.resize(off + n, 0.0f);
+    return (int)off;
   };
   static const int NG[16] = GB_NG_LIST, NGS0[16] = GB_NGS0_LIST;
   const Entry *nspa = need("nspa"), *nspb = need("nspb"), *ngb = need("ngb");
@@ -96,7 +97,7 @@ bool gb_build_tables(const char* ref_path, const char* k_path, double cpdair, Gb
   T.zero_row = push(16);
   for (int b = 1; b <= 16; ++b) {
     GbBandTab& B = T.band[b - 1];
-    const int ng = NG[b - 1];
+    const int ng = NG[b - 1], pitch = gb_pitch(ng);
     B.ng = ng;
     B.g0 = NGS0[b - 1];
     B.ka = B.kb = B.fa = B.fb = B.sr = B.fo = -1;
@@ -107,51 +108,51 @@ bool gb_build_tables(const char* ref_path, const char* k_path, double cpdair, Gb
       return std::string(key);
     };
     auto has = [&](const char* n) { return tab.count(name(n)) > 0; };
-    // [rows][ng] from Fortran (rows..., ng): transpose
+    // [rows][pitch] from Fortran (rows..., ng): transpose
     auto put_rows_g = [&](const char* n) {
       const Entry* e = need(name(n));
       if (!e) return -1;
       size_t rows = e->size() / ng;
-      int off = push(rows * ng);
+      int off = push(rows * pitch);
       for (size_t r = 0; r < rows; ++r)
-        for (int g = 0; g < ng; ++g) blob[off + r * ng + g] = (float)e->d[r + rows * g];
+        for (int g = 0; g < ng; ++g) blob[off + r * pitch + g] = (float)e->d[r + rows * g];
       return off;
     };
     B.ka = put_rows_g("ka");
     if (has("kb")) B.kb = put_rows_g("kb");
     B.sr = put_rows_g("selfref");
     B.fo = put_rows_g("forref");
-    // Planck fractions: Fortran (ng) or (ng, neta) -> [neta + 1][ng]
+    // Planck fractions: Fortran (ng) or (ng, neta) -> [neta + 1][pitch]
     auto put_frac = [&](const char* n, int& nrows) {
       const Entry* e = need(name(n));
       if (!e) return -1;
       int neta = (int)(e->size() / ng);
       nrows = neta;
-      int off = push((size_t)(neta + 1) * ng);
+      int off = push((size_t)(neta + 1) * pitch);
       for (int r = 0; r < neta; ++r)
-        for (int g = 0; g < ng; ++g) blob[off + r * ng + g] = (float)e->d[g + (size_t)ng * r];
-      for (int g = 0; g < ng; ++g) blob[off + neta * ng + g] = blob[off + (neta - 1) * ng + g];
+        for (int g = 0; g < ng; ++g) blob[off + r * pitch + g] = (float)e->d[g + (size_t)ng * r];
+      for (int g = 0; g < ng; ++g) blob[off + neta * pitch + g] = blob[off + (neta - 1) * pitch + g];
       return off;
     };
     B.fa = put_frac("fracrefa", B.na_eta);
     if (has("fracrefb")) B.fb = put_frac("fracrefb", B.nb_eta);
-    // minor tables: Fortran (19, ng) -> [19][ng]; (neta, 19, ng) -> [19][neta][ng]
+    // minor tables: Fortran (19, ng) -> [19][pitch]; (neta, 19, ng) -> [19][neta][pitch]
     auto put_minor = [&](const char* n) {
       const Entry* e = need(name(n));
       if (!e) return -1;
       if (e->ndim == 2) return put_rows_g(n);
       int neta = e->dims[0];
-      int off = push((size_t)19 * neta * ng);
+      int off = push((size_t)19 * neta * pitch);
       for (int t = 0; t < 19; ++t)
         for (int a = 0; a < neta; ++a)
           for (int g = 0; g < ng; ++g)
-            blob[off + ((size_t)t * neta + a) * ng + g] = (float)e->d[a + (size_t)neta * (t + 19 * (size_t)g)];
+            blob[off + ((size_t)t * neta + a) * pitch + g] = (float)e->d[a + (size_t)neta * (t + 19 * (size_t)g)];
       return off;
     };
     auto put_vec = [&](const char* n) {
       const Entry* e = need(name(n));
       if (!e) return -1;
-      int off = push(ng);
+      int off = push(pitch);
       for (int g = 0; g < ng; ++g) blob[off + g] = (float)e->d[g];
       return off;
     };

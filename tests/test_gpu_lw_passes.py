@@ -1,0 +1,72 @@
+"""Longwave batches through taumol's planes: column counts around the 32-column
+tiles, ragged grids in one batch, shallow and deep columns, and a batch that
+takes several passes over the planes."""
+import numpy as np
+import pytest
+
+import pyoracle
+from brams_gb300 import rrtmg_lw as R
+from brams_gb300 import surrogate as S
+from brams_gb300.profiles import ProfileSpec, make_state
+
+pytestmark = pytest.mark.gpu
+
+FLUX_TOL, HR_TOL = 0.05, 0.01  # the solver's parity tolerances (W m-2, K/day)
+OUTS = ("uflx", "dflx", "hr", "uflxc", "dflxc", "hrc", "duflx_dt", "duflxc_dt")
+
+
+def _solve(ctx, grids, seeds):
+    import torch
+
+    ctx.rrtmg_lw_batch_device([g.desc(seed0=s) for g, s in zip(grids, seeds)])
+    torch.cuda.synchronize()
+    assert ctx.sync_status() == 0
+    return [g.outputs() for g in grids]
+
+
+@pytest.mark.parametrize("shapes", [[(1, 3)], [(31, 45)], [(32, 38)], [(33, 60)], [(65, 7), (1, 128), (30, 46)]])
+def test_ragged_batches_against_oracle(ctx, shapes):
+    grids, refs, seeds = [], [], []
+    for i, (ncol, nlay) in enumerate(shapes):
+        st = make_state(ProfileSpec(ncol=ncol, nlay=nlay, seed=300 + i, t_noise=4.0, h2o_sigma=0.5))
+        tauc = pyoracle.cldprop_columns(st)
+        seeds.append(50 + 1000 * i)
+        grids.append(S.DeviceGrid(st, tauc))
+        refs.append(pyoracle.rrtmg_lw(st, pyoracle.mcica_per_column(st, tauc, icld=3, base_seed=seeds[-1]), icld=3))
+    for got, ref in zip(_solve(ctx, grids, seeds), refs):
+        for k in ("uflx", "dflx", "uflxc", "dflxc"):
+            assert np.abs(got[k] - ref[k]).max() <= FLUX_TOL, k
+        for k in ("hr", "hrc"):
+            assert np.abs(got[k] - ref[k]).max() <= HR_TOL, k
+
+
+def test_several_passes_equal_separate_calls(ctx):
+    """More columns than the planes hold at once (their buffer is 1.5 GiB: about
+    30,000 columns of 38 layers), in two grids: every column has the bits of a
+    call of its own slice."""
+    import torch
+
+    from brams_gb300.shard import slice_grid
+
+    n = [40001, 30003]
+    grids = []
+    for i, ncol in enumerate(n):
+        g = S.DeviceGrid(make_state(ProfileSpec(ncol=1000, nlay=38, seed=7 + i, t_noise=4.0)))
+        rep = (ncol + 999) // 1000
+        for k, v in list(g.d.items()):
+            g.d[k] = torch.cat([v] * rep, dim=-1)[..., :ncol].contiguous()
+        g.d["tauc"] = torch.zeros((38, ncol, 16), dtype=torch.float64, device="cuda")
+        g.ncol = ncol
+        grids.append(g)
+    whole = _solve(ctx, grids, [11, 99])
+    for g, seed, ref in zip(grids, (11, 99), whole):
+        for k in OUTS:
+            g.d[k].zero_()
+        d = g.desc(seed0=seed)
+        for c0 in range(0, g.ncol, 9973):
+            ctx.rrtmg_lw_batch_device([slice_grid(d, c0, min(c0 + 9973, g.ncol))])
+        torch.cuda.synchronize()
+        got = g.outputs()
+        for k in OUTS:
+            assert np.array_equal(got[k], ref[k]), k
+    assert ctx.sync_status() == 0
