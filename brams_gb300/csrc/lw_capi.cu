@@ -182,13 +182,13 @@ int batch_kind(const LwBatch& b) {
   return k;
 }
 
-// Default shape: variant 0 at as many resident blocks as fit.  Batches with
+// Default shape: as many resident blocks as fit, with the registers these leave.  Batches with
 // learned gas optics index the shapes of the transfer kernel on the
 // network's outputs.
 gb_lw_tuning default_tuning(gb_lw_context* ctx, int nlay, int kind) {
   gb_lw_tuning t{};
   const bool lean = kind & GB_LW_KIND_LEARNED;
-  t.variant = 0;
+  t.variant = gb_lw_default_variant(nlay);
   t.threads = gb_lw_variant(t.variant, lean).threads;
   t.min_blocks = gb_lw_variant(t.variant, lean).min_blocks;
   const int occ = std::max(1, gb_lw_slots(nlay, t.variant, lean) / std::max(1, ctx->num_sms));

@@ -1,10 +1,11 @@
 // RRTMG_LW column kernels for GB300 (sm_103a).
 //
 // The reference solves one column at a time (rrtmg_lw_rad.f90:486-593):
-// inatm, cldprmc, setcoef, taumol, the aerosol add and rtrnmc.  Here one
-// thread block of 160 threads solves a column, thread t standing for g-point
-// t (the last warp has 12 live lanes), and persistent blocks walk the columns
-// of a batch of grids.  Nothing per cell goes to global scratch:
+// inatm, cldprmc, setcoef, taumol, the aerosol add and rtrnmc.  Here a unit of
+// 160 threads solves two neighbouring columns, 80 threads a column, each
+// standing for a pair of g-points of one band (70 live); an SM holds up to four units, which
+// walk the columns of a batch of grids.  Nothing per cell goes to global scratch
+// but the clouds of caller sub-columns:
 //
 //   taumol -- of a batch, by kernels of its own (lw_taumol.cu), into a plane
 //     per column that the transfer reads; the batch goes through in passes of
@@ -26,16 +27,21 @@
 //     downward pass from the model top and an upward pass from the surface.
 //     Each pass evaluates a cell's transmittance and sources in registers from
 //     taug, the Planck fraction, the layer's Planck values and rtrnmc's
-//     exp_tbl/tfn_tbl/tau_tbl (rrtmg_lw_init.f90:120-142, built in double
-//     precision at set-up) at the reference's quantised index
+//     exp_tbl/tfn_tbl (rrtmg_lw_init.f90:120-142, built in double
+//     precision at set-up, held in shared memory) at the reference's quantised index
 //     (rtrnmc.f90:350-455 down, 486-529 up); the up pass recomputes what the
-//     down pass computed instead of storing it.  The passes are software
-//     pipelined: while layer l is finished, the gas optics of the layer two
-//     ahead are loaded and the table entry of the next layer is looked up.
-//     Per level the 32 lanes' weighted radiances are summed with a transposed
-//     butterfly (two streams down, four up); the five warps' fp32 partials
+//     down pass computed instead of storing it.  The sums over the g-points
+//     of a level go by transposed butterflies over a group of 32 g-points (two
+//     streams down, four up); the five groups' fp32 partials
 //     are added error-free (two-sum) into fp64, and the net fluxes and heating
 //     rates heatfac*dF/dp are fp64 (rtrnmc.f90:566-592).
+//
+//     A thread had one g-point of one column before, with the table in L1:
+//     66,000 warp instructions a column of 60 layers at 52% of the issue
+//     slots, 28.8 ms for 262,144 columns.  Two g-points a thread share a layer's
+//     records, loop and branches and half the sums (46,900 instructions); what
+//     bounds it is those instructions, at 15 to 20 warps an SM, and the
+//     latency of the set-up phases.  1.34 ms for 16,384 columns (1.80 before).
 //
 // Kernels: lw_rt_kernel (the transfer, on taumol's planes or on the network's
 // fp16 taug and Planck fractions; there, columns with a layer off the network
@@ -66,8 +72,11 @@ namespace gb {
 constexpr float BPADE = 1.0f / 0.278f;
 constexpr float REC_6 = 0.166667f;
 constexpr int TGROUP = MAXT_ALL;  // term slots per layer of a band's term list
-constexpr int RT_NT = 160;        // threads per column block: one per g-point
-constexpr int RT_NW = RT_NT / 32;
+constexpr int RT_NT = 160;        // threads per block of two columns; virtual threads per column in the
+                                  // phases whose order of operations goes by thread
+constexpr int RT_CT = 80;         // threads per column in the passes: one per pair of g-points
+constexpr int RT_NW = RT_NT / 32; // groups of 32 g-points of a column
+constexpr int LIST_PER_SM = 2;    // hand-over kernel blocks per SM
 
 __constant__ int c_icb[16] = {1, 2, 3, 3, 3, 4, 4, 4, 5, 5, 5, 5, 5, 5, 5, 5};  // cldprmc.f90:133
 // diffusivity-angle coefficients (rtrnmc.f90:236-247)
@@ -78,84 +87,111 @@ __constant__ float c_a2[16] = {0.f, -12.0f, -11.7f, 0.f, -0.72f, -0.243f, 0.19f,
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
 // ------------------------------------------------------------------ helpers
-// Warp sums of two values per lane at once: lane i returns the sum over the
-// 32 lanes of v(i & 1) (one exchange, then four xor steps).
-__device__ __forceinline__ float reduce2(float v0, float v1, int lane) {
-  const unsigned F = 0xffffffffu;
-  const bool lo = lane & 1;
-  float k = lo ? v1 : v0;
-  const float s = lo ? v0 : v1;
-  k += __shfl_xor_sync(F, s, 1);
-  k += __shfl_xor_sync(F, k, 2);
-  k += __shfl_xor_sync(F, k, 4);
-  k += __shfl_xor_sync(F, k, 8);
-  k += __shfl_xor_sync(F, k, 16);
+// ---- two g-points per thread: packed fp32 arithmetic (each half rounds as
+// the scalar operation does)
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 pk(float2 v) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
+  return r;
+}
+__device__ __forceinline__ float2 upk(u64 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  u64 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk(a)), "l"(pk(b)), "l"(pk(c)));
+  return upk(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  u64 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk(a)), "l"(pk(b)));
+  return upk(r);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  u64 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk(a)), "l"(pk(b)));
+  return upk(r);
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 sel2(bool c, float2 a, float2 b) { return c ? a : b; }
+__device__ __forceinline__ float2 shfl2(float2 v, int m) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+
+// Sums over the 32 g-points of a group: 16 lanes, lane l holding g-points 2l
+// and 2l + 1 of the group in the halves of a value.  Transposed butterflies;
+// the order of the additions (over bits of the g-point's number in the group)
+// is part of the result: sum2 adds over bits 0, 1, 2, 3, 4; sum4 over 1, 0, 2,
+// 3, 4; sum8 over 2, 1, 0, 3, 4 -- the orders of a butterfly with one g-point
+// per lane, which is what the fluxes' last bits were before.
+// sum2: lane l returns the sum of v[l & 1]
+__device__ __forceinline__ float sum2(float2 v0, float2 v1, int l) {
+  const float k0 = v0.x + v0.y, k1 = v1.x + v1.y;
+  const bool h = l & 1;
+  float k = h ? k1 : k0;
+  k += __shfl_xor_sync(0xffffffffu, h ? k0 : k1, 1);
+  k += __shfl_xor_sync(0xffffffffu, k, 2);
+  k += __shfl_xor_sync(0xffffffffu, k, 4);
+  k += __shfl_xor_sync(0xffffffffu, k, 8);
+  return k;
+}
+// sum4: lane l returns the sum of v[sum4_at(l)]
+__device__ __forceinline__ int sum4_at(int l) { return 2 * (l & 1) + ((l >> 1) & 1); }
+__device__ __forceinline__ float sum4(float2 v0, float2 v1, float2 v2, float2 v3, int l) {
+  const bool h = l & 1;
+  const float2 a0 = add2(sel2(h, v2, v0), shfl2(sel2(h, v0, v2), 1));
+  const float2 a1 = add2(sel2(h, v3, v1), shfl2(sel2(h, v1, v3), 1));
+  const float k0 = a0.x + a0.y, k1 = a1.x + a1.y;
+  const bool g = l & 2;
+  float k = g ? k1 : k0;
+  k += __shfl_xor_sync(0xffffffffu, g ? k0 : k1, 2);
+  k += __shfl_xor_sync(0xffffffffu, k, 4);
+  k += __shfl_xor_sync(0xffffffffu, k, 8);
+  return k;
+}
+// sum8: lane l returns the sum of v[sum8_at(l)]
+__device__ __forceinline__ int sum8_at(int l) { return 4 * ((l >> 1) & 1) + 2 * (l & 1) + ((l >> 2) & 1); }
+__device__ __forceinline__ float sum8(float2 v0, float2 v1, float2 v2, float2 v3, float2 v4, float2 v5, float2 v6,
+                                      float2 v7, int l) {
+  const bool h = l & 2;
+  const float2 a0 = add2(sel2(h, v4, v0), shfl2(sel2(h, v0, v4), 2));
+  const float2 a1 = add2(sel2(h, v5, v1), shfl2(sel2(h, v1, v5), 2));
+  const float2 a2 = add2(sel2(h, v6, v2), shfl2(sel2(h, v2, v6), 2));
+  const float2 a3 = add2(sel2(h, v7, v3), shfl2(sel2(h, v3, v7), 2));
+  const bool g = l & 1;
+  const float2 c0 = add2(sel2(g, a2, a0), shfl2(sel2(g, a0, a2), 1));
+  const float2 c1 = add2(sel2(g, a3, a1), shfl2(sel2(g, a1, a3), 1));
+  const float k0 = c0.x + c0.y, k1 = c1.x + c1.y;
+  const bool f = l & 4;
+  float k = f ? k1 : k0;
+  k += __shfl_xor_sync(0xffffffffu, f ? k0 : k1, 4);
+  k += __shfl_xor_sync(0xffffffffu, k, 8);
   return k;
 }
 
-// Warp sums of four values per lane at once (a transposed butterfly, 6
-// shuffles instead of 20): lane i returns the sum over the 32 lanes of v[i & 3].
-__device__ __forceinline__ float reduce4(float v0, float v1, float v2, float v3, int lane) {
-  const unsigned F = 0xffffffffu;
-  const bool hi = lane & 2;
-  float k0 = hi ? v2 : v0, k1 = hi ? v3 : v1;
-  const float s0 = hi ? v0 : v2, s1 = hi ? v1 : v3;
-  k0 += __shfl_xor_sync(F, s0, 2);
-  k1 += __shfl_xor_sync(F, s1, 2);
-  const bool lo = lane & 1;
-  float k = lo ? k1 : k0;
-  const float sx = lo ? k0 : k1;
-  k += __shfl_xor_sync(F, sx, 1);
-  k += __shfl_xor_sync(F, k, 4);
-  k += __shfl_xor_sync(F, k, 8);
-  k += __shfl_xor_sync(F, k, 16);
-  return k;
+// od / (bpade + od) as __fdividef forms it (a divisor above 2^126 gives 0), without its scaling of
+// subnormal divisors, which bpade + od is not
+__device__ __forceinline__ float tbl_quotient(float od) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(BPADE + od));
+  return od * r;
 }
-
-// Warp sums of eight values per lane at once: lane i returns the sum over the
-// 32 lanes of v[i & 7] (three exchanges, then two xor steps: 9 shuffles).
-__device__ __forceinline__ float reduce8(float v0, float v1, float v2, float v3, float v4, float v5, float v6,
-                                         float v7, int lane) {
-  const unsigned F = 0xffffffffu;
-  const bool h4 = lane & 4;
-  float a0 = h4 ? v4 : v0, a1 = h4 ? v5 : v1, a2 = h4 ? v6 : v2, a3 = h4 ? v7 : v3;
-  const float b0 = h4 ? v0 : v4, b1 = h4 ? v1 : v5, b2 = h4 ? v2 : v6, b3 = h4 ? v3 : v7;
-  a0 += __shfl_xor_sync(F, b0, 4);
-  a1 += __shfl_xor_sync(F, b1, 4);
-  a2 += __shfl_xor_sync(F, b2, 4);
-  a3 += __shfl_xor_sync(F, b3, 4);
-  const bool h2 = lane & 2;
-  float c0 = h2 ? a2 : a0, c1 = h2 ? a3 : a1;
-  const float d0 = h2 ? a0 : a2, d1 = h2 ? a1 : a3;
-  c0 += __shfl_xor_sync(F, d0, 2);
-  c1 += __shfl_xor_sync(F, d1, 2);
-  const bool h1 = lane & 1;
-  float k = h1 ? c1 : c0;
-  const float e = h1 ? c0 : c1;
-  k += __shfl_xor_sync(F, e, 1);
-  k += __shfl_xor_sync(F, k, 8);
-  k += __shfl_xor_sync(F, k, 16);
-  return k;
-}
-
 // rtrnmc's table index of an optical depth (rrtmg_lw_rtrnmc.f90:385-388):
-// itr = int(tblint * od / (bpade + od) + 0.5), within 0 .. ntbl
+// itr = int(tblint * od / (bpade + od) + 0.5), within 0 .. ntbl (od >= 0, and
+// a quotient that is not a number converts to 0)
 __device__ __forceinline__ int tbl_index(float od) {
   const float tblind = __fdividef(od, BPADE + od);
   const int itr = (int)fmaf(10000.0f, tblind, 0.5f);
   return itr < 0 ? 0 : (itr > 10000 ? 10000 : itr);
 }
-// (exp_tbl, tfn_tbl) and tau_tbl at an index (rrtmg_lw_init.f90:120-142,
-// computed in double precision at set-up and stored as float)
-__device__ __forceinline__ float2 tbl_tt(const float* __restrict__ T, int itr) {
-  return __ldg(reinterpret_cast<const float2*>(T + c_T.tbl_tt) + itr);
-}
 // tau_tbl at an index formed in registers, bpade * t / (1 - t) at t = itr /
 // 10000 (1e10 at the last entry; rrtmg_lw_init.f90:120-142), instead of a
 // table load that depends on the clear cell's lookup (fp32 arithmetic: within
 // a few units in the last place of the fp64-built table's float)
-__device__ __forceinline__ float tbl_tau(const float* __restrict__ T, int itr) {
-  (void)T;
+__device__ __forceinline__ float tbl_tau(int itr) {
   const float t = (float)itr * 1.0e-4f;
   return itr >= 10000 ? 1.0e10f : BPADE * t / (1.0f - t);
 }
@@ -307,16 +343,15 @@ __device__ void gas_column(const LwArgs& a, long long icol, const GasSmem& s, co
 // + a constant), then the per-warp level sums.
 struct RtHead {
   float misc[64];         // secdiff[16], plankbnd[16], dplankbnd[16], semiss[16]
-  float red[2 * RT_NW];   // per-warp column sums for pwvcm
-  int iscal[4];           // stop code, lower-layer count
+  float red[2 * RT_NW];   // column sums for pwvcm of 32 layers each
+  int iscal[4];           // stop code, lower-layer count, cloud-band count or off the network, check bits
   int pad[2];
 };
 struct RtLayer {
-  float4 rec[16];     // per band: Planck value of the layer, level-minus-layer Planck below and
-                      // above (dplankdn, dplankup), aerosol optical depth
-  float tcl[16];      // fused clouds: cloud optical depth per band; caller sub-columns: the
-                      // first five words are fbits (bit g: cldfmcl neither 0 nor 1); band
-                      // clouds: secdiff(ib) * taucloud per cloud band ib (rtrn's odcld)
+  float4 rec[16];     // per band: Planck value of the layer, that of the level above it, aerosol optical
+                      // depth, cloud optical depth (fused clouds; band clouds: secdiff(ib) * taucloud
+                      // per cloud band ib, rtrn's odcld).  The record before layer 0 has the
+                      // Planck value of the lowest level.
   int cldlay;         // 1: a cell of the layer has cldfmc == 1 (rtrnmc's icldlyr), or band
                       // clouds: cldfrac >= 1e-6; in the first phase: 1 where the layer is in
                       // the lower atmosphere
@@ -326,153 +361,105 @@ struct RtLayer {
   // 14 floats (RtSmem::ovl): cldfrac, rtrnmr's upward overlap factors at lev+1
   // (facclr1, facclr2, faccld1, faccld2, faccmb1, faccmb2) and the downward
   // ones at lev-1, in that order
-  unsigned cbits[5];  // bit g set where the cell is cloudy (cldfmc == 1)
-  int pad0;
+  unsigned cbits[5];  // per group of 32 g-points: bit l set where g-point 2l of the group is cloudy
+                      // (cldfmc == 1; caller sub-columns: or a fraction, in a layer with a cell
+                      // of 1), bit 16 + l where g-point 2l + 1 is
+  int pad0;           // caller sub-columns: five words from here on (RtSmem::fbits), as cbits:
+                      // cldfmcl neither 0 nor 1
   long long cthr;     // fused clouds: McICA threshold 1 - cldf as double bits
   long long pad1;
   float4 lcw;         // (ciwp, clwp, radice, radliq) as floats
 };
-static_assert(sizeof(RtHead) == 320 && sizeof(RtLayer) == 384, "transfer shared-memory records");
+static_assert(sizeof(RtHead) == 320 && sizeof(RtLayer) == 320, "transfer shared-memory records");
 static_assert(offsetof(RtLayer, lcw) + sizeof(float4) - offsetof(RtLayer, cbits) == 14 * sizeof(float),
               "band-cloud overlay of the McICA words");
+static_assert(offsetof(RtLayer, lcw) - offsetof(RtLayer, pad0) == 5 * sizeof(unsigned), "fraction bits of caller sub-columns");
 
 struct RtSmem {
   RtHead* h;
-  RtLayer* L;   // [nl]; in the last phase: fp64 net fluxes [nl+1][2]
-  float* part;  // [RT_NW][nl+1][6] per-warp level sums: dn, dn clear, up, up clear, dup/dT,
-                // dup clear/dT; in the first phase: float4 per level, the Planck-table row and
-                // fraction of tlev and tlay
-  __device__ __forceinline__ unsigned* fbits(int lay) const { return reinterpret_cast<unsigned*>(L[lay].tcl); }
+  RtLayer* L;   // [-1 .. nl-1]; in the last phase: fp64 net fluxes [nl+1][2]
+  float4* prow; // [nl+1] first phase: the Planck-table row and fraction of tlev and tlay; then band
+                // clouds' fractions in fp64
+  float* part;  // [RT_NW][nl+1][6] level sums per group of 32 g-points: dn, dn clear, up, up clear, dup/dT,
+                // dup clear/dT (global scratch)
+  __device__ __forceinline__ unsigned* fbits(int lay) const { return reinterpret_cast<unsigned*>(&L[lay].pad0); }
   __device__ __forceinline__ float* ovl(int lay) const { return reinterpret_cast<float*>(L[lay].cbits); }
 };
 
 __host__ __device__ inline size_t rt_layers_bytes(int nl) {
-  const size_t layers = (size_t)(nl < 1 ? 1 : nl) * sizeof(RtLayer);
-  return layers > (size_t)(nl + 1) * 16 ? layers : (size_t)(nl + 1) * 16;
+  return (size_t)(nl + 1) * sizeof(RtLayer);
 }
 __host__ __device__ inline size_t rt_smem_bytes(int nl) {
-  return sizeof(RtHead) + rt_layers_bytes(nl) + align16((size_t)RT_NW * (nl + 1) * 6 * 4);
+  return sizeof(RtHead) + rt_layers_bytes(nl) + align16((size_t)(nl + 1) * 24);
 }
+// floats of a column's level sums
+__host__ __device__ inline size_t rt_part_floats(int nl) { return (size_t)RT_NW * (nl + 1) * 6; }
 
-__device__ inline RtSmem rt_carve(char* p, int nl) {
+__device__ inline RtSmem rt_carve(char* p, int nl, float* part) {
   RtSmem s;
   s.h = (RtHead*)p;
   p += sizeof(RtHead);
-  s.L = (RtLayer*)p;
+  s.L = (RtLayer*)p + 1;
   p += rt_layers_bytes(nl);
-  s.part = (float*)p;
+  s.prow = (float4*)p;
+  s.part = part;
   return s;
 }
 
 // Where taug and the Planck fractions of a column come from.
 struct GasSrc {
   const float* plane;         // taumol's plane of the column (rows of GB_LW_PROW floats), or NULL
-  float* gc;                  // caller sub-columns: the cells' cloud plane [nl][140], or NULL
+  float* gc;                  // caller sub-columns: the cells' cloud plane [nl][140]
   const __half* nt;           // fp16 rows [nl][140] (network), or NULL
   const __half* nf;
   const unsigned char* flag;  // per layer: 1 -> network, 0 -> fp32 planes
 };
-enum RtMode { RT_GAS = 0, RT_NET = 1, RT_MIX = 2 };
-
-template <int MODE>
-__device__ __forceinline__ bool layer_on_net(const GasSrc& src, int lay) {
-  if (MODE == RT_GAS) return false;
-  if (MODE == RT_NET) return true;
-  return src.flag[lay] != 0;
-}
+// taumol's planes; the network's rows, on 4-byte boundaries or on any; per
+// layer one or the other
+enum RtMode { RT_GAS = 0, RT_NET = 1, RT_NETODD = 2, RT_MIX = 3 };
 
 // g-point gi of band b (1..16) in a plane row: its taug, and its Planck fraction two floats on
 __host__ __device__ constexpr int plane_pos(int b, int gi) { return 4 * (gb_pair0(b) + gi / 2) + gi % 2; }
 
-// po: the g-point's position in a plane row
+// taug (x, y) and Planck fractions (z, w) of the pair of g-points g, g + 1 of
+// a layer; po: the pair's position in a plane row
 template <int MODE>
-__device__ __forceinline__ void gas_at(const GasSrc& src, bool net, int lay, int g, int po, float& tg, float& pf) {
-  if (MODE != RT_GAS && net) {
+__device__ __forceinline__ float4 gas_at(const GasSrc& src, int lay, int g, int po) {
+  if (MODE == RT_NET) {
     const int o = lay * GB_NGPT + g;
-    tg = __half2float(__ldg(src.nt + o));
-    pf = __half2float(__ldg(src.nf + o));
-  } else {
-    const float* p = src.plane + lay * GB_LW_PROW + po;  // plain loads: the hand-over kernel's taumol
-    tg = p[0];                                           // wrote its planes in the same launch
-    pf = p[2];
+    const float2 t = __half22float2(__ldg(reinterpret_cast<const __half2*>(src.nt + o)));
+    const float2 f = __half22float2(__ldg(reinterpret_cast<const __half2*>(src.nf + o)));
+    return make_float4(t.x, t.y, f.x, f.y);
   }
-}
-
-// Clear-sky layer transmittance and source factor of a cell: rtrnmc's
-// odepth <= 0.06 expansion or its table lookup (rtrnmc.f90:380-413).  x is
-// odepth/6 or tfn; the source from level Planck values is
-// plfrac * (blay + x * dplank).  itr is the table index (used above 0.06).
-struct Clr {
-  float atrans, x;
-  int itr;
-  bool thin;
-};
-__device__ __forceinline__ Clr clear_cell(const float* __restrict__ T, float od) {
-  Clr c;
-  c.thin = od <= 0.06f;
-  c.itr = tbl_index(od);
-  const float2 e = tbl_tt(T, c.itr);  // looked up for every cell (branch-free), used above 0.06
-  c.atrans = c.thin ? fmaf(-0.5f * od, od, od) : 1.0f - e.x;
-  c.x = c.thin ? REC_6 * od : e.y;
-  return c;
+  if (MODE == RT_NETODD || (MODE == RT_MIX && src.flag[lay] != 0)) {
+    const int o = lay * GB_NGPT + g;
+    return make_float4(__half2float(__ldg(src.nt + o)), __half2float(__ldg(src.nt + o + 1)),
+                       __half2float(__ldg(src.nf + o)), __half2float(__ldg(src.nf + o + 1)));
+  }
+  // plain loads: the hand-over kernel's taumol wrote its planes in the same launch
+  return *reinterpret_cast<const float4*>(src.plane + lay * GB_LW_PROW + po);
 }
 
 // Total (gas + cloud) absorptance and source factor of a cloudy cell
 // (rtrnmc.f90:356-379): the expansion below 0.06, else the table at the
 // clear cell's optical depth (odepth itself below 0.06, else tau_tbl at its
 // index) plus the cloud's.
-__device__ __forceinline__ void cloud_total(const float* __restrict__ T, const Clr& c, float od, float odcld,
-                                            float& atot, float& x) {
+__device__ __forceinline__ void cloud_total(const float2* tt, int itr, float od, float odcld, float& atot,
+                                            float& x) {
   const float odtot = od + odcld;
   if (odtot < 0.06f) {
     atot = fmaf(-0.5f * odtot, odtot, odtot);
     x = REC_6 * odtot;
   } else {
-    const float tauq = c.thin ? od : tbl_tau(T, c.itr);
-    const float2 et = tbl_tt(T, tbl_index(tauq + odcld));
+    const float tauq = od <= 0.06f ? od : tbl_tau(itr);
+    const float2 et = tt[tbl_index(tauq + odcld)];
     atot = 1.0f - et.x;
     x = et.y;
   }
 }
 
-// McICA cloud of a cell flagged cloudy in the layer bits: returns cldfmc and
-// sets the cloud optical depth along the diffusivity angle and its
-// absorptance (cldprmc.f90:178-266, rtrnmc.f90:300-312); a fractional
-// cldfmc (caller sub-columns only) enters with zero cloud optical depth.
-__device__ __forceinline__ float cell_cloud(const LwArgs& a, const RtSmem& S, long long icol, int g, int lay,
-                                            int band, float secdiff, bool one, const float* __restrict__ T,
-                                            float& odcld, float& efcl) {
-  odcld = 0.0f;
-  efcl = 0.0f;
-  if (a.cloud_mode == LW_CLOUD_FUSED) {
-    odcld = secdiff * S.L[lay].tcl[band];
-    efcl = 1.0f - __expf(-odcld);
-    return 1.0f;
-  }
-  const long long o = (long long)g + GB_NGPT * (icol + (long long)a.ld * lay);
-  if (!one) return (float)__ldg(a.cldfmcl + o);
-  const double ciwp = __ldg(a.ciwpmcl + o), clwp = __ldg(a.clwpmcl + o);
-  // the optical depth from this cell's water paths and the layer's radii, or the caller's taucmcl
-  float tauc = 0.0f;
-  bool from_paths = a.inflag == 2 && ciwp + clwp >= 1.e-20;
-  if (!from_paths) {
-    const double tin = __ldg(a.taucmcl + o);
-    const long long tb = __double_as_longlong(tin);
-    from_paths = a.inflag == 2 && tb >= __double_as_longlong(1.0e-20) && tb <= 0x7FF0000000000000LL;
-    tauc = (float)tin;
-  }
-  if (from_paths) {
-    const int fl = ((__double_as_longlong(ciwp) << 1) != 0LL ? 1 : 0) | ((__double_as_longlong(clwp) << 1) != 0LL ? 2 : 0);
-    const float4 r = S.L[lay].lcw;
-    tauc = cloud_tau_layer(a, band, T, make_float4((float)ciwp, (float)clwp, r.z, r.w), fl);
-  }
-  odcld = secdiff * tauc;
-  efcl = 1.0f - __expf(-odcld);
-  return 1.0f;
-}
-
 // a caller sub-column cell's cloud value for the transfer: its cloud optical
-// depth (cldprmc.f90:178-266, formed as cell_cloud does) where cldfmcl = 1,
+// depth (cldprmc.f90:178-266, rtrnmc.f90:300-312) where cldfmcl = 1,
 // the fraction itself where it is neither 0 nor 1
 __device__ __forceinline__ float cell_value(const LwArgs& a, const RtSmem& S, int lay, int band, bool one,
                                             double cf, double ciwp, double clwp, double tin,
@@ -493,7 +480,8 @@ __device__ __forceinline__ float cell_value(const LwArgs& a, const RtSmem& S, in
   return tauc;
 }
 
-// the transfer's cloud of a caller sub-column cell from its hand-over value
+// the transfer's cloud of a caller sub-column cell from its hand-over value; a
+// fractional cldfmc enters with zero cloud optical depth
 __device__ __forceinline__ float cell_from_value(bool one, float v, float secdiff, float& odcld, float& efcl) {
   if (!one) {
     odcld = 0.0f;
@@ -517,6 +505,32 @@ __device__ __forceinline__ int ice_code(int iceflag, double rice) {
 __device__ __forceinline__ int liq_code(int liqflag, double rliq) {
   return liqflag == 1 && (rliq < 2.5 || rliq > 60.0) ? GB_COL_LIQ_BOUNDS : 0;
 }
+
+// a unit of a block: the threads that solve a unit's columns, with a barrier of their own
+struct Unit {
+  int tid, nt, bar;
+  const float2* tt;  // rtrnmc's (exp_tbl, tfn_tbl), in shared memory
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory"); }
+};
+// the columns of a unit: n (1 or 2) neighbouring columns of one grid from
+// col0 on, `last` the grid's last column (the second column of a grid's last
+// unit may be missing: it reads the last column's inputs and writes nothing)
+struct Cols {
+  char* smem;
+  size_t stride;  // shared memory per column
+  float* part;    // level sums of the first column
+  int n, nlmax;
+  long long col0, last;
+  // item i of a loop over the unit's columns and something else: its column and the rest
+  __device__ __forceinline__ int c(int i) const { return i & (n - 1); }
+  __device__ __forceinline__ int rest(int i) const { return i >> (n - 1); }
+  __device__ __forceinline__ RtSmem S(int c) const {
+    return rt_carve(smem + c * stride, nlmax, part + c * rt_part_floats(nlmax));
+  }
+  __device__ __forceinline__ long long icol(int c) const { return col0 + c < last ? col0 + c : last; }
+};
+// fp64 fractions for the overlap factors, after the Planck-table rows of the first phase
+__device__ __forceinline__ double* band_cf64(const RtSmem& S, int nl) { return reinterpret_cast<double*>(S.prow + nl + 1); }
 
 // rtrnmr's maximum/random overlap factors (rrtmg_lw_rtrnmr.f90:345-514), by
 // one thread in fp64 from the layer fractions cf[0 .. nl-1]; lev is the
@@ -655,37 +669,42 @@ __device__ __noinline__ void band_overlap(const RtSmem& S, const double* __restr
 }
 
 // The band clouds of the non-McICA driver (nomcica.f90:886-920, rtrn.f90:319-336,
-// rtrnmr.f90:334-343): per layer the fraction, icldlyr (cldfrac >= 1e-6) and
+// rtrnmr.f90:334-343), for each of the block's columns: per layer the fraction, icldlyr (cldfrac >= 1e-6) and
 // odcld = secdiff(ib) * taucloud(ib) for the cloud bands ib < ncbands, then
 // for maximum/random overlap the overlap factors.  Ends with a barrier when
 // it computes them.
-__device__ __forceinline__ void band_clouds(const LwArgs& a, long long icol, const RtSmem& S, int nl, bool clouds) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void band_clouds(const LwArgs& a, const Unit& U, const Cols& C, int nl, bool clouds) {
+  const int tid = U.tid, nt = U.nt;
   if (!clouds) {
-    for (int lay = tid; lay < nl; lay += RT_NT) S.L[lay].cldlay = 0;
+    for (int it = tid; it < C.n * nl; it += nt) C.S(C.c(it)).L[C.rest(it)].cldlay = 0;
     return;
   }
-  // fp64 fractions for the overlap factors, after the Planck-table rows of the first phase
-  double* cf64 = reinterpret_cast<double*>(S.part + 4 * (nl + 1));
-  const int ncb = __ldg(a.ncbands + icol);
-  if (tid == 0) S.h->iscal[2] = ncb;
-  for (int lay = tid; lay < nl; lay += RT_NT) {
-    const double cf = in2(a.cldfrac, a.ld, icol, lay);
+  for (int it = tid; it < C.n * nl; it += nt) {
+    const int c = C.c(it), lay = C.rest(it);
+    const RtSmem S = C.S(c);
+    const double cf = in2(a.cldfrac, a.ld, C.icol(c), lay);
     S.L[lay].cldlay = cf >= 1.e-6;
     S.L[lay].lfl = 0;
     float* ov = S.ovl(lay);
     ov[0] = (float)cf;
 #pragma unroll
     for (int k = 1; k < 14; ++k) ov[k] = 0.0f;
-    cf64[lay] = cf;
+    band_cf64(S, nl)[lay] = cf;
+    if (lay == 0) S.h->iscal[2] = __ldg(a.ncbands + C.icol(c));
   }
-  for (int it = tid; it < nl * 16; it += RT_NT) {
-    const int lay = it >> 4, ib = it & 15;
-    S.L[lay].tcl[ib] = ib < ncb ? S.h->misc[ib] * (float)__ldg(a.tauc + ib + 16 * (icol + a.ld * lay)) : 0.0f;
+  for (int it = tid; it < C.n * nl * 16; it += nt) {
+    const int c = C.c(it), lay = C.rest(it) >> 4, ib = C.rest(it) & 15;
+    const RtSmem S = C.S(c);
+    const long long icol = C.icol(c);
+    S.L[lay].rec[ib].w = ib < __ldg(a.ncbands + icol)
+                           ? S.h->misc[ib] * (float)__ldg(a.tauc + ib + 16 * (icol + a.ld * lay)) : 0.0f;
   }
   if (a.icld >= 2) {
-    __syncthreads();
-    if (tid == 0) band_overlap(S, cf64, nl);
+    U.sync();
+    if (tid % RT_CT == 0 && tid / RT_CT < C.n) {
+      const RtSmem S = C.S(tid / RT_CT);
+      band_overlap(S, band_cf64(S, nl), nl);
+    }
   }
 }
 
@@ -696,238 +715,578 @@ __device__ __forceinline__ int cloud_band(int ncb, int band) {
   return band;
 }
 
-// The transfer of one column by the block (see the file header).  RT_NET: a
-// column with any layer off the network is not solved (returns false in
-// every thread).  BAND: the non-McICA driver's band clouds (random overlap
-// for icld 1, maximum/random otherwise).  Ends with a barrier.
+// ---------------------------------------------------------------- the passes
+// Clouds of the passes: in-kernel sub-columns (or none), caller sub-columns,
+// band clouds with random or with maximum/random overlap.
+enum PassKind { PK_FUSED = 0, PK_SUBCOL = 1, PK_RANDOM = 2, PK_MAXRAN = 3 };
+
+// The downward and the upward pass of one column by the threads of its pairs of
+// g-points (rtrnmc.f90:347-529), level sums per group of 32 g-points into part.
+// What a thread reads of a layer is one 16-byte word of shared memory (its
+// band's record), one word of cloud bits and one 16-byte load of gas optics.
+// The layers go two by two.  Software pipelined: the gas optics are loaded two
+// pairs of layers ahead, the exponential table is looked up one pair ahead; the
+// level sums of a pair share one transposed butterfly.  A pair of layers in
+// which no lane of the warp has a cloud is one run of code without a branch,
+// so that its four cells' chains, the next pair's lookups and the sums
+// overlap in one warp's instruction stream: an SM holds 20 of these warps,
+// and a chain of a layer's cells is some 900 cycles long.
+template <int MODE, int KIND>
+struct Passes {
+  static constexpr bool BAND = KIND >= PK_RANDOM;
+  struct Stage {
+    float od0, od1;  // optical depths
+    float2 e0, e1;   // (exp_tbl, tfn_tbl) at their indices (used above 0.06; index 0 below, so that such
+                     // lanes share a load's line)
+    float2 pf;       // Planck fractions
+  };
+  const GasSrc& src;
+  const RtLayer* L0;
+  const float2* tt;  // (exp_tbl, tfn_tbl), in shared memory
+  const float* gc;
+  float* part;
+  float sd;
+  float2 wgt;
+  int nl, band, cband, g, po, grp, l16, lw;
+  float2 cr, kr, radm;  // rtrnmr's cloudy and clear radiances and overlap term
+
+  __device__ __forceinline__ static int index(float od) {
+    return min((int)fmaf(10000.0f, tbl_quotient(od), 0.5f), 10000);
+  }
+  __device__ __forceinline__ float4 gas(int lay) const { return gas_at<MODE>(src, lay, g, po); }
+  // stages layer lay, whose gas optics are p
+  __device__ __forceinline__ Stage stage(int lay, const float4& p) const {
+    Stage s;
+    const float taua = L0[lay].rec[band].z;
+    s.pf = make_float2(p.z, p.w);
+    s.od0 = fmaxf(sd * (p.x + taua), 0.0f);
+    s.od1 = fmaxf(sd * (p.y + taua), 0.0f);
+    s.e0 = tt[s.od0 <= 0.06f ? 0 : index(s.od0)];
+    s.e1 = tt[s.od1 <= 0.06f ? 0 : index(s.od1)];
+    return s;
+  }
+  __device__ __forceinline__ unsigned bits(int lay) const {
+    return BAND ? (unsigned)L0[lay].cldlay : (L0[lay].cbits[grp] >> l16) & 0x10001u;
+  }
+  // caller sub-columns: the cloud values of the layer's cells (where one has a cloud)
+  __device__ __forceinline__ float2 cell_values(int lay, unsigned cl) const {
+    return KIND == PK_SUBCOL && cl ? *reinterpret_cast<const float2*>(gc + lay * GB_NGPT) : make_float2(0.0f, 0.0f);
+  }
+  // a layer's clear-sky transmittance and source: rtrnmc's odepth <= 0.06
+  // expansion or its table (rtrnmc.f90:380-413); x is odepth/6 or tfn, the
+  // source plfrac * (blay + x * dplank)
+  struct Clear {
+    float2 at, tr, gs;
+    float blay, dpl;  // layer Planck value, that of the level the pass comes to minus it
+  };
+  template <bool UP>
+  __device__ __forceinline__ Clear clear(const Stage& s, int lay) const {
+    Clear c;
+    const float2 q = *reinterpret_cast<const float2*>(&L0[lay].rec[band]);
+    c.blay = q.x;
+    c.dpl = (UP ? q.y : L0[lay - 1].rec[band].y) - q.x;
+    const bool t0 = s.od0 <= 0.06f, t1 = s.od1 <= 0.06f;
+    c.at = make_float2(t0 ? fmaf(-0.5f * s.od0, s.od0, s.od0) : 1.0f - s.e0.x,
+                       t1 ? fmaf(-0.5f * s.od1, s.od1, s.od1) : 1.0f - s.e1.x);
+    const float x0 = t0 ? REC_6 * s.od0 : s.e0.y, x1 = t1 ? REC_6 * s.od1 : s.e1.y;
+    c.gs = mul2(mul2(s.pf, make_float2(fmaf(x0, c.dpl, c.blay), fmaf(x1, c.dpl, c.blay))), c.at);
+    c.tr = make_float2(1.0f - c.at.x, 1.0f - c.at.y);
+    return c;
+  }
+  // the clouds of a layer: A and B of the total radiance's step r' = r A + B,
+  // and D, by which its temperature derivative goes down
+  template <bool UP>
+  __device__ __forceinline__ void cloud(const Stage& s, const Clear& c, int lay, unsigned cl, const float2& cv,
+                                        const float2& r, float2& A, float2& B, float2& D) {
+    const RtLayer& L = L0[lay];
+    float odl = 0.0f, efl = 0.0f;  // cloud optical depth and absorptance of the (layer, band)
+    if (KIND == PK_FUSED) odl = sd * L.rec[band].w;
+    if (BAND) odl = L.rec[cband].w;
+    if (KIND == PK_FUSED || KIND == PK_RANDOM) efl = 1.0f - __expf(-odl);
+    const unsigned frac = KIND == PK_SUBCOL ? reinterpret_cast<const unsigned*>(&L.pad0)[grp] >> l16 : 0u;
+    auto cell = [&](bool cloudy, bool one, float od, float pf, float at, float gs, float tr, float v, float r1, float& A1,
+                    float& B1, float& D1, float& cr1, float& kr1, float& rm1) {
+      if constexpr (BAND) {
+        const float* ov = reinterpret_cast<const float*>(L.cbits);
+        const float cf = ov[0];
+        float atot, x;
+        cloud_total(tt, index(od), od, odl, atot, x);
+        const float bbd = pf * fmaf(x, c.dpl, c.blay);
+        if (UP) D1 = fmaf(cf, 1.0f - atot, (1.0f - cf) * (1.0f - at));
+        if (KIND == PK_RANDOM) {  // rtrn.f90:370-432, 495-507
+          const float efcl = efl * cf;
+          A1 = 1.0f - fmaf(efcl, 1.0f - at, at);
+          B1 = fmaf(cf, fmaf(bbd, atot, -gs), gs);
+        } else {  // rtrnmr.f90:590-609, 688-713
+          constexpr int o = UP ? 1 : 7;
+          if (L.lfl & (UP ? 1 : 2)) {
+            cr1 = cf * r1;
+            kr1 = r1 - cr1;
+            rm1 = 0.0f;
+          }
+          const float ttot = 1.0f - atot, cldsrc = bbd * atot;
+          cr1 = fmaf(cr1, ttot, cf * cldsrc);
+          kr1 = fmaf(kr1, tr, (1.0f - cf) * gs);
+          A1 = 0.0f;
+          B1 = cr1 + kr1;
+          const float radmod = fmaf(rm1, fmaf(ov[o], tr, ov[o + 2] * ttot), fmaf(ov[o + 5], cldsrc, -ov[o + 4] * gs));
+          const float oc = cr1 - radmod, ok = kr1 + radmod;
+          rm1 = fmaf(ov[o + 1], ok, fmaf(-ov[o + 3], oc, -radmod));
+          cr1 += rm1;
+          kr1 -= rm1;
+        }
+      } else {
+        if (!cloudy) return;
+        float odcld = odl, efcl = efl, cldf = 1.0f, atot, x;
+        if (KIND == PK_SUBCOL) cldf = cell_from_value(one, v, sd, odcld, efcl);
+        cloud_total(tt, index(od), od, odcld, atot, x);
+        A1 = 1.0f - fmaf(efcl, 1.0f - at, at);
+        B1 = fmaf(cldf, fmaf(pf * fmaf(x, c.dpl, c.blay), atot, -gs), gs);
+        if (UP) D1 = fmaf(cldf, 1.0f - atot, (1.0f - cldf) * (1.0f - at));
+      }
+    };
+    cell(cl & 1u, !(frac & 1u), s.od0, s.pf.x, c.at.x, c.gs.x, c.tr.x, cv.x, r.x, A.x, B.x, D.x, cr.x, kr.x, radm.x);
+    cell(cl >> 16, !(frac >> 16 & 1u), s.od1, s.pf.y, c.at.y, c.gs.y, c.tr.y, cv.y, r.y, A.y, B.y, D.y, cr.y, kr.y, radm.y);
+  }
+
+  // one layer of the downward pass: total and clear-sky radiance
+  __device__ __forceinline__ void fall(const Stage& s, int lay, unsigned cl, const float2& cv, float2& rd,
+                                       float2& rc) {
+    const Clear c = clear<false>(s, lay);
+    rc = fma2(rc, c.tr, c.gs);
+    float2 A = c.tr, B = c.gs, D;
+    if (cl) cloud<false>(s, c, lay, cl, cv, rd, A, B, D);
+    rd = fma2(rd, A, B);
+  }
+  // one layer of the upward pass: total and clear-sky radiance and their temperature derivatives
+  __device__ __forceinline__ void rise(const Stage& s, int lay, unsigned cl, const float2& cv, float2& ru,
+                                       float2& rc, float2& du, float2& dc) {
+    const Clear c = clear<true>(s, lay);
+    rc = fma2(rc, c.tr, c.gs);
+    dc = mul2(dc, c.tr);
+    float2 A = c.tr, B = c.gs, D = c.tr;
+    if (cl) cloud<true>(s, c, lay, cl, cv, ru, A, B, D);
+    ru = fma2(ru, A, B);
+    du = mul2(du, D);
+  }
+
+  // whether a lane of the warp has a cloud in either of two layers
+  __device__ __forceinline__ bool cloudy(int l0, int l1) const {
+    const unsigned w = BAND ? (unsigned)(L0[l0].cldlay | L0[l1].cldlay) : L0[l0].cbits[grp] | L0[l1].cbits[grp];
+    return __any_sync(0xffffffffu, w != 0u);
+  }
+
+  // ---------------- downward pass (rtrnmc.f90:347-455): total and clear-sky streams; f1: layer 0's fractions
+  __device__ __forceinline__ void down(float2& rd, float2& rc, float2& f1) {
+    const int s4 = sum4_at(l16);
+    float4 pa = gas(nl - 1), pb = gas(max(nl - 2, 0));
+    Stage sa = stage(nl - 1, pa), sb = stage(max(nl - 2, 0), pb);
+    pa = gas(max(nl - 3, 0)), pb = gas(max(nl - 4, 0));
+    int lay = nl - 1;
+#pragma unroll 1
+    for (; lay >= 1; lay -= 2) {
+      f1 = sb.pf;
+      float2 p0, p1;
+      if (cloudy(lay, lay - 1)) {
+        const unsigned c0 = bits(lay), c1 = bits(lay - 1);
+        const float2 v0 = cell_values(lay, c0), v1 = cell_values(lay - 1, c1);
+        fall(sa, lay, c0, v0, rd, rc);
+        p0 = mul2(rd, wgt), p1 = mul2(rc, wgt);
+        fall(sb, lay - 1, c1, v1, rd, rc);
+        sa = stage(max(lay - 2, 0), pa), sb = stage(max(lay - 3, 0), pb);
+        pa = gas(max(lay - 4, 0)), pb = gas(max(lay - 5, 0));
+        const float s = sum4(p0, p1, mul2(rd, wgt), mul2(rc, wgt), l16);
+        if (lw < 4) part[(lay - (s4 >> 1)) * 6 + (s4 & 1)] = s;
+      } else {
+        const Clear c0 = clear<false>(sa, lay), c1 = clear<false>(sb, lay - 1);
+        sa = stage(max(lay - 2, 0), pa), sb = stage(max(lay - 3, 0), pb);
+        pa = gas(max(lay - 4, 0)), pb = gas(max(lay - 5, 0));
+        rd = fma2(rd, c0.tr, c0.gs), rc = fma2(rc, c0.tr, c0.gs);
+        p0 = mul2(rd, wgt), p1 = mul2(rc, wgt);
+        rd = fma2(rd, c1.tr, c1.gs), rc = fma2(rc, c1.tr, c1.gs);
+        const float s = sum4(p0, p1, mul2(rd, wgt), mul2(rc, wgt), l16);
+        if (lw < 4) part[(lay - (s4 >> 1)) * 6 + (s4 & 1)] = s;
+      }
+    }
+    if (lay == 0) {  // layer 0 on its own
+      f1 = sa.pf;
+      fall(sa, 0, bits(0), cell_values(0, bits(0)), rd, rc);
+      const float s = sum2(mul2(rd, wgt), mul2(rc, wgt), l16);
+      if (lw < 2) part[l16] = s;
+    }
+  }
+
+  // ---------------- upward pass (rtrnmc.f90:486-529): level lay+1 above layer lay
+  template <bool IDRV>
+  __device__ __forceinline__ void up(float2& ru, float2& rc, float2& du, float2& dc) {
+    const int s4 = sum4_at(l16), s8 = sum8_at(l16), top = nl - 1;
+    auto put1 = [&](float* p) {
+      if (IDRV) {
+        const float s = sum4(mul2(ru, wgt), mul2(rc, wgt), mul2(du, wgt), mul2(dc, wgt), l16);
+        if (lw < 4) p[s4] = s;
+      } else {
+        const float s = sum2(mul2(ru, wgt), mul2(rc, wgt), l16);
+        if (lw < 2) p[l16] = s;
+      }
+    };
+    float2 q0, q1, q2, q3;
+    auto put2 = [&](int lay) {
+      float* p = part + (lay + 1) * 6 + 2;  // levels lay+1 and lay+2
+      if (IDRV) {
+        const float s = sum8(q0, q1, q2, q3, mul2(ru, wgt), mul2(rc, wgt), mul2(du, wgt), mul2(dc, wgt), l16);
+        if (lw < 8) p[(s8 >> 2) * 6 + (s8 & 3)] = s;
+      } else {
+        const float s = sum4(q0, q1, mul2(ru, wgt), mul2(rc, wgt), l16);
+        if (lw < 4) p[(s4 >> 1) * 6 + (s4 & 1)] = s;
+      }
+    };
+    put1(part + 2);
+    float4 pa = gas(0), pb = gas(min(1, top));
+    Stage sa = stage(0, pa), sb = stage(min(1, top), pb);
+    pa = gas(min(2, top)), pb = gas(min(3, top));
+    int lay = 0;
+#pragma unroll 1
+    for (; lay + 1 < nl; lay += 2) {
+      if (cloudy(lay, lay + 1)) {
+        const unsigned c0 = bits(lay), c1 = bits(lay + 1);
+        const float2 v0 = cell_values(lay, c0), v1 = cell_values(lay + 1, c1);
+        rise(sa, lay, c0, v0, ru, rc, du, dc);
+        q0 = mul2(ru, wgt), q1 = mul2(rc, wgt), q2 = mul2(du, wgt), q3 = mul2(dc, wgt);
+        rise(sb, lay + 1, c1, v1, ru, rc, du, dc);
+        sa = stage(min(lay + 2, top), pa), sb = stage(min(lay + 3, top), pb);
+        pa = gas(min(lay + 4, top)), pb = gas(min(lay + 5, top));
+        put2(lay);
+      } else {
+        const Clear c0 = clear<true>(sa, lay), c1 = clear<true>(sb, lay + 1);
+        sa = stage(min(lay + 2, top), pa), sb = stage(min(lay + 3, top), pb);
+        pa = gas(min(lay + 4, top)), pb = gas(min(lay + 5, top));
+        ru = fma2(ru, c0.tr, c0.gs), rc = fma2(rc, c0.tr, c0.gs), du = mul2(du, c0.tr), dc = mul2(dc, c0.tr);
+        q0 = mul2(ru, wgt), q1 = mul2(rc, wgt), q2 = mul2(du, wgt), q3 = mul2(dc, wgt);
+        ru = fma2(ru, c1.tr, c1.gs), rc = fma2(rc, c1.tr, c1.gs), du = mul2(du, c1.tr), dc = mul2(dc, c1.tr);
+        put2(lay);
+      }
+    }
+    if (lay < nl) {  // level nl on its own
+      rise(sa, lay, bits(lay), cell_values(lay, bits(lay)), ru, rc, du, dc);
+      put1(part + nl * 6 + 2);
+    }
+  }
+};
+
+template <int MODE, int KIND>
+__device__ __forceinline__ void rt_passes(const LwArgs& a, const RtSmem& S, const GasSrc& src,
+                                          const float2* tt, int band, int g, int po, int grp, int l16, bool inblk,
+                                          float wgt) {
+  const float2 zero = make_float2(0.0f, 0.0f);
+  const int nl = a.nlay;
+  Passes<MODE, KIND> P{src, S.L, tt,
+                       KIND == PK_SUBCOL ? src.gc + g : nullptr, S.part + grp * (nl + 1) * 6, S.h->misc[band],
+                       make_float2(wgt, wgt), nl, band, KIND >= PK_RANDOM ? cloud_band(S.h->iscal[2], band) : band, g, po,
+                       grp, l16, inblk ? l16 : 16, zero, zero, zero};
+  float2 rd = zero, rc = zero, f1 = zero;
+  P.down(rd, rc, f1);
+  // surface emission and reflection (rtrnmc.f90:465-485)
+  const float2 rad0 = make_float2(f1.x * S.h->misc[16 + band], f1.y * S.h->misc[16 + band]);
+  const float reflect = 1.0f - S.h->misc[48 + band];  // scalar: the assembler fuses a packed product and sum
+  float2 ru = make_float2(rad0.x + reflect * rd.x, rad0.y + reflect * rd.y);
+  float2 rcu = make_float2(rad0.x + reflect * rc.x, rad0.y + reflect * rc.y);
+  float2 du = make_float2(f1.x * S.h->misc[32 + band], f1.y * S.h->misc[32 + band]);
+  float2 dcu = du;
+  if (a.idrv == 1)
+    P.template up<true>(ru, rcu, du, dcu);
+  else
+    P.template up<false>(ru, rcu, du, dcu);
+}
+
+// The transfer of a unit's columns (see the file header); src is that of this
+// thread's column.  RT_NET: a column with any layer off the network is not
+// solved; returns whether this thread's column was solved.  BAND: the non-McICA
+// driver's band clouds (random overlap for icld 1, maximum/random otherwise).
+// Ends with a barrier.
 template <int MODE, bool BAND = false>
-__device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, const GasSrc& src,
-                          const float* __restrict__ T) {
+__device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const Cols& C, const GasSrc& src,
+                           const float* __restrict__ T) {
+  constexpr bool NET = MODE == RT_NET || MODE == RT_NETODD;
   const unsigned FULL = 0xffffffffu;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = U.tid, lane = tid & 31, warp = tid >> 5, nt = U.nt;
   const int nl = a.nlay;
   const bool fused = a.cloud_mode == LW_CLOUD_FUSED;
   const bool clouds = a.icld >= 1;
-  if (MODE == RT_NET) {
-    int off = src.flag == nullptr;
-    for (int l = tid; l < nl && !off; l += RT_NT) off = src.flag[l] == 0;
-    if (__syncthreads_or(off)) return false;
+  // this thread's column (threads past the unit's columns go along with the last one and write nothing),
+  // group of 32 g-points, lane in the group's 16, and pair of g-points (the last group has 6 live pairs)
+  const int half = tid / RT_CT;
+  const bool inblk = half < C.n;
+  const int col = inblk ? half : C.n - 1;
+  const int t = tid - half * RT_CT, grp = t >> 4, l16 = t & 15;
+  const RtSmem S = C.S(col);
+  const long long icol = C.icol(col);
+  bool act = inblk && C.col0 + col <= C.last;
+  if (tid < 4 * C.n) C.S(tid >> 2).h->iscal[tid & 3] = 0;
+  if (NET) {
+    U.sync();
+    int off = 0;
+    for (int l = t; l < nl && inblk; l += RT_CT) off |= src.flag[l] == 0;
+    if (off) S.h->iscal[2] = 1;
+    U.sync();
+    act = act && S.h->iscal[2] == 0;
+    if (C.S(0).h->iscal[2] != 0 && (C.n == 1 || C.col0 + 1 > C.last || C.S(1).h->iscal[2] != 0)) return false;
   }
-  if (tid < 4) S.h->iscal[tid] = 0;
-  // this thread's g-point, its band and flux weight (read from the table blob:
-  // a constant-bank lookup indexed by the thread would be re-issued in the
-  // loops wherever the compiler does not keep the value in a register)
-  const bool live = tid < GB_NGPT;
-  const int g = live ? tid : GB_NGPT - 1;
+  // this thread's g-points and their band (read from the table blob: a
+  // constant-bank lookup indexed by the thread would be re-issued in the loops
+  // wherever the compiler does not keep the value in a register)
+  const bool live = inblk && t < GB_NGPT / 2;
+  const int g = live ? 2 * t : GB_NGPT - 2;
   const int band = __float_as_int(__ldg(T + c_T.gpt_band + g));
-  const float wgt = live ? __ldg(T + c_T.gpt_wgt + g) : 0.0f;
   const int po = plane_pos(band + 1, g - c_T.band[band].g0);
-  __syncthreads();
+  U.sync();
 
   // ---------------- per layer: inatm's column amounts (pwvcm), value checks, laytrop, Planck rows
   const float amd = 28.9660f, amw = 18.0160f;
-  float amttl = 0.0f, wvttl = 0.0f;
-  int bad = 0;
-  float4* prow = reinterpret_cast<float4*>(S.part);
-  for (int lay = tid; lay < nl; lay += RT_NT) {
-    const double pd = in2(a.play, a.ld, icol, lay);
-    const float pavel = (float)pd;
-    const float tavel = (float)in2(a.tlay, a.ld, icol, lay);
-    const double dpz = in2(a.plev, a.ld, icol, lay) - in2(a.plev, a.ld, icol, lay + 1);
-    const float w1 = (float)in2(a.h2ovmr, a.ld, icol, lay);
-    const float tz = (float)in2(a.tlev, a.ld, icol, lay);
-    const float amm = (1.0f - w1) * amd + w1 * amw;
-    const float coldry = (float)dpz * 1.e3f * (float)c_T.avogad / (1.e2f * (float)c_T.grav * amm * (1.0f + w1));
-    const float wk1 = coldry * w1;
-    amttl += coldry + wk1;
-    wvttl += wk1;
-    if (!(pavel > 0.0f) || !(tavel > 0.0f) || !isfinite(pavel) || !isfinite(tavel)) bad = 1;
-    const bool lower = lower_atmosphere(pd, __logf(pavel));
-    S.L[lay].cldlay = lower;
-    if (lower) atomicAdd(&S.h->iscal[1], 1);
-    // Planck-table rows of the level below and of the layer (setcoef.f90:173-269)
-    const int ind = clampi((int)(tz - 159.0f), 1, 180);
-    const int il = clampi((int)(tavel - 159.0f), 1, 180);
-    prow[lay] = make_float4(__int_as_float(ind), tz - 159.0f - (float)ind, __int_as_float(il), tavel - 159.0f - (float)il);
-    if (lay == nl - 1) {
-      const float tt = (float)in2(a.tlev, a.ld, icol, nl);
-      const int it = clampi((int)(tt - 159.0f), 1, 180);
-      prow[nl] = make_float4(__int_as_float(it), tt - 159.0f - (float)it, 0.0f, 0.0f);
+  const int nvw = min(RT_NW, (nl + 31) >> 5);  // sums of 32 layers each (layers 160 apart in one lane)
+  for (int i = warp; i < C.n * nvw; i += nt >> 5) {
+    const int c = C.c(i), vw = C.rest(i);
+    const RtSmem Sc = C.S(c);
+    const long long ic = C.icol(c);
+    float4* prow = Sc.prow;
+    float amttl = 0.0f, wvttl = 0.0f;
+    int bad = 0;
+    for (int lay = vw * 32 + lane; lay < nl; lay += RT_NT) {
+      const double pd = in2(a.play, a.ld, ic, lay);
+      const float pavel = (float)pd;
+      const float tavel = (float)in2(a.tlay, a.ld, ic, lay);
+      const double dpz = in2(a.plev, a.ld, ic, lay) - in2(a.plev, a.ld, ic, lay + 1);
+      const float w1 = (float)in2(a.h2ovmr, a.ld, ic, lay);
+      const float tz = (float)in2(a.tlev, a.ld, ic, lay);
+      const float amm = (1.0f - w1) * amd + w1 * amw;
+      const float coldry = (float)dpz * 1.e3f * (float)c_T.avogad / (1.e2f * (float)c_T.grav * amm * (1.0f + w1));
+      const float wk1 = coldry * w1;
+      amttl += coldry + wk1;
+      wvttl += wk1;
+      if (!(pavel > 0.0f) || !(tavel > 0.0f) || !isfinite(pavel) || !isfinite(tavel)) bad = 1;
+      const bool lower = lower_atmosphere(pd, __logf(pavel));
+      Sc.L[lay].cldlay = lower;
+      if (lower) atomicAdd(&Sc.h->iscal[1], 1);
+      // Planck-table rows of the level below and of the layer (setcoef.f90:173-269)
+      const int ind = clampi((int)(tz - 159.0f), 1, 180);
+      const int il = clampi((int)(tavel - 159.0f), 1, 180);
+      prow[lay] = make_float4(__int_as_float(ind), tz - 159.0f - (float)ind, __int_as_float(il), tavel - 159.0f - (float)il);
+      if (lay == nl - 1) {
+        const float tt = (float)in2(a.tlev, a.ld, ic, nl);
+        const int it = clampi((int)(tt - 159.0f), 1, 180);
+        prow[nl] = make_float4(__int_as_float(it), tt - 159.0f - (float)it, 0.0f, 0.0f);
+      }
     }
-  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {  // fixed-order sums: within the warp, then over the warps in order
-    amttl += __shfl_xor_sync(FULL, amttl, o);
-    wvttl += __shfl_xor_sync(FULL, wvttl, o);
+    for (int o = 16; o > 0; o >>= 1) {  // fixed-order sums: 32 layers, then these in order
+      amttl += __shfl_xor_sync(FULL, amttl, o);
+      wvttl += __shfl_xor_sync(FULL, wvttl, o);
+    }
+    if (lane == 0) {
+      Sc.h->red[2 * vw] = amttl;
+      Sc.h->red[2 * vw + 1] = wvttl;
+    }
+    if (bad) atomicOr(&Sc.h->iscal[3], 1);
   }
-  if (lane == 0) {
-    S.h->red[2 * warp] = amttl;
-    S.h->red[2 * warp + 1] = wvttl;
-  }
-  bad = __syncthreads_or(bad);
+  U.sync();
   // lower-atmosphere layers must form the prefix 0 .. laytrop-1
-  const int laytrop = S.h->iscal[1];
-  int notpre = 0;
-  for (int lay = tid; lay < nl; lay += RT_NT) notpre |= S.L[lay].cldlay != (lay < laytrop ? 1 : 0);
-  if (tid < 16) {
+  for (int i = tid; i < C.n * nl; i += nt) {
+    const RtSmem Sc = C.S(C.c(i));
+    const int lay = C.rest(i);
+    if (Sc.L[lay].cldlay != (lay < Sc.h->iscal[1] ? 1 : 0)) atomicOr(&Sc.h->iscal[3], 2);
+  }
+  if (tid < 16 * C.n) {
     // pwvcm (inatm :869-870) and secdiff (rtrnmc.f90:258-266), one band per thread
-    const int ib = tid;
-    float at = S.h->red[0], wt = S.h->red[1];
-    for (int w = 1; w < RT_NW; ++w) {
-      at += S.h->red[2 * w];
-      wt += S.h->red[2 * w + 1];
+    const int ib = C.rest(tid);
+    const RtSmem Sc = C.S(C.c(tid));
+    const long long ic = C.icol(C.c(tid));
+    float at = Sc.h->red[0], wt = Sc.h->red[1];
+    for (int w = 1; w < nvw; ++w) {
+      at += Sc.h->red[2 * w];
+      wt += Sc.h->red[2 * w + 1];
     }
     const float wvsh = (amw * wt) / (amd * at);
-    const float pz0 = (float)in2(a.plev, a.ld, icol, 0);
+    const float pz0 = (float)in2(a.plev, a.ld, ic, 0);
     const float pwvcm = wvsh * (1.e3f * pz0) / (1.e2f * (float)c_T.grav);
     float sd = 1.66f;
     if (!(ib == 0 || ib == 3 || ib >= 9)) {
       sd = c_a0[ib] + c_a1[ib] * __expf(c_a2[ib] * pwvcm);
       sd = fminf(fmaxf(sd, 1.50f), 1.80f);
     }
-    S.h->misc[ib] = sd;
+    Sc.h->misc[ib] = sd;
     // surface source and its temperature derivative (setcoef.f90:270-282)
-    const float tb = (float)__ldg(a.tsfc + icol);
+    const float tb = (float)__ldg(a.tsfc + ic);
     const int ind = clampi((int)(tb - 159.0f), 1, 180);
     const float fr = tb - 159.0f - (float)ind;
-    const float se = (float)__ldg(a.emis + icol + a.ld * ib);
+    const float se = (float)__ldg(a.emis + ic + a.ld * ib);
     const float* tp = T + c_T.totplnk + ib * 181;
     const float* td = T + c_T.totplnkderiv + ib * 181;
-    S.h->misc[16 + ib] = se * (tp[ind - 1] + fr * (tp[ind] - tp[ind - 1]));
-    S.h->misc[32 + ib] = se * (td[ind - 1] + fr * (td[ind] - td[ind - 1]));
-    S.h->misc[48 + ib] = se;
+    Sc.h->misc[16 + ib] = se * (tp[ind - 1] + fr * (tp[ind] - tp[ind - 1]));
+    Sc.h->misc[32 + ib] = se * (td[ind - 1] + fr * (td[ind] - td[ind - 1]));
+    Sc.h->misc[48 + ib] = se;
   }
-  notpre = __syncthreads_or(notpre);
+  U.sync();
   // ---------------- per (layer, band): Planck values and the aerosol optical depth (rrtmg_lw_rad.f90:548-553)
 #pragma unroll 2
-  for (int it = tid; it < nl * 16; it += RT_NT) {
-    const int lay = it >> 4, ib = it & 15;
+  for (int i = tid; i < C.n * nl * 16; i += nt) {
+    const int lay = C.rest(i) >> 4, ib = C.rest(i) & 15;
+    const RtSmem Sc = C.S(C.c(i));
+    const float4* prow = Sc.prow;
     const float* tp = T + c_T.totplnk + ib * 181;
     const float4 r0 = prow[lay], r1 = prow[lay + 1];
     const int i0 = __float_as_int(r0.x), il = __float_as_int(r0.z), i1 = __float_as_int(r1.x);
     const float pdn = tp[i0 - 1] + r0.y * (tp[i0] - tp[i0 - 1]);
     const float pup = tp[i1 - 1] + r1.y * (tp[i1] - tp[i1 - 1]);
     const float blay = tp[il - 1] + r0.w * (tp[il] - tp[il - 1]);
-    const float taua = (float)__ldg(a.tauaer + icol + a.ld * (lay + (long long)nl * ib));
-    S.L[lay].rec[ib] = make_float4(blay, pdn - blay, pup - blay, taua);
+    const float taua = (float)__ldg(a.tauaer + C.icol(C.c(i)) + a.ld * (lay + (long long)nl * ib));
+    float4& r = Sc.L[lay].rec[ib];  // its w is the clouds'
+    *reinterpret_cast<float2*>(&r) = make_float2(blay, pup);
+    r.z = taua;
+    if (lay == 0) Sc.L[-1].rec[ib].y = pdn;
   }
   // ---------------- clouds: the cells' McICA bits, cldprmc's optical depths and stop conditions
-  int err = 0;
   if constexpr (BAND) {
-    band_clouds(a, icol, S, nl, clouds);
+    band_clouds(a, U, C, nl, clouds);
   } else {
-  for (int i = tid; i < nl * 5; i += RT_NT) {
-    const int l = i / 5, w = i - 5 * l;
-    S.L[l].cbits[w] = 0u;
-    S.fbits(l)[w] = 0u;  // caller sub-columns
+  for (int i = tid; i < C.n * nl * 5; i += nt) {
+    const int r = C.rest(i), l = r / 5, w = r - 5 * l;
+    const RtSmem Sc = C.S(C.c(i));
+    Sc.L[l].cbits[w] = 0u;
   }
+  // a group's word of a layer from the ballots over the low and the high g-points of its pairs
+  auto word = [&](unsigned lo, unsigned hi) {
+    return lane < 16 ? (lo & 0xffffu) | (hi << 16) : (lo >> 16) | (hi & 0xffff0000u);
+  };
   if (clouds && fused) {
     // per layer, once: the McICA threshold and the layer's cloud quantities
-    for (int lay = tid; lay < nl; lay += RT_NT) {
-      double cf = in2(a.cldfrac, a.ld, icol, lay);
-      cf = cf < 1.0e-20 ? 0.0 : cf;  // mcica_subcol_gen_lw.f90:463-470
-      // cdf >= 1 - cf, compared on the bit patterns (cdf is in [0, 1], so
+    for (int i = tid; i < C.n * nl; i += nt) {
+      const int lay = C.rest(i);
+      const RtSmem Sc = C.S(C.c(i));
+      const long long ic = C.icol(C.c(i));
+      double cf = in2(a.cldfrac, a.ld, ic, lay);
+      if (cf < 1.0e-20) cf = 0.0;
+      // draws are in [0, 1], so cdf >= 1 - cldf compares the bit patterns (and
       // for a threshold >= 0 the integer order is the floating-point order);
       // a negative threshold takes every cell, a NaN none
       const double thr = 1.0 - cf;
-      S.L[lay].cthr = thr < 0.0 ? LLONG_MIN : (thr == thr ? __double_as_longlong(thr) : LLONG_MAX);
-      const double ciwp = in2(a.ciwp, a.ld, icol, lay), clwp = in2(a.clwp, a.ld, icol, lay);
-      const double rice = in2(a.reicmcl, a.ld, icol, lay), rliq = in2(a.relqmcl, a.ld, icol, lay);
+      Sc.L[lay].cthr = thr < 0.0 ? LLONG_MIN : (thr == thr ? __double_as_longlong(thr) : LLONG_MAX);
+      const double ciwp = in2(a.ciwp, a.ld, ic, lay), clwp = in2(a.clwp, a.ld, ic, lay);
+      const double rice = in2(a.reicmcl, a.ld, ic, lay), rliq = in2(a.relqmcl, a.ld, ic, lay);
       const int fl = (ciwp != 0.0 ? 1 : 0) | (clwp != 0.0 ? 2 : 0) | (ciwp + clwp >= 1.e-20 ? 4 : 0);
       int e = 0;
       if (ciwp != 0.0) e = ice_code(a.iceflag, rice);
       if (clwp != 0.0 && liq_code(a.liqflag, rliq)) e = GB_COL_LIQ_BOUNDS;
-      S.L[lay].lfl = fl | (e << 8);
-      S.L[lay].lcw = make_float4((float)ciwp, (float)clwp, (float)rice, (float)rliq);
+      Sc.L[lay].lfl = fl | (e << 8);
+      Sc.L[lay].lcw = make_float4((float)ciwp, (float)clwp, (float)rice, (float)rliq);
     }
-    // this g-point's draw (mcica_subcol_gen_lw.f90:484-512, icld 3) as a bit
-    // pattern, and the warp's largest
-    const long long cdb = __double_as_longlong(__ldg(a.draws + icol * GB_NGPT + g));
-    long long mx = live ? cdb : LLONG_MIN;
+    // these g-points' draws (mcica_subcol_gen_lw.f90:484-512, icld 3) as bit
+    // patterns, and the warp's largest
+    const double2 dr = __ldg(reinterpret_cast<const double2*>(a.draws + icol * GB_NGPT + g));
+    const long long d0 = __double_as_longlong(dr.x), d1 = __double_as_longlong(dr.y);
+    long long mx = live ? (d0 > d1 ? d0 : d1) : LLONG_MIN;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 8; o > 0; o >>= 1) {
       const long long v = __shfl_xor_sync(FULL, mx, o);
       mx = v > mx ? v : mx;
     }
-    __syncthreads();
+    U.sync();
     // cloudy cells: cdf(g) >= 1 - cldf(lay) (mcica_subcol_gen_lw.f90:650); a
     // layer whose threshold is above every draw of the warp has none there
     for (int lay = 0; lay < nl; ++lay) {
       const long long tb = S.L[lay].cthr;
-      if (tb > mx) continue;
-      const unsigned m = __ballot_sync(FULL, live && cdb >= tb);
-      if (lane == 0) S.L[lay].cbits[warp] = m;
+      if (__all_sync(FULL, tb > mx)) continue;
+      const unsigned m0 = __ballot_sync(FULL, live && d0 >= tb), m1 = __ballot_sync(FULL, live && d1 >= tb);
+      if (l16 == 0 && inblk) S.L[lay].cbits[grp] = word(m0, m1);
     }
-    __syncthreads();
-    for (int lay = tid; lay < nl; lay += RT_NT) {
-      const unsigned* c = S.L[lay].cbits;
-      S.L[lay].cldlay = (c[0] | c[1] | c[2] | c[3] | c[4]) != 0u;
+    U.sync();
+    for (int i = tid; i < C.n * nl; i += nt) {
+      const RtSmem Sc = C.S(C.c(i));
+      const unsigned* c = Sc.L[C.rest(i)].cbits;
+      Sc.L[C.rest(i)].cldlay = (c[0] | c[1] | c[2] | c[3] | c[4]) != 0u;
     }
-    __syncthreads();
+    U.sync();
     // cloud optical depth per (layer, band) where the band has a cloudy
     // sub-column (the values cldprmc computes for every such cell), and
-    // cldprmc's stop conditions
+    // cldprmc's stop conditions (of several in a column the one that 160
+    // threads, each going up the column, would be left with)
     const long long kMin = __double_as_longlong(1.0e-20), kInf = 0x7FF0000000000000LL;
-    for (int it = tid; it < nl * 16; it += RT_NT) {
-      const int lay = it >> 4, ib = it & 15;
-      if (!S.L[lay].cldlay) continue;
-      const int g0 = c_T.band[ib].g0, ng = c_T.band[ib].ng;
-      bool any = false;
-      for (int k = g0; k < g0 + ng; ++k) any |= (S.L[lay].cbits[k >> 5] >> (k & 31)) & 1u;
-      if (!any) continue;
-      const double tin = __ldg(a.tauc + ib + 16 * (icol + a.ld * lay));
-      const long long tinb = __double_as_longlong(tin);
-      const bool tin_ok = tinb >= kMin && tinb <= kInf;  // tin >= 1e-20
-      const int fl = S.L[lay].lfl;
-      const bool cond = (fl & 4) || tin_ok;
-      S.L[lay].tcl[ib] = a.inflag == 2 && cond ? cloud_tau_layer(a, ib, T, S.L[lay].lcw, fl) : (float)tin;
-      if (cond) {
-        if (a.inflag == 1) err = GB_COL_INFLAG1;
-        if (a.inflag == 2 && (fl >> 8)) err = fl >> 8;
+    for (int v = tid; v < C.n * RT_NT; v += nt) {
+      const RtSmem Sc = C.S(C.c(v));
+      const long long ic = C.icol(C.c(v));
+      int err = 0;
+      for (int it = C.rest(v); it < nl * 16; it += RT_NT) {
+        const int lay = it >> 4, ib = it & 15;
+        if (!Sc.L[lay].cldlay) continue;
+        const int p0 = c_T.band[ib].g0 >> 1, np = c_T.band[ib].ng >> 1;
+        bool any = false;
+        for (int k = p0; k < p0 + np; ++k) {
+          const unsigned w = Sc.L[lay].cbits[k >> 4];
+          any |= ((w | w >> 16) >> (k & 15)) & 1u;
+        }
+        if (!any) continue;
+        const double tin = __ldg(a.tauc + ib + 16 * (ic + a.ld * lay));
+        const long long tinb = __double_as_longlong(tin);
+        const bool tin_ok = tinb >= kMin && tinb <= kInf;  // tin >= 1e-20
+        const int fl = Sc.L[lay].lfl;
+        const bool cond = (fl & 4) || tin_ok;
+        Sc.L[lay].rec[ib].w = a.inflag == 2 && cond ? cloud_tau_layer(a, ib, T, Sc.L[lay].lcw, fl) : (float)tin;
+        if (cond) {
+          if (a.inflag == 1) err = GB_COL_INFLAG1;
+          if (a.inflag == 2 && (fl >> 8)) err = fl >> 8;
+        }
       }
+      if (err) atomicMax(&Sc.h->iscal[0], err);
     }
   } else if (clouds) {
     // caller sub-columns: the layer radii as floats and the codes cldprmc's
     // radius checks stop with: bits 0-7 ice, 8-15 liquid
-    for (int lay = tid; lay < nl; lay += RT_NT) {
-      const double rice = in2(a.reicmcl, a.ld, icol, lay), rliq = in2(a.relqmcl, a.ld, icol, lay);
-      S.L[lay].lfl = ice_code(a.iceflag, rice) | (liq_code(a.liqflag, rliq) << 8);
-      S.L[lay].lcw = make_float4(0.0f, 0.0f, (float)rice, (float)rliq);
+    for (int i = tid; i < C.n * nl; i += nt) {
+      const int lay = C.rest(i);
+      const RtSmem Sc = C.S(C.c(i));
+      const long long ic = C.icol(C.c(i));
+      const double rice = in2(a.reicmcl, a.ld, ic, lay), rliq = in2(a.relqmcl, a.ld, ic, lay);
+      Sc.L[lay].lfl = ice_code(a.iceflag, rice) | (liq_code(a.liqflag, rliq) << 8);
+      Sc.L[lay].lcw = make_float4(0.0f, 0.0f, (float)rice, (float)rliq);
     }
-    __syncthreads();
-    // per layer, each warp: its 32 cldfmcl values tested on their bit
-    // patterns: == 1, /= 0, >= 1e-20
+    U.sync();
+    // per layer, each group: its 32 cldfmcl values tested on their bit
+    // patterns: == 1, /= 0, >= 1e-20.  A pair is one 16-byte load where the
+    // caller's arrays start on such a boundary (rows are 1,120 bytes).
     const long long kOne = 0x3FF0000000000000LL, kInf = 0x7FF0000000000000LL;
     const long long kMin = __double_as_longlong(1.0e-20);
+    const bool wide = (((uintptr_t)a.cldfmcl | (uintptr_t)a.ciwpmcl | (uintptr_t)a.clwpmcl | (uintptr_t)a.taucmcl) & 15) == 0;
+    auto pair = [&](const double* p, long long o) {
+      return wide ? __ldg(reinterpret_cast<const double2*>(p + o)) : make_double2(__ldg(p + o), __ldg(p + o + 1));
+    };
 #pragma unroll 8
     for (int lay = 0; lay < nl; ++lay) {
-      const long long o = g + GB_NGPT * (icol + a.ld * lay);
-      const long long cb = live ? __double_as_longlong(__ldg(a.cldfmcl + o)) : 0LL;
-      const bool one = cb == kOne;
-      const bool frac = !one && (cb << 1) != 0LL;  // neither +-0 nor 1 (NaN included, as /= 0 is)
-      const unsigned m1 = __ballot_sync(FULL, one), mf = __ballot_sync(FULL, frac);
-      if (lane == 0) {
-        S.L[lay].cbits[warp] = m1;
-        S.fbits(lay)[warp] = mf;
+      const double2 cf = pair(a.cldfmcl, g + GB_NGPT * (icol + a.ld * lay));
+      const long long b0 = live ? __double_as_longlong(cf.x) : 0LL, b1 = live ? __double_as_longlong(cf.y) : 0LL;
+      const bool one0 = b0 == kOne, one1 = b1 == kOne;
+      const bool fr0 = !one0 && (b0 << 1) != 0LL, fr1 = !one1 && (b1 << 1) != 0LL;  // neither +-0 nor 1 (NaN included, as /= 0 is)
+      const unsigned m0 = __ballot_sync(FULL, one0), m1 = __ballot_sync(FULL, one1);
+      const unsigned f0 = __ballot_sync(FULL, fr0), f1 = __ballot_sync(FULL, fr1);
+      if (l16 == 0 && inblk) {
+        S.L[lay].cbits[grp] = word(m0, m1);
+        S.fbits(lay)[grp] = word(f0, f1);
       }
     }
     __syncwarp();
-    // then, per cell with a cloud (independent iterations, so that several
-    // cells' loads are in flight): the water paths for cldprmc's checks and,
-    // where the transfer has a cloud plane, the cell's optical depth formed
-    // once instead of in both passes
-    const unsigned mybit = 1u << lane;
+    // then, per pair with a cloud (independent iterations, so that several
+    // pairs' loads are in flight): the water paths for cldprmc's checks and
+    // the cells' optical depths, formed once instead of in both passes
+    int err0 = 0, err1 = 0;
 #pragma unroll 4
     for (int lay = 0; lay < nl; ++lay) {
-      const bool one = S.L[lay].cbits[warp] & mybit, frac = S.fbits(lay)[warp] & mybit;
-      if (!(one || frac)) continue;
+      const unsigned ob = S.L[lay].cbits[grp] >> l16, fb = S.fbits(lay)[grp] >> l16;
+      if (!live || !((ob | fb) & 0x10001u)) continue;
       const long long o = g + GB_NGPT * (icol + a.ld * lay);
-      const double cfv = one ? 1.0 : __ldg(a.cldfmcl + o);
-      const long long cb = __double_as_longlong(cfv);
-      if (cb >= kMin && cb <= kInf) {  // cldfmc >= cldmin (cldprmc.f90:178)
-        const double ciwp = __ldg(a.ciwpmcl + o), clwp = __ldg(a.clwpmcl + o);
-        const double tin = __ldg(a.taucmcl + o);
-        if (src.gc) src.gc[lay * GB_NGPT + g] = cell_value(a, S, lay, band, one, cfv, ciwp, clwp, tin, T);
+      const double2 cf = fb & 0x10001u ? pair(a.cldfmcl, o) : make_double2(ob & 1u, ob >> 16 & 1u);
+      const double2 ci = pair(a.ciwpmcl, o), cl = pair(a.clwpmcl, o), ti = pair(a.taucmcl, o);
+      auto cell = [&](bool one, bool cloudy, double cfv, double ciwp, double clwp, double tin, int& err) {
+        if (!cloudy) return 0.0f;
+        const long long cb = __double_as_longlong(cfv);
+        if (!(cb >= kMin && cb <= kInf)) return (float)cfv;  // a fraction below cldmin: cldfmcl itself, no cloud optics
+        const float v = cell_value(a, S, lay, band, one, cfv, ciwp, clwp, tin, T);  // cldfmc >= cldmin (cldprmc.f90:178)
         const long long tb = __double_as_longlong(tin);
         if (ciwp + clwp >= 1.e-20 || (tb >= kMin && tb <= kInf)) {
           const int e = S.L[lay].lfl;
@@ -937,25 +1296,30 @@ __device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, cons
             if ((__double_as_longlong(clwp) << 1) != 0LL && (e >> 8)) err = e >> 8;      // clwp /= 0
           }
         }
-      } else if (src.gc) {
-        src.gc[lay * GB_NGPT + g] = (float)cfv;  // a fraction below cldmin: cldfmcl itself, no cloud optics
-      }
+        return v;
+      };
+      const float v0 = cell(ob & 1u, (ob | fb) & 1u, cf.x, ci.x, cl.x, ti.x, err0);
+      const float v1 = cell(ob >> 16 & 1u, (ob | fb) >> 16 & 1u, cf.y, ci.y, cl.y, ti.y, err1);
+      *reinterpret_cast<float2*>(src.gc + lay * GB_NGPT + g) = make_float2(v0, v1);
     }
-    __syncthreads();
-    for (int lay = tid; lay < nl; lay += RT_NT) {
-      const unsigned* c = S.L[lay].cbits;
-      S.L[lay].cldlay = (c[0] | c[1] | c[2] | c[3] | c[4]) != 0u;
+    if (err0 || err1) atomicMax(&S.h->iscal[0], max(err0, err1));
+    U.sync();
+    for (int i = tid; i < C.n * nl; i += nt) {
+      const RtSmem Sc = C.S(C.c(i));
+      unsigned* c = Sc.L[C.rest(i)].cbits;
+      const unsigned* f = Sc.fbits(C.rest(i));
+      const bool any = (c[0] | c[1] | c[2] | c[3] | c[4]) != 0u;
+      for (int w = 0; w < RT_NW; ++w) c[w] = any ? c[w] | f[w] : 0u;
     }
   } else {
-    for (int lay = tid; lay < nl; lay += RT_NT) S.L[lay].cldlay = 0;
+    for (int i = tid; i < C.n * nl; i += nt) C.S(C.c(i)).L[C.rest(i)].cldlay = 0;
   }
   }
-  if (err) atomicMax(&S.h->iscal[0], err);
-  __syncthreads();
-  if (tid == 0) {
-    err = S.h->iscal[0];
-    if (notpre) err = GB_COL_LAYTROP;
-    if (bad) err = GB_COL_BADVAL;
+  U.sync();
+  if (t == 0 && act) {
+    int err = S.h->iscal[0];
+    if (S.h->iscal[3] & 2) err = GB_COL_LAYTROP;
+    if (S.h->iscal[3] & 1) err = GB_COL_BADVAL;
     if (BAND) {  // the column status already holds cldprop's code
       if (err) {
         if (a.col_err) atomicMax(a.col_err + icol, err);
@@ -969,211 +1333,39 @@ __device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, cons
     }
   }
 
-  const float sd = S.h->misc[band];
-  const unsigned bit = 1u << lane;
-  const int cband = BAND ? cloud_band(S.h->iscal[2], band) : 0;
-  const bool maxrand = BAND && a.icld >= 2;
-  float cr = 0.0f, kr = 0.0f, radm = 0.0f;  // rtrnmr's cloudy and clear radiances and overlap term
-  float* part = S.part + warp * (nl + 1) * 6;  // this warp's level sums
-
-  // ---------------- downward pass (rtrnmc.f90:347-455): total and clear-sky streams
-  // The next layer's gas optics are loaded while this one is done; the
-  // level sums of two layers share one transposed butterfly.
-  float rd = 0.0f, rc = 0.0f, f1 = 0.0f, tgn, pfn, p0 = 0.0f, p1 = 0.0f;
-  const float* gcp = !BAND && clouds && !fused ? src.gc : nullptr;  // the cells' cloud values, if handed over
-  float cvn = 0.0f;
-  bool pend = false;  // a layer's weighted radiances wait in p0, p1 (the same in every lane)
-  gas_at<MODE>(src, layer_on_net<MODE>(src, nl - 1), nl - 1, g, po, tgn, pfn);
-  if (gcp) cvn = gcp[(nl - 1) * GB_NGPT + g];
-  for (int lay = nl - 1; lay >= 0; --lay) {
-    const float tg = tgn, pf = pfn, cv = cvn;
-    if (lay > 0) {  // in flight meanwhile
-      gas_at<MODE>(src, layer_on_net<MODE>(src, lay - 1), lay - 1, g, po, tgn, pfn);
-      if (gcp) cvn = gcp[(lay - 1) * GB_NGPT + g];
-    }
-    const float4 r = S.L[lay].rec[band];
-    const float od = fmaxf(sd * (tg + r.w), 0.0f);
-    const Clr c = clear_cell(T, od);
-    const float gsd = pf * fmaf(c.x, r.y, r.x) * c.atrans;
-    const float tr = 1.0f - c.atrans;
-    rc = fmaf(rc, tr, gsd);
-    float A = tr, B = gsd;
-    if (clouds && S.L[lay].cldlay) {
-      if constexpr (BAND) {
-        const float* ov = S.ovl(lay);
-        const float cf = ov[0], odcld = S.L[lay].tcl[cband];
-        float atot, x;
-        cloud_total(T, c, od, odcld, atot, x);
-        const float bbdtot = pf * fmaf(x, r.y, r.x);
-        if (!maxrand) {  // rtrn.f90:370-432
-          const float efcl = (1.0f - __expf(-odcld)) * cf;
-          A = 1.0f - fmaf(efcl, 1.0f - c.atrans, c.atrans);
-          B = fmaf(cf, fmaf(bbdtot, atot, -gsd), gsd);
-        } else {  // rtrnmr.f90:590-609
-          if (S.L[lay].lfl & 2) {
-            cr = cf * rd;
-            kr = rd - cr;
-            radm = 0.0f;
-          }
-          const float ttot = 1.0f - atot, cldsrc = bbdtot * atot;
-          cr = fmaf(cr, ttot, cf * cldsrc);
-          kr = fmaf(kr, tr, (1.0f - cf) * gsd);
-          A = 0.0f;
-          B = cr + kr;
-          const float radmod = fmaf(radm, fmaf(ov[7], tr, ov[9] * ttot), fmaf(ov[12], cldsrc, -ov[11] * gsd));
-          const float oc = cr - radmod, ok = kr + radmod;
-          radm = fmaf(ov[8], ok, fmaf(-ov[10], oc, -radmod));
-          cr += radm;
-          kr -= radm;
-        }
-      } else {
-        const bool one = S.L[lay].cbits[warp] & bit;
-        if (one || (!fused && (S.fbits(lay)[warp] & bit))) {
-          float odcld, efcl, atot, x;
-          const float cldf = gcp ? cell_from_value(one, cv, sd, odcld, efcl)
-                                 : cell_cloud(a, S, icol, g, lay, band, sd, one, T, odcld, efcl);
-          cloud_total(T, c, od, odcld, atot, x);
-          A = 1.0f - fmaf(efcl, 1.0f - c.atrans, c.atrans);
-          B = fmaf(cldf, fmaf(pf * fmaf(x, r.y, r.x), atot, -gsd), gsd);
-        }
-      }
-    }
-    rd = fmaf(rd, A, B);
-    if (lay == 0) f1 = pf;
-    if (pend) {  // lanes 0, 1: layer lay+1; lanes 2, 3: layer lay
-      const float s = reduce4(p0, p1, rd * wgt, rc * wgt, lane);
-      if (lane < 4) part[(lay + 1 - (lane >> 1)) * 6 + (lane & 1)] = s;
-    } else {
-      p0 = rd * wgt;
-      p1 = rc * wgt;
-    }
-    pend = !pend;
+  if (warp * 32 < C.n * RT_CT) {  // a warp with threads of the unit's columns
+    const float wgt = live ? __ldg(T + c_T.gpt_wgt + g) : 0.0f;
+    if (BAND && a.icld >= 2)
+      rt_passes<MODE, BAND ? PK_MAXRAN : PK_FUSED>(a, S, src, U.tt, band, g, po, grp, l16, inblk, wgt);
+    else if (BAND)
+      rt_passes<MODE, BAND ? PK_RANDOM : PK_FUSED>(a, S, src, U.tt, band, g, po, grp, l16, inblk, wgt);
+    else if (clouds && !fused)
+      rt_passes<MODE, BAND ? PK_FUSED : PK_SUBCOL>(a, S, src, U.tt, band, g, po, grp, l16, inblk, wgt);
+    else
+      rt_passes<MODE, PK_FUSED>(a, S, src, U.tt, band, g, po, grp, l16, inblk, wgt);
   }
-  if (pend) {  // layer 0 on its own
-    const float s = reduce2(p0, p1, lane);
-    if (lane < 2) part[lane] = s;
-  }
-
-  // ---------------- surface emission and reflection (rtrnmc.f90:465-485)
-  const bool idrv = a.idrv == 1;
-  const float rad0 = f1 * S.h->misc[16 + band];
-  const float reflect = 1.0f - S.h->misc[48 + band];
-  float ru = rad0 + reflect * rd;
-  float rcu = rad0 + reflect * rc;
-  float du = f1 * S.h->misc[32 + band];
-  float dcu = du;
-  if (idrv) {
-    const float s = reduce4(ru * wgt, rcu * wgt, du * wgt, dcu * wgt, lane);
-    if (lane < 4) part[2 + lane] = s;
-  } else {
-    const float s = reduce2(ru * wgt, rcu * wgt, lane);
-    if (lane < 2) part[2 + lane] = s;
-  }
-  // ---------------- upward pass (rtrnmc.f90:486-529): level lay+1 above layer lay
-  float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f, q3 = 0.0f;
-  pend = false;  // a layer's weighted values wait in q0..q3
-  gas_at<MODE>(src, layer_on_net<MODE>(src, 0), 0, g, po, tgn, pfn);
-  if (gcp) cvn = gcp[g];
-  for (int lay = 0; lay < nl; ++lay) {
-    const float tg = tgn, pf = pfn, cv = cvn;
-    if (lay + 1 < nl) {
-      gas_at<MODE>(src, layer_on_net<MODE>(src, lay + 1), lay + 1, g, po, tgn, pfn);
-      if (gcp) cvn = gcp[(lay + 1) * GB_NGPT + g];
-    }
-    const float4 r = S.L[lay].rec[band];
-    const float od = fmaxf(sd * (tg + r.w), 0.0f);
-    const Clr c = clear_cell(T, od);
-    const float gsu = pf * fmaf(c.x, r.z, r.x) * c.atrans;
-    const float tr = 1.0f - c.atrans;
-    rcu = fmaf(rcu, tr, gsu);
-    dcu *= tr;
-    float A = tr, B = gsu, D = tr;
-    if (clouds && S.L[lay].cldlay) {
-      if constexpr (BAND) {
-        const float* ov = S.ovl(lay);
-        const float cf = ov[0], odcld = S.L[lay].tcl[cband];
-        float atot, x;
-        cloud_total(T, c, od, odcld, atot, x);
-        const float bbutot = pf * fmaf(x, r.z, r.x);
-        D = fmaf(cf, 1.0f - atot, (1.0f - cf) * (1.0f - c.atrans));
-        if (!maxrand) {  // rtrn.f90:495-507
-          const float efcl = (1.0f - __expf(-odcld)) * cf;
-          A = 1.0f - fmaf(efcl, 1.0f - c.atrans, c.atrans);
-          B = fmaf(cf, fmaf(bbutot, atot, -gsu), gsu);
-        } else {  // rtrnmr.f90:688-713
-          if (S.L[lay].lfl & 1) {
-            cr = cf * ru;
-            kr = ru - cr;
-            radm = 0.0f;
-          }
-          const float ttot = 1.0f - atot, cldsrc = bbutot * atot;
-          cr = fmaf(cr, ttot, cf * cldsrc);
-          kr = fmaf(kr, tr, (1.0f - cf) * gsu);
-          A = 0.0f;
-          B = cr + kr;
-          const float radmod = fmaf(radm, fmaf(ov[1], tr, ov[3] * ttot), fmaf(ov[6], cldsrc, -ov[5] * gsu));
-          const float oc = cr - radmod, ok = kr + radmod;
-          radm = fmaf(ov[2], ok, fmaf(-ov[4], oc, -radmod));
-          cr += radm;
-          kr -= radm;
-        }
-      } else {
-        const bool one = S.L[lay].cbits[warp] & bit;
-        if (one || (!fused && (S.fbits(lay)[warp] & bit))) {
-          float odcld, efcl, atot, x;
-          const float cldf = gcp ? cell_from_value(one, cv, sd, odcld, efcl)
-                                 : cell_cloud(a, S, icol, g, lay, band, sd, one, T, odcld, efcl);
-          cloud_total(T, c, od, odcld, atot, x);
-          A = 1.0f - fmaf(efcl, 1.0f - c.atrans, c.atrans);
-          B = fmaf(cldf, fmaf(pf * fmaf(x, r.z, r.x), atot, -gsu), gsu);
-          D = fmaf(cldf, 1.0f - atot, (1.0f - cldf) * (1.0f - c.atrans));
-        }
-      }
-    }
-    ru = fmaf(ru, A, B);
-    du *= D;
-    if (pend) {  // levels lay (the layer below) and lay+1
-      if (idrv) {
-        const float s = reduce8(q0, q1, q2, q3, ru * wgt, rcu * wgt, du * wgt, dcu * wgt, lane);
-        if (lane < 8) part[(lay + (lane >> 2)) * 6 + 2 + (lane & 3)] = s;
-      } else {
-        const float s = reduce4(q0, q1, ru * wgt, rcu * wgt, lane);
-        if (lane < 4) part[(lay + (lane >> 1)) * 6 + 2 + (lane & 1)] = s;
-      }
-    } else {
-      q0 = ru * wgt;
-      q1 = rcu * wgt;
-      q2 = du * wgt;
-      q3 = dcu * wgt;
-    }
-    pend = !pend;
-  }
-  if (pend) {  // level nl on its own
-    float* p = part + nl * 6 + 2;
-    if (idrv) {
-      const float s = reduce4(q0, q1, q2, q3, lane);
-      if (lane < 4) p[lane] = s;
-    } else {
-      const float s = reduce2(q0, q1, lane);
-      if (lane < 2) p[lane] = s;
-    }
-  }
-  __syncthreads();
+  U.sync();
 
   // ---------------- fp64 outputs: fluxes, net fluxes, heating rates (rtrnmc.f90:566-592)
   const long long ldo = a.ldo;
-  double* fnet = reinterpret_cast<double*>(S.L);  // [nl+1][2]
-  for (int lev = tid; lev <= nl; lev += RT_NT) {
-    // the five warps' fp32 partials summed without rounding error: Knuth's
+  const bool idrv = a.idrv == 1;
+  auto solved = [&](int c) {  // a column of the grid, and on the network where that was asked
+    return C.col0 + c <= C.last && (!NET || C.S(c).h->iscal[2] == 0);
+  };
+  for (int i = tid; i < C.n * (nl + 1); i += nt) {
+    const int c = C.c(i), lev = C.rest(i);
+    const RtSmem Sc = C.S(c);
+    double* fnet = reinterpret_cast<double*>(Sc.L);  // [nl+1][2]
+    // the five groups' fp32 partials summed without rounding error: Knuth's
     // two-sum keeps each addition's rounding error, and the sum and the
     // accumulated errors go to fp64 together
     double acc[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      float hi = S.part[lev * 6 + k], lo = 0.0f;
+      float hi = Sc.part[lev * 6 + k], lo = 0.0f;
 #pragma unroll
       for (int w = 1; w < RT_NW; ++w) {
-        const float b = S.part[(w * (nl + 1) + lev) * 6 + k];
+        const float b = Sc.part[(w * (nl + 1) + lev) * 6 + k];
         const float sum = hi + b, bv = sum - hi;
         lo += (hi - (sum - bv)) + (b - bv);
         hi = sum;
@@ -1181,7 +1373,10 @@ __device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, cons
       acc[k] = (double)hi + (double)lo;
     }
     if (lev == nl) acc[0] = acc[1] = 0.0;  // no downward radiation at the model top
-    const long long o = icol + ldo * lev;
+    fnet[lev * 2 + 0] = acc[2] - acc[0];
+    fnet[lev * 2 + 1] = acc[3] - acc[1];
+    if (!solved(c)) continue;
+    const long long o = C.col0 + c + ldo * lev;
     a.uflx[o] = acc[2];
     a.dflx[o] = acc[0];
     a.uflxc[o] = acc[3];
@@ -1190,19 +1385,20 @@ __device__ bool rt_column(const LwArgs& a, long long icol, const RtSmem& S, cons
       a.duflx_dt[o] = acc[4];
       a.duflxc_dt[o] = acc[5];
     }
-    fnet[lev * 2 + 0] = acc[2] - acc[0];
-    fnet[lev * 2 + 1] = acc[3] - acc[1];
   }
-  __syncthreads();
-  for (int l = tid; l < nl; l += RT_NT) {
-    const double dp = in2(a.plev, a.ld, icol, l) - in2(a.plev, a.ld, icol, l + 1);
+  U.sync();
+  for (int i = tid; i < C.n * nl; i += nt) {
+    const int c = C.c(i), l = C.rest(i);
+    if (!solved(c)) continue;
+    const double* fnet = reinterpret_cast<const double*>(C.S(c).L);
+    const double dp = in2(a.plev, a.ld, C.col0 + c, l) - in2(a.plev, a.ld, C.col0 + c, l + 1);
     const double f = c_T.heatfac / dp;  // one division for both heating rates
-    const long long o = icol + ldo * l;
+    const long long o = C.col0 + c + ldo * l;
     a.hr[o] = f * (fnet[l * 2] - fnet[(l + 1) * 2]);
     a.hrc[o] = f * (fnet[l * 2 + 1] - fnet[(l + 1) * 2 + 1]);
   }
-  __syncthreads();
-  return true;
+  U.sync();
+  return act;
 }
 
 // ------------------------------------------------------------------ kernels
@@ -1218,13 +1414,23 @@ __device__ __forceinline__ int grid_of(const LwBatch& B, long long gc, int gi) {
 // field in a register.
 constexpr size_t ARGS_BYTES = (sizeof(LwArgs) + 15) & ~size_t(15);
 static_assert(sizeof(LwArgs) % 4 == 0, "LwArgs copied as 32-bit words");
-__device__ __forceinline__ const LwArgs& stage_args(const LwArgs& a, char* smem) {
-  __syncthreads();  // every thread is done with the previous column's copy
+__device__ __forceinline__ const LwArgs& stage_args(const LwArgs& a, char* smem, const Unit& U) {
+  U.sync();  // every thread is done with the previous column's copy
   int* dst = reinterpret_cast<int*>(smem);
   const int* src = reinterpret_cast<const int*>(&a);
-  for (int k = threadIdx.x; k < (int)(sizeof(LwArgs) / 4); k += blockDim.x) dst[k] = src[k];
-  __syncthreads();
+  for (int k = U.tid; k < (int)(sizeof(LwArgs) / 4); k += U.nt) dst[k] = src[k];
+  U.sync();
   return *reinterpret_cast<const LwArgs*>(smem);
+}
+
+// rtrnmc's (exp_tbl, tfn_tbl) copied to shared memory by the whole block; ends with a barrier
+constexpr size_t TABLE_BYTES = (size_t(10001) * 8 + 15) & ~size_t(15);
+__device__ __forceinline__ const float2* stage_table(const float* __restrict__ T, char* smem) {
+  const float4* src = reinterpret_cast<const float4*>(T + c_T.tbl_tt);  // tables start on 16-byte boundaries
+  float4* dst = reinterpret_cast<float4*>(smem);
+  for (int k = threadIdx.x; k < (int)(TABLE_BYTES / 16); k += blockDim.x) dst[k] = __ldg(src + k);
+  __syncthreads();
+  return reinterpret_cast<const float2*>(smem);
 }
 
 // taumol's outputs as [layer][140] planes
@@ -1255,81 +1461,95 @@ __global__ void __launch_bounds__(NT) lw_gas_kernel(const __grid_constant__ LwBa
   int gi = 0;
   for (long long i = c0 + blockIdx.x; i < c1; i += gridDim.x) {
     gi = grid_of(B, i, gi);
-    const LwArgs& a = stage_args(B.g[gi], smem_raw);
+    const LwArgs& a = stage_args(B.g[gi], smem_raw, Unit{(int)threadIdx.x, NT, 1, nullptr});
     const long long slot = i - c0;
     gas_column<NT>(a, i - B.col0[gi], s, SampleOut{B.gtau + slot * B.gstride, B.gfrac + slot * B.gstride}, T);
   }
 }
 
-// The transfer over batch columns [c0, c1), one block per column.  RT_GAS: on
-// taumol's planes, column c0 + k in slot k (BAND: the non-McICA driver's band
-// clouds).  RT_NET: on the network's gas optics; a column with a layer off the
-// network is appended to B.fall instead.
-template <int MINB, int MODE, bool BAND>
-__global__ void __launch_bounds__(RT_NT, MINB) lw_rt_kernel(const __grid_constant__ LwBatch B,
-                                                             const float* __restrict__ T, long long c0, long long c1) {
+// what a thread's column reads its gas optics from
+__device__ __forceinline__ GasSrc net_source(const LwArgs& a, long long icol) {
+  GasSrc src{};
+  const long long row = icol * a.nlay * GB_NGPT;
+  src.nt = a.sur_tau + row;
+  src.nf = a.sur_frac + row;
+  src.flag = a.sur_flag + icol * a.nlay;
+  return src;
+}
+
+// The transfer over units [u0, u1).  A block is the SM's only one: MAXU units
+// at most, of RT_NT threads (two columns) or of half as many (one), that go
+// through the batch side by side, each with its own barrier; they share one copy of
+// rtrnmc's table (80 KB) in shared memory.  In L1 the table's lookups, spread
+// over 32 lines a warp, missed to L2 in every second case.
+// RT_GAS: on taumol's planes, unit u in plane slots (u - u0) * cpb .. (BAND: the
+// non-McICA driver's band clouds).  RT_NET: on the network's gas optics; a
+// column with a layer off the network is appended to B.fall instead.
+template <int MAXU, int MODE, bool BAND>
+__global__ void __launch_bounds__(RT_NT * MAXU, 1) lw_rt_kernel(const __grid_constant__ LwBatch B,
+                                                                const float* __restrict__ T, long long u0,
+                                                                long long u1, int nunit) {
   extern __shared__ __align__(16) char smem_raw[];
-  const RtSmem S = rt_carve(smem_raw + ARGS_BYTES, B.nsmax);
+  const float2* tt = stage_table(T, smem_raw);
+  const int nt = blockDim.x / nunit, unit = threadIdx.x / nt;
+  const Unit U{(int)threadIdx.x - unit * nt, nt, 1 + unit, tt};
+  const int slot = blockIdx.x * nunit + unit;  // of the resident units
+  char* smem = smem_raw + TABLE_BYTES + unit * (ARGS_BYTES + B.cpb * rt_smem_bytes(B.nsmax));
+  const int half = U.tid / RT_CT, col = half < B.cpb ? half : B.cpb - 1;
   int gi = 0;
-  for (long long i = c0 + blockIdx.x; i < c1; i += gridDim.x) {
-    gi = grid_of(B, i, gi);
-    const LwArgs& a = stage_args(B.g[gi], smem_raw);
-    const long long icol = i - B.col0[gi];
+  for (long long u = u0 + slot; u < u1; u += (long long)gridDim.x * nunit) {
+    while (u >= B.unit0[gi + 1]) ++gi;
+    const LwArgs& a = stage_args(B.g[gi], smem, U);
+    const Cols C{smem + ARGS_BYTES, rt_smem_bytes(B.nsmax), B.part + (size_t)slot * B.cpb * rt_part_floats(B.nsmax),
+                 B.cpb, B.nsmax, (u - B.unit0[gi]) * B.cpb, a.ncol - 1};
     GasSrc src{};
-    if (MODE == RT_GAS) {
-      src.plane = B.plane + (i - c0) * B.nsmax * GB_LW_PROW;
-      src.gc = !BAND && B.gcld ? B.gcld + (long long)blockIdx.x * B.nsmax * GB_NGPT : nullptr;
-    } else {
-      const long long row = icol * a.nlay * GB_NGPT;
-      src.nt = a.sur_tau ? a.sur_tau + row : nullptr;
-      src.nf = a.sur_frac ? a.sur_frac + row : nullptr;
-      src.flag = a.sur_flag ? a.sur_flag + icol * a.nlay : nullptr;
-    }
-    const bool done = rt_column<MODE, BAND>(a, icol, S, src, T);
-    if (MODE == RT_NET && !done && threadIdx.x == 0) B.fall[atomicAdd(B.nfall, 1u)] = i;
+    if (MODE == RT_GAS)
+      src.plane = B.plane + ((u - u0) * B.cpb + col) * B.nsmax * GB_LW_PROW;
+    else if (a.sur_flag)
+      src = net_source(a, C.icol(col));
+    if (!BAND) src.gc = B.gcld + ((long long)slot * B.cpb + col) * B.nsmax * GB_NGPT;
+    const bool done = (MODE == RT_GAS || a.sur_flag) && rt_columns<MODE, BAND>(a, U, C, src, T);
+    if (MODE != RT_GAS && !done && U.tid == half * RT_CT && half < B.cpb && C.col0 + col <= C.last)
+      B.fall[atomicAdd(B.nfall, 1u)] = B.col0[gi] + C.col0 + col;
   }
 }
 
-// The columns handed over by the network's transfer kernel (B.fall): taumol
-// into the block's plane slot, then the transfer with each layer's gas optics
-// from the network or from taumol.
-template <int MINB>
-__global__ void __launch_bounds__(RT_NT, MINB) lw_list_kernel(const __grid_constant__ LwBatch B,
-                                                               const float* __restrict__ T) {
+// The columns handed over by the network's transfer kernel (B.fall), one per
+// block: taumol into the block's plane slot, then the transfer with each
+// layer's gas optics from the network or from taumol.
+__global__ void __launch_bounds__(RT_NT, LIST_PER_SM) lw_list_kernel(const __grid_constant__ LwBatch B,
+                                                                     const float* __restrict__ T) {
   extern __shared__ __align__(16) char smem_raw[];
-  const GasSmem gs = gas_carve(smem_raw + ARGS_BYTES, B.nsmax);
-  const RtSmem S = rt_carve(smem_raw + ARGS_BYTES, B.nsmax);  // used after taumol is done with the same memory
-  float* plane = B.plane + (long long)blockIdx.x * B.nsmax * GB_LW_PROW;
   const long long n = (long long)*B.nfall;
+  if (blockIdx.x >= n) return;
+  const Unit U{(int)threadIdx.x, RT_NT, 1, stage_table(T, smem_raw)};
+  char* smem = smem_raw + TABLE_BYTES;
+  const GasSmem gs = gas_carve(smem + ARGS_BYTES, B.nsmax);  // the transfer uses the same memory afterwards
+  float* plane = B.plane + (long long)blockIdx.x * B.nsmax * GB_LW_PROW;
   for (long long i = blockIdx.x; i < n; i += gridDim.x) {
     const long long gc = B.fall[i];
     const int gi = grid_of(B, gc, 0);  // the list is in no particular order
-    const LwArgs& a = stage_args(B.g[gi], smem_raw);
+    const LwArgs& a = stage_args(B.g[gi], smem, U);
     const long long icol = gc - B.col0[gi];
     gas_column<RT_NT>(a, icol, gs, PlaneOut{plane}, T);
-    GasSrc src{};
+    const Cols C{smem + ARGS_BYTES, rt_smem_bytes(B.nsmax), B.part + blockIdx.x * rt_part_floats(B.nsmax), 1, B.nsmax,
+                 icol, icol};
+    GasSrc src = a.sur_flag ? net_source(a, icol) : GasSrc{};
     src.plane = plane;
-    src.gc = B.gcld ? B.gcld + (long long)blockIdx.x * B.nsmax * GB_NGPT : nullptr;
-    if (a.sur_flag) {
-      const long long row = icol * a.nlay * GB_NGPT;
-      src.nt = a.sur_tau + row;
-      src.nf = a.sur_frac + row;
-      src.flag = a.sur_flag + icol * a.nlay;
-      rt_column<RT_MIX>(a, icol, S, src, T);
-    } else {
-      rt_column<RT_GAS>(a, icol, S, src, T);
-    }
+    src.gc = B.gcld + (long long)blockIdx.x * B.nsmax * GB_NGPT;
+    if (a.sur_flag)
+      rt_columns<RT_MIX>(a, U, C, src, T);
+    else
+      rt_columns<RT_GAS>(a, U, C, src, T);
   }
 }
 
 constexpr int GAS_NT = 128;      // threads of the taumol kernel
-constexpr int BAND_MINB = 6;
-constexpr int LIST_PER_SM = 2;   // hand-over kernel blocks per SM
-constexpr int LIST_MINB = 6;
+constexpr int BAND_MAXU = 4;
 
-// compiled shapes (min blocks per SM for the register allocation, 160
-// threads each); variant 0 is the default
-#define GB_LW_VARIANTS(X) X(0, 6) X(1, 7) X(2, 5) X(3, 4)
+// compiled shapes: the most units (column blocks) of an SM that the register
+// allocation is sized for; variant 0 is the default
+#define GB_LW_VARIANTS(X) X(0, 4) X(1, 3) X(2, 5) X(3, 2)
 
 }  // namespace gb
 
@@ -1337,27 +1557,41 @@ constexpr int LIST_MINB = 6;
 namespace {
 
 struct VariantInfo {
-  int min_blocks;
+  int max_units;
   const void* fn;  // the kernel this shape launches
-  cudaError_t (*launch)(const LwBatch&, const float*, long long, long long, int, size_t, cudaStream_t);
+  cudaError_t (*launch)(const LwBatch&, const float*, long long, long long, int, int, int, size_t, cudaStream_t);
 };
 
-template <int MINB, int MODE>
-cudaError_t launch_rt(const LwBatch& b, const float* T, long long c0, long long c1, int nblocks, size_t smem,
-                      cudaStream_t st) {
-  gb::lw_rt_kernel<MINB, MODE, false><<<nblocks, gb::RT_NT, smem, st>>>(b, T, c0, c1);
+template <int MAXU, int MODE, bool BAND>
+cudaError_t launch_rt(const LwBatch& b, const float* T, long long u0, long long u1, int nblocks, int threads, int nunit,
+                      size_t smem, cudaStream_t st) {
+  gb::lw_rt_kernel<MAXU, MODE, BAND><<<nblocks, threads, smem, st>>>(b, T, u0, u1, nunit);
   return cudaGetLastError();
 }
+template <int MAXU, int MODE, bool BAND>
+constexpr VariantInfo variant_of() {
+  return {MAXU, (const void*)gb::lw_rt_kernel<MAXU, MODE, BAND>, launch_rt<MAXU, MODE, BAND>};
+}
 
-// the transfer kernel on taumol's planes, and on the network's outputs
-#define GB_LW_GAS_ENTRY(i, mb) {mb, (const void*)gb::lw_rt_kernel<mb, gb::RT_GAS, false>, launch_rt<mb, gb::RT_GAS>},
-#define GB_LW_NET_ENTRY(i, mb) {mb, (const void*)gb::lw_rt_kernel<mb, gb::RT_NET, false>, launch_rt<mb, gb::RT_NET>},
+// the transfer kernel on taumol's planes, on the network's outputs (also where
+// these do not start on 4-byte boundaries), and for band clouds
+#define GB_LW_GAS_ENTRY(i, mu) variant_of<mu, gb::RT_GAS, false>(),
+#define GB_LW_NET_ENTRY(i, mu) variant_of<mu, gb::RT_NET, false>(),
 const VariantInfo kVariants[] = {GB_LW_VARIANTS(GB_LW_GAS_ENTRY)};
 const VariantInfo kLean[] = {GB_LW_VARIANTS(GB_LW_NET_ENTRY)};
+const VariantInfo kOdd = variant_of<4, gb::RT_NETODD, false>();
+const VariantInfo kBand = variant_of<gb::BAND_MAXU, gb::RT_GAS, true>();
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-constexpr int kMaxPerSm = 16;  // most resident column blocks per SM any shape launches
+constexpr int kMaxPerSm = 5;  // most units of an SM any shape launches
 
 const VariantInfo& info(int variant, bool lean) { return lean ? kLean[variant] : kVariants[variant]; }
+
+size_t device_smem() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return (size_t)n;
+}
 
 int device_sms() {
   int dev = 0, nsm = 1;
@@ -1367,8 +1601,12 @@ int device_sms() {
 }
 
 // shared memory of a block of the transfer kernel, and of the hand-over kernel (taumol or transfer area)
-size_t block_smem(int nlay) { return gb::ARGS_BYTES + gb::rt_smem_bytes(nlay); }
-size_t list_smem(int nlay) { return gb::ARGS_BYTES + std::max(gb::rt_smem_bytes(nlay), gb::gas_smem_bytes(nlay)); }
+size_t block_smem(int nlay, int cpb, int units) {
+  return gb::TABLE_BYTES + units * (gb::ARGS_BYTES + cpb * gb::rt_smem_bytes(nlay));
+}
+size_t list_smem(int nlay) {
+  return gb::TABLE_BYTES + gb::ARGS_BYTES + std::max(gb::rt_smem_bytes(nlay), gb::gas_smem_bytes(nlay));
+}
 
 // Shared-memory carve-out for `per` resident blocks of `smem` bytes: just what
 // they need, so that the rest of the SM's memory stays L1 for the table
@@ -1427,7 +1665,7 @@ int gb_lw_num_variants() { return kNumVariants; }
 
 LwVariant gb_lw_variant(int v, bool lean) {
   if (v < 0 || v >= kNumVariants) return LwVariant{0, 0};
-  return LwVariant{gb::RT_NT, info(v, lean).min_blocks};
+  return LwVariant{gb::RT_NT, info(v, lean).max_units};
 }
 
 size_t gb_lw_smem_bytes(int nlay) { return list_smem(nlay); }
@@ -1437,44 +1675,71 @@ cudaError_t gb_lw_set_tables(const GbTables& T) {
   return e == cudaSuccess ? gb_lw_taumol_set_tables(T) : e;
 }
 
+namespace {
+// Columns per unit: two, a thread per pair of g-points (80 a column), where
+// two columns fit in a block's shared memory, and where the batch has more
+// columns than the device has SMs: of fewer, each gets an SM to itself.
+int cols_per_unit(int nlay, long long ncols) {
+  return ncols > device_sms() && block_smem(nlay, 2, 1) <= device_smem() ? 2 : 1;
+}
+int unit_threads(int cpb) { return cpb == 2 ? gb::RT_NT : (gb::RT_CT + 31) / 32 * 32; }
+int units_per_sm(int nlay, int cpb, const VariantInfo& v) {
+  int n = v.max_units;
+  while (n > 1 && block_smem(nlay, cpb, n) > device_smem()) --n;
+  return n;
+}
+}  // namespace
+
+// Four units where their shared memory fits (96 registers a thread), else
+// three with 128: at 60 layers three fit, and 32,768 columns of the learned
+// path take 3.65 ms with 128 registers, 3.76 with 96 (in-kernel clouds with
+// taumol 4.37 and 4.51); at 45 layers four with 96 take 4.90 ms, three with
+// 128 5.12 (caller sub-columns).  Five with 72 registers spill (5.8 ms).
+int gb_lw_default_variant(int nlay) {
+  const int cpb = cols_per_unit(nlay, LLONG_MAX);
+  for (int v : {0, 1, 3})
+    if (units_per_sm(nlay, cpb, kVariants[v]) == kVariants[v].max_units) return v;
+  return 3;
+}
+
 int gb_lw_slots(int nlay, int variant, bool lean) {
   if (variant < 0 || variant >= kNumVariants) variant = 0;
-  const VariantInfo& v = info(variant, lean);
-  int per = 0;
-  if (occupancy(v.fn, gb::RT_NT, block_smem(nlay), &per) != cudaSuccess || per < 1) per = 1;
-  return device_sms() * std::min(per, kMaxPerSm);
+  return device_sms() * units_per_sm(nlay, cols_per_unit(nlay, LLONG_MAX), info(variant, lean));
 }
 
 namespace {
 // plane bytes of one column slot: its rows, setcoef's words, laytrop
 size_t slot_bytes(int nlay) { return (size_t)nlay * (GB_LW_PROW + GB_LW_COEF_WORDS) * 4 + sizeof(int); }
-// cloud planes of the resident columns
-size_t cloud_slots() { return (size_t)device_sms() * kMaxPerSm; }
-size_t cloud_bytes(int nlay) { return cloud_slots() * (size_t)nlay * GB_NGPT * sizeof(float); }
+// per resident column: the cloud plane of caller sub-columns, the level sums
+size_t resident_cols() { return (size_t)device_sms() * kMaxPerSm * 2; }
+size_t resident_bytes(int nlay) {
+  return resident_cols() * ((size_t)nlay * GB_NGPT + gb::rt_part_floats(nlay)) * sizeof(float);
+}
 size_t round_slots(size_t n) { return (n + 31) & ~size_t(31); }
 // a pass's planes: enough columns that the tail of a pass is small beside it
-// (a wave of the transfer is about 900 columns), few enough that the buffer
+// (a wave of the transfer is about 1,200 columns), few enough that the buffer
 // stays small beside the batch's own arrays
 constexpr size_t kPlaneBytes = size_t(1536) << 20;
 }  // namespace
 
 size_t gb_lw_gas_bytes(int nlay, long long ncols, bool learned) {
   const size_t room = std::max<size_t>(kPlaneBytes / slot_bytes(nlay) & ~size_t(31), 32);
-  const size_t want = learned ? 0 : round_slots((size_t)ncols + GB_LW_MAX_GRIDS);
+  const size_t want = learned ? 0 : round_slots((size_t)ncols + GB_LW_MAX_GRIDS);  // a column may be missing per grid
   const size_t slots = std::max(std::min(want, room), round_slots((size_t)gb_lw_list_slots()));
-  return cloud_bytes(nlay) + slots * slot_bytes(nlay);
+  return resident_bytes(nlay) + slots * slot_bytes(nlay);
 }
 
 size_t gb_lw_gas_min_bytes(int nlay) { return gb_lw_gas_bytes(nlay, 0, true); }
 
 void gb_lw_attach_gas(LwBatch& b, void* buf, size_t bytes) {
-  const size_t cloud = cloud_bytes(b.nsmax);
-  b.cslots = (long long)cloud_slots();
-  b.pslots = bytes > cloud ? (long long)((bytes - cloud) / slot_bytes(b.nsmax) & ~size_t(31)) : 0;
+  const size_t res = resident_bytes(b.nsmax);
+  b.rcols = (long long)resident_cols();
+  b.pslots = bytes > res ? (long long)((bytes - res) / slot_bytes(b.nsmax) & ~size_t(31)) : 0;
   b.plane = static_cast<float*>(buf);  // the rows first: each on a 32-byte boundary
   b.coef = b.plane + (size_t)b.pslots * b.nsmax * GB_LW_PROW;
   b.gcld = b.coef + (size_t)b.pslots * b.nsmax * GB_LW_COEF_WORDS;
-  b.laytrop = reinterpret_cast<int*>(b.gcld + (size_t)b.cslots * b.nsmax * GB_NGPT);
+  b.part = b.gcld + (size_t)b.rcols * b.nsmax * GB_NGPT;
+  b.laytrop = reinterpret_cast<int*>(b.part + (size_t)b.rcols * gb::rt_part_floats(b.nsmax));
 }
 
 long long gb_lw_list_slots() { return (long long)device_sms() * gb::LIST_PER_SM; }
@@ -1493,8 +1758,10 @@ cudaError_t gb_lw_launch_batch(const LwBatch& bin, const float* d_tables, int va
   const long long n = b.col0[b.ngrid];
   if (n <= 0 || nblocks <= 0) return cudaSuccess;
   if (!b.plane || b.pslots < 32) return cudaErrorInvalidValue;
-  b.cpb = 1;
-  for (int i = 0; i <= b.ngrid; ++i) b.unit0[i] = b.col0[i];
+  b.cpb = cols_per_unit(b.nsmax, n);
+  b.unit0[0] = 0;
+  for (int i = 0; i < b.ngrid; ++i) b.unit0[i + 1] = b.unit0[i] + (b.col0[i + 1] - b.col0[i] + b.cpb - 1) / b.cpb;
+  const long long units = b.unit0[b.ngrid];
   for (int i = 0; i < b.ngrid; ++i)  // fused-cloud grids come with their McICA draws
     if (b.g[i].cloud_mode == LW_CLOUD_FUSED && b.g[i].icld >= 1 && b.g[i].ncol > 0 && !b.g[i].draws)
       return cudaErrorInvalidValue;
@@ -1505,24 +1772,25 @@ cudaError_t gb_lw_launch_batch(const LwBatch& bin, const float* d_tables, int va
     ++nband;
     if (g.icld >= 1 && g.ncol > 0 && (!g.ncbands || !g.cldfrac || !g.tauc)) return cudaErrorInvalidValue;
   }
-  if ((long long)nblocks > n) nblocks = (int)n;
-  if ((long long)nblocks > b.cslots) nblocks = (int)b.cslots;
-  const size_t smem = block_smem(b.nsmax);
+  // nblocks units, over the SMs: nunit of them in a block, a block per SM
+  const int nsm = device_sms();
+  auto transfer = [&](const VariantInfo& v, long long u0, long long u1) -> cudaError_t {
+    const long long want = std::min<long long>(nblocks, std::min(u1 - u0, b.rcols / b.cpb));
+    const int nunit = (int)std::min<long long>((want + nsm - 1) / nsm, units_per_sm(b.nsmax, b.cpb, v));
+    const int blocks = (int)std::min<long long>((want + nunit - 1) / nunit, nsm);
+    const size_t smem = block_smem(b.nsmax, b.cpb, nunit);
+    const cudaError_t e = cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return v.launch(b, d_tables, u0, u1, blocks, nunit * unit_threads(b.cpb), nunit, smem, stream);
+  };
   if (!b.fall || !b.nfall) {
     // pass by pass: taumol into the planes, then the transfer
     if (nband && nband != b.ngrid) return cudaErrorInvalidValue;  // band clouds: every grid in that mode
-    const VariantInfo& v = info(variant, false);
-    const void* fn = nband ? (const void*)gb::lw_rt_kernel<gb::BAND_MINB, gb::RT_GAS, true> : v.fn;
-    const long long passes = (n + b.pslots - 1) / b.pslots, step = (n + passes - 1) / passes;
-    for (long long c0 = 0; c0 < n; c0 += step) {
-      const long long c1 = std::min(c0 + step, n);
-      cudaError_t e = gb_lw_launch_taumol(b, d_tables, c0, c1, stream);
-      if (e != cudaSuccess) return e;
-      e = launch_resident(fn, gb::RT_NT, smem, (int)std::min<long long>(nblocks, c1 - c0), [&](int nb) {
-        if (!nband) return v.launch(b, d_tables, c0, c1, nb, smem, stream);
-        gb::lw_rt_kernel<gb::BAND_MINB, gb::RT_GAS, true><<<nb, gb::RT_NT, smem, stream>>>(b, d_tables, c0, c1);
-        return cudaGetLastError();
-      });
+    const long long room = b.pslots / b.cpb, passes = (units + room - 1) / room, step = (units + passes - 1) / passes;
+    for (long long u0 = 0; u0 < units; u0 += step) {
+      const long long u1 = std::min(u0 + step, units);
+      cudaError_t e = gb_lw_launch_taumol(b, d_tables, u0, u1, stream);
+      if (e == cudaSuccess) e = transfer(nband ? kBand : info(variant, false), u0, u1);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1530,16 +1798,17 @@ cudaError_t gb_lw_launch_batch(const LwBatch& bin, const float* d_tables, int va
   // learned gas optics: the transfer kernel on the network's outputs, then the
   // hand-over kernel over the columns it passed on (its blocks find an empty
   // list and return when every column was on the network)
-  if (nband || b.pslots < gb_lw_list_slots()) return cudaErrorInvalidValue;
+  if (nband || b.pslots < gb_lw_list_slots() || b.rcols < gb_lw_list_slots()) return cudaErrorInvalidValue;
   cudaError_t e = cudaMemsetAsync(b.nfall, 0, sizeof(unsigned), stream);
   if (e != cudaSuccess) return e;
-  const VariantInfo& v = info(variant, true);
-  e = launch_resident(v.fn, gb::RT_NT, smem, nblocks, [&](int nb) { return v.launch(b, d_tables, 0, n, nb, smem, stream); });
+  bool odd = false;  // network rows (280 bytes) that do not start on 4-byte boundaries
+  for (int i = 0; i < b.ngrid; ++i) odd |= (((uintptr_t)b.g[i].sur_tau | (uintptr_t)b.g[i].sur_frac) & 3) != 0;
+  e = transfer(odd ? kOdd : info(variant, true), 0, units);
   if (e != cudaSuccess) return e;
-  const void* fn = (const void*)gb::lw_list_kernel<gb::LIST_MINB>;
+  const void* fn = (const void*)gb::lw_list_kernel;
   const size_t lsmem = list_smem(b.nsmax);
   return launch_resident(fn, gb::RT_NT, lsmem, (int)gb_lw_list_slots(), [&](int nb) {
-    gb::lw_list_kernel<gb::LIST_MINB><<<nb, gb::RT_NT, lsmem, stream>>>(b, d_tables);
+    gb::lw_list_kernel<<<nb, gb::RT_NT, lsmem, stream>>>(b, d_tables);
     return cudaGetLastError();
   });
 }

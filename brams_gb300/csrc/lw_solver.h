@@ -92,7 +92,8 @@ struct LwBatch {
   long long pslots = 0;                   // plane slots available (a multiple of 32)
   float* gcld = nullptr;                  // caller sub-columns: each cloudy cell's optical depth (or
                                           // fractional cldfmcl), [nsmax][140] per resident column
-  long long cslots = 0;                   // such slots available
+  float* part = nullptr;                  // level sums per resident column
+  long long rcols = 0;                    // resident columns there is room for
   float* gtau = nullptr;                  // taumol-only launch (see above)
   float* gfrac = nullptr;
   long long gstride = 0;                  // floats per slot (>= nsmax * 140)
@@ -102,15 +103,18 @@ struct LwBatch {
   LwArgs g[GB_LW_MAX_GRIDS];
 };
 
-// Compiled shapes of the column kernels: threads per block (one column per
-// block, one g-point per thread) and the minimum resident blocks per SM the
-// register allocation is sized for.
+// Compiled shapes of the transfer kernel: threads per column block (a unit of
+// two columns, a pair of g-points per thread) and the most of them on an SM
+// that the register allocation is sized for.
 struct LwVariant {
   int threads, min_blocks;
 };
 // The learned-gas-optics transfer kernel (lean = true) has its own table of as many shapes.
 int gb_lw_num_variants();
 LwVariant gb_lw_variant(int v, bool lean = false);
+
+// the variant sized for the units (column blocks) that fit on an SM at this nlay
+int gb_lw_default_variant(int nlay);
 
 // shared memory one block needs at this nlay (one column's taumol or
 // transfer area); a launch is possible iff this fits in one block

@@ -1,6 +1,7 @@
 """Longwave batches through taumol's planes: column counts around the 32-column
-tiles, ragged grids in one batch, shallow and deep columns, and a batch that
-takes several passes over the planes."""
+tiles and the two columns of a unit, ragged grids in one batch, shallow and
+deep columns, a batch that takes several passes over the planes, and the
+network's rows at any address."""
 import numpy as np
 import pytest
 
@@ -24,7 +25,8 @@ def _solve(ctx, grids, seeds):
     return [g.outputs() for g in grids]
 
 
-@pytest.mark.parametrize("shapes", [[(1, 3)], [(31, 45)], [(32, 38)], [(33, 60)], [(65, 7), (1, 128), (30, 46)]])
+@pytest.mark.parametrize("shapes", [[(1, 3)], [(31, 45)], [(32, 38)], [(33, 60)], [(65, 7), (1, 128), (30, 46)],
+                                    [(153, 38)], [(160, 46), (3, 45), (200, 5)], [(155, 230)]])
 def test_ragged_batches_against_oracle(ctx, shapes):
     grids, refs, seeds = [], [], []
     for i, (ncol, nlay) in enumerate(shapes):
@@ -70,3 +72,29 @@ def test_several_passes_equal_separate_calls(ctx):
         for k in OUTS:
             assert np.array_equal(got[k], ref[k]), k
     assert ctx.sync_status() == 0
+
+
+@pytest.mark.parametrize("ncol", [7, 401])
+def test_network_rows_on_any_address(ctx, ncol):
+    """The learned batch reads its fp16 rows wherever they start: the same bits
+    from rows on 4-byte boundaries and from rows one half word on."""
+    import torch
+
+    mlp = S.load(ctx)
+    st = make_state(ProfileSpec(ncol=ncol, nlay=45, seed=5, t_noise=4.0))
+    g = S.DeviceGrid(st, pyoracle.cldprop_columns(st))
+    n = ncol * 45 * 140
+    rows = torch.zeros((2, n + 4), dtype=torch.float16, device="cuda")
+    flag = torch.zeros(ncol * 45, dtype=torch.uint8, device="cuda")
+    mlp.infer(g.desc(), rows[0], rows[1], flag)
+    got = []
+    for shift in (0, 1):
+        r = torch.zeros((2, n + 4), dtype=torch.float16, device="cuda")
+        r[:, shift:shift + n] = rows[:, :n]
+        ctx.rrtmg_lw_batch_device([g.desc(seed0=3, sur_tau=r[0, shift:], sur_frac=r[1, shift:], sur_flag=flag)])
+        torch.cuda.synchronize()
+        got.append(g.outputs())
+    assert ctx.sync_status() == 0
+    for k in OUTS:
+        assert np.array_equal(got[0][k], got[1][k]), k
+    mlp.close()
