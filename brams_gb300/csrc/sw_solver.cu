@@ -1,9 +1,8 @@
 // RRTMG_SW host side: the shortwave tables (rrtmg_sw_init.f90) reduced to
 // 112 g-points, uploaded in fp64 and fp32, and the launch of the column kernel
 // (sw_kernel.cuh) in either precision; and the band cloud optics cldprop_sw
-// on the device.  This unit holds the fp64 kernels and is compiled without fp
-// contraction, so that they round as the fp64 restatement does; the fp32
-// kernels are in sw_solver_f32.cu.
+// on the device, compiled without fp contraction.  The column kernels are in
+// sw_solver_f64.cu and sw_solver_f32.cu.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -195,6 +194,7 @@ int gb_sw_load(gb_lw_context* ctx, double cpdair, const char* table_dir) {
   if (e == cudaSuccess) e = cudaMemcpy(ctx->d_sw_tables_f, blobf.data(), blobf.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && upload) e = gbsw::sw_set_tab(S);
   if (e == cudaSuccess && upload) e = gb_sw_set_tab_f32(&S);
+  if (e == cudaSuccess && upload) e = gb_sw_set_tab_f64(&S);
   if (e != cudaSuccess) {
     drop_hold();
     return gb_ctx_fail(ctx, e, "SW tables");
@@ -217,7 +217,7 @@ long long gb_sw_slots(int num_sms, int bits) { return (long long)num_sms * (bits
 cudaError_t gb_sw_launch(const SwArgs& a, int bits, const void* d_tables, void* scratch, long long slots,
                          cudaStream_t stream) {
   if (bits == 32) return gb_sw_launch_f32(a, (const float*)d_tables, (float*)scratch, slots, stream);
-  return gbsw::sw_launch_t<double, SW_MINB_F64>(a, (const double*)d_tables, (double*)scratch, slots, stream);
+  return gb_sw_launch_f64(a, (const double*)d_tables, (double*)scratch, slots, stream);
 }
 
 // ------------------------------------------------------------------ cldprop_sw

@@ -55,3 +55,7 @@ cudaError_t gb_sw_launch(const SwArgs& a, int bits, const void* d_tables, void* 
 cudaError_t gb_sw_set_tab_f32(const void* tab);
 cudaError_t gb_sw_launch_f32(const SwArgs& a, const float* d_tables, float* scratch, long long slots,
                              cudaStream_t stream);
+// the fp64 kernels' unit (sw_solver_f64.cu): the same
+cudaError_t gb_sw_set_tab_f64(const void* tab);
+cudaError_t gb_sw_launch_f64(const SwArgs& a, const double* d_tables, double* scratch, long long slots,
+                             cudaStream_t stream);
