@@ -39,6 +39,13 @@ struct gb_lw_graph {
   unsigned* nfall = nullptr;
 };
 
+bool gb_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return false;
+}
+
 int gb_ctx_fail(gb_lw_context* c, cudaError_t e, const char* where) {
   if (c) c->last_error = std::string(where) + ": " + cudaGetErrorString(e);
   return GB_LW_E_CUDA;
@@ -140,17 +147,12 @@ cudaError_t copy2d(double* dst, size_t dpitch, const double* src, size_t spitch,
   return cudaMemcpy2DAsync(dst, dpitch * 8, src, spitch * 8, width * 8, rows, kind, s);
 }
 
-bool capturing(cudaStream_t s) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
-}
-
 // a gas-optics hand-over buffer of about `bytes` (grown on demand).  A buffer of
 // at least `least` bytes also does, with more passes per call: it is kept
 // under stream capture, where nothing can be allocated, and taken in place of
 // a larger one that does not fit on the device.
 int ensure_buffer(gb_lw_context* ctx, float** buf, size_t* have, size_t bytes, size_t least, cudaStream_t stream) {
-  if (*buf && (*have >= bytes || (*have >= least && capturing(stream)))) return 0;
+  if (*buf && (*have >= bytes || (*have >= least && gb_capturing(stream)))) return 0;
   cudaFree(*buf);
   *buf = nullptr;
   *have = 0;

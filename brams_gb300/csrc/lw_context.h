@@ -83,6 +83,8 @@ enum GbConstKind { GB_CONST_LW = 0, GB_CONST_SW = 1 };
 bool gb_const_acquire(int kind, int device, const void* bytes, size_t n, bool* upload);
 void gb_const_release(int kind, int device);
 
+// whether the stream is being captured (nothing can be allocated then)
+bool gb_capturing(cudaStream_t s);
 // records a CUDA error on the context; returns GB_LW_E_CUDA
 int gb_ctx_fail(gb_lw_context* c, cudaError_t e, const char* where);
 // validates a batched call's grids and fills the launch descriptor (frac < 1: sample of each grid)

@@ -2,6 +2,7 @@
 // rrtmg_sw (rrtmg_sw_init.f90:47, rrtmg_sw_rad.f90:243) on device or host arrays.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -64,20 +65,28 @@ int prepare(gb_lw_context* ctx, int ncol, int nlay, int* icld, int* iaer, double
 int launch(gb_lw_context* ctx, const SwArgs& a, cudaStream_t stream) {
   const int bits = ctx->sw_bits;
   const long long slots = gb_sw_slots(ctx->num_sms, bits);
-  const size_t need = gb_sw_scratch_bytes(a.nlay, bits, slots);
-  if (need > ctx->sw_scratch_bytes) {
+  const size_t need = gb_sw_scratch_bytes(a.nlay, bits, slots, a.ncol), least = gb_sw_scratch_bytes(a.nlay, bits, slots, 1);
+  // grown on demand; a smaller buffer, with more passes, is kept under stream
+  // capture and taken where the wanted one does not fit on the device
+  if (need > ctx->sw_scratch_bytes && !(least <= ctx->sw_scratch_bytes && gb_capturing(stream))) {
     cudaFree(ctx->d_sw_scratch);
     ctx->d_sw_scratch = nullptr;
     ctx->sw_scratch_bytes = 0;
-    if (cudaMalloc(&ctx->d_sw_scratch, need) != cudaSuccess) {
+    for (size_t n = need;; n = std::max(n / 2, least)) {
+      if (cudaMalloc(&ctx->d_sw_scratch, n) == cudaSuccess) {
+        ctx->sw_scratch_bytes = n;
+        break;
+      }
       cudaGetLastError();
-      ctx->last_error = "device allocation of the SW scratch slots failed";
-      return GB_LW_E_NOMEM;
+      ctx->d_sw_scratch = nullptr;
+      if (n <= least) {
+        ctx->last_error = "device allocation of the SW scratch slots failed";
+        return GB_LW_E_NOMEM;
+      }
     }
-    ctx->sw_scratch_bytes = need;
   }
   const void* tables = bits == 32 ? (const void*)ctx->d_sw_tables_f : (const void*)ctx->d_sw_tables;
-  cudaError_t e = gb_sw_launch(a, bits, tables, ctx->d_sw_scratch, slots, stream);
+  cudaError_t e = gb_sw_launch(a, bits, tables, ctx->d_sw_scratch, ctx->sw_scratch_bytes, slots, stream);
   return e == cudaSuccess ? GB_LW_OK : gb_ctx_fail(ctx, e, "SW column kernel");
 }
 

@@ -209,15 +209,15 @@ int gb_sw_load(gb_lw_context* ctx, double cpdair, const char* table_dir) {
   return GB_LW_OK;
 }
 
-size_t gb_sw_scratch_bytes(int nlay, int bits, long long slots) {
-  return (size_t)slots * (size_t)gbsw::sw_slot_elems(nlay) * (bits == 32 ? sizeof(float) : sizeof(double));
+size_t gb_sw_scratch_bytes(int nlay, int bits, long long slots, long long ncol) {
+  return bits == 32 ? gb_sw_scratch_f32(nlay, slots, ncol) : gb_sw_scratch_f64(nlay, slots, ncol);
 }
 long long gb_sw_slots(int num_sms, int bits) { return (long long)num_sms * (bits == 32 ? SW_MINB_F32 : SW_MINB_F64); }
 
-cudaError_t gb_sw_launch(const SwArgs& a, int bits, const void* d_tables, void* scratch, long long slots,
+cudaError_t gb_sw_launch(const SwArgs& a, int bits, const void* d_tables, void* scratch, size_t bytes, long long slots,
                          cudaStream_t stream) {
-  if (bits == 32) return gb_sw_launch_f32(a, (const float*)d_tables, (float*)scratch, slots, stream);
-  return gb_sw_launch_f64(a, (const double*)d_tables, (double*)scratch, slots, stream);
+  if (bits == 32) return gb_sw_launch_f32(a, (const float*)d_tables, scratch, bytes, slots, stream);
+  return gb_sw_launch_f64(a, (const double*)d_tables, scratch, bytes, slots, stream);
 }
 
 // ------------------------------------------------------------------ cldprop_sw

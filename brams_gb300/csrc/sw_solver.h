@@ -43,19 +43,23 @@ int gb_sw_load(gb_lw_context* ctx, double cpdair, const char* table_dir);
 // blocks per SM of the column kernel in each precision (its launch bounds)
 #define SW_MINB_F64 4
 #define SW_MINB_F32 6
-// persistent blocks (= scratch slots) for a device of num_sms SMs, and the
-// scratch bytes of `slots` slots, for a precision of 32 or 64 bits
+// persistent blocks for a device of num_sms SMs, and the scratch bytes of a
+// call of ncol columns with them (their records and the gas optics hand-over
+// of a pass of columns), for a precision of 32 or 64 bits; a call runs with
+// the bytes of any smaller ncol, in more passes
 long long gb_sw_slots(int num_sms, int bits);
-size_t gb_sw_scratch_bytes(int nlay, int bits, long long slots);
-// all columns of `a` with at most `slots` persistent blocks (block k uses slot
-// k of scratch); d_tables is the table blob of the precision (fp32 or fp64)
-cudaError_t gb_sw_launch(const SwArgs& a, int bits, const void* d_tables, void* scratch, long long slots,
+size_t gb_sw_scratch_bytes(int nlay, int bits, long long slots, long long ncol);
+// all columns of `a` with at most `slots` persistent blocks; d_tables is the
+// table blob of the precision (fp32 or fp64)
+cudaError_t gb_sw_launch(const SwArgs& a, int bits, const void* d_tables, void* scratch, size_t bytes, long long slots,
                          cudaStream_t stream);
-// the fp32 kernels' unit (sw_solver_f32.cu): its table directory (a gbsw::SwTab) and its launch
+// the fp32 kernels' unit (sw_solver_f32.cu): its table directory (a gbsw::SwTab), scratch and launch
 cudaError_t gb_sw_set_tab_f32(const void* tab);
-cudaError_t gb_sw_launch_f32(const SwArgs& a, const float* d_tables, float* scratch, long long slots,
+size_t gb_sw_scratch_f32(int nlay, long long slots, long long ncol);
+cudaError_t gb_sw_launch_f32(const SwArgs& a, const float* d_tables, void* scratch, size_t bytes, long long slots,
                              cudaStream_t stream);
 // the fp64 kernels' unit (sw_solver_f64.cu): the same
 cudaError_t gb_sw_set_tab_f64(const void* tab);
-cudaError_t gb_sw_launch_f64(const SwArgs& a, const double* d_tables, double* scratch, long long slots,
+size_t gb_sw_scratch_f64(int nlay, long long slots, long long ncol);
+cudaError_t gb_sw_launch_f64(const SwArgs& a, const double* d_tables, void* scratch, size_t bytes, long long slots,
                              cudaStream_t stream);

@@ -5,7 +5,11 @@
 
 cudaError_t gb_sw_set_tab_f64(const void* tab) { return gbsw::sw_set_tab(*static_cast<const gbsw::SwTab*>(tab)); }
 
-cudaError_t gb_sw_launch_f64(const SwArgs& a, const double* d_tables, double* scratch, long long slots,
+size_t gb_sw_scratch_f64(int nlay, long long slots, long long ncol) {
+  return gbsw::sw_scratch_bytes_t<double>(nlay, slots, ncol);
+}
+
+cudaError_t gb_sw_launch_f64(const SwArgs& a, const double* d_tables, void* scratch, size_t bytes, long long slots,
                              cudaStream_t stream) {
-  return gbsw::sw_launch_t<double, SW_MINB_F64>(a, d_tables, scratch, slots, stream);
+  return gbsw::sw_launch_t<double, SW_MINB_F64>(a, d_tables, scratch, bytes, slots, stream);
 }

@@ -1,0 +1,51 @@
+"""Shortwave calls through the gas optics planes: column counts around the
+32-column tiles, shallow and deep columns, very thin and very thick clouds, and
+a call that takes several passes."""
+import numpy as np
+import pytest
+
+import pyoracle
+from test_sw import BITS, _parity, _solve, sw_mcica, sw_state
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def swctx(ctx):
+    ctx.sw_ini(1004.0)
+    yield ctx
+    ctx.sw_set_precision(32)
+
+
+@pytest.mark.parametrize("bits", BITS)
+@pytest.mark.parametrize("ncol,nlay", [(1, 4), (31, 45), (32, 38), (33, 60), (65, 7), (5, 230)])
+def test_shapes_against_oracle(swctx, ncol, nlay, bits):
+    st = sw_state(ncol=ncol, nlay=nlay, seed=600 + ncol, cloud_prob=0.6)
+    mc = sw_mcica(st, seed=ncol)
+    ref = pyoracle.rrtmg_sw(st, mc, icld=3, iaer=10)
+    _parity(_solve(swctx, bits, st, mc, icld=3, iaer=10), ref, bits)
+
+
+@pytest.mark.parametrize("bits", BITS)
+def test_very_thin_and_very_thick_clouds(swctx, bits):
+    """Direct input: cloud optical depths of 1e-8 to 1e3 in neighbouring g-points."""
+    st = sw_state(ncol=40, nlay=33, seed=44, cloud_prob=0.8)
+    mc = sw_mcica(st, seed=3)
+    rng = np.random.default_rng(8)
+    mc["taucmcl"] = np.asfortranarray(mc["cldfmcl"] * 10.0 ** rng.uniform(-8.0, 3.0, mc["taucmcl"].shape))
+    ref = pyoracle.rrtmg_sw(st, mc, icld=2, iaer=10, inflgsw=0)
+    _parity(_solve(swctx, bits, st, mc, icld=2, iaer=10, inflgsw=0), ref, bits)
+
+
+@pytest.mark.parametrize("bits", BITS)
+def test_several_passes_repeat_their_columns(swctx, bits):
+    """131 columns of 128 layers, 115 times over (the planes hold about 14,000
+    columns in fp32, 7,000 in fp64): every copy has the bits of the first call."""
+    st = sw_state(ncol=131, nlay=128, seed=12)
+    one = _solve(swctx, bits, st, None, icld=0, iaer=0)
+    rep = {k: np.asfortranarray(np.concatenate([v] * 115, axis=0)) if getattr(v, "shape", (0,))[:1] == (131,) else v
+           for k, v in st.items()}
+    many = _solve(swctx, bits, rep, None, icld=0, iaer=0)
+    for k in ("swuflx", "swdflx", "swhr", "swuflxc", "swdflxc", "swhrc"):
+        v = one[k]
+        assert np.array_equal(many[k].reshape(115, 131, -1), np.broadcast_to(v, (115,) + v.shape)), k
