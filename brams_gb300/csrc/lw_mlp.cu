@@ -3,11 +3,9 @@
 // Training (hand-written, no library GEMM):
 //   gemm_kernel      bf16 tensor-core GEMM (mma.sync m16n8k16, fp32
 //                    accumulators) with transposes and fused epilogues:
-//                    bias+SiLU (forward hidden layers), bias (output layer),
-//                    *silu'(z) (backward), fp32 atomics (weight gradients,
-//                    split over the batch);
-//   loss_kernel      dL/dy of the weighted mean-square loss and the loss;
-//   colsum_kernel    bias gradients;
+//                    bias+SiLU (forward hidden layers), bias, loss and dL/dy
+//                    (output layer), *silu'(z) (backward), fp32 atomics
+//                    (weight and bias gradients, split over the batch);
 //   adam_kernel      Adam on fp32 master weights, writing the bf16 copy.
 // Inference:
 //   infer_kernel     the whole network per warp on 16 layers at a time, the
@@ -21,6 +19,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "lw_mlp.cuh"
 #include "lw_mlp.h"
 
@@ -29,7 +29,7 @@ using bf16 = __nv_bfloat16;
 namespace gbmlp {
 
 // ------------------------------------------------------------------ generic GEMM
-enum Epi { EPI_F32 = 0, EPI_ATOMIC = 1, EPI_BIAS_SILU = 2, EPI_BIAS_F32 = 3, EPI_DSILU = 4 };
+enum Epi { EPI_ATOMIC = 1, EPI_BIAS_SILU = 2, EPI_LOSS = 3, EPI_DSILU = 4 };
 
 struct GemmArgs {
   int M, N, K, ksplit;
@@ -38,22 +38,39 @@ struct GemmArgs {
   const bf16* B;
   long long ldb;  // BT = false: B[k * ldb + n]; BT = true: B[n * ldb + k]
   float* C;
-  long long ldc;  // fp32 output (EPI_F32, EPI_ATOMIC, EPI_BIAS_F32)
+  long long ldc;  // fp32 output (EPI_ATOMIC; EPI_LOSS, where not NULL)
   bf16* Z;
   bf16* Act;
-  long long ldz;  // EPI_BIAS_SILU: Z = acc + bias, Act = silu(acc + bias); EPI_DSILU: Z = acc * silu'(Zin)
+  long long ldz;  // EPI_BIAS_SILU: Z = acc + bias, Act = silu(acc + bias); EPI_DSILU: Z = acc * silu'(Zin);
+                  // EPI_LOSS: Z = dL/dy
   const float* bias;
   const bf16* Zin;
+  float* colsum;  // EPI_ATOMIC: += the column sums of B over this block's rows
+  const float *t, *w;
+  float* loss;    // EPI_LOSS: L = sum_j w_j (y_j - t_j)^2 / (rows * 280) over j < 280, added to loss where not NULL
 };
 
 constexpr int BM = 64, BN = 64, BK = 32, PAD = 8;
+constexpr int STAGES = 4;  // tiles of 32 along K in flight: a hidden layer's whole K
+
+// 16 bytes to shared memory; zeros where `on` is false (the address is not read)
+__device__ __forceinline__ void cp16(void* d, const void* g, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(d)), "l"(g), "r"(on ? 16 : 0) : "memory");
+}
+
+// What bounds it at the training batch (16,384 rows, layers of 16 to 288) is
+// latency: a block has four K steps at most but for the weight gradients, whose
+// K is the batch.  So the tiles are copied ahead of their use, and the weight
+// gradients are split into about four blocks per SM of 256 rows or more.  With one
+// tile at a time and 2,048 rows per block (8 to 80 blocks, 64 steps) a gradient
+// call took 558 us, of it the four weight gradients four fifths; now 139 us.
 
 template <bool AT, bool BT, int EPI>
 __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
   constexpr int SA = AT ? BK * (BM + PAD) : BM * (BK + PAD);
   constexpr int SB = BT ? BN * (BK + PAD) : BK * (BN + PAD);
-  __shared__ __align__(16) bf16 sA[SA];
-  __shared__ __align__(16) bf16 sB[SB];
+  __shared__ __align__(16) bf16 tA[STAGES][SA];
+  __shared__ __align__(16) bf16 tB[STAGES][SB];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 1, wn = warp & 1;
   const int bm = blockIdx.y * BM, bn = blockIdx.x * BN;
@@ -66,27 +83,48 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0f;
 
-  for (int kb = k0; kb < k1; kb += BK) {
-    // ---- stage A and B tiles (8 bf16 per vector; all extents are multiples of 8)
-    for (int v = tid; v < BM * BK / 8; v += 128) {
-      int r, c;  // r: row of the staged tile, c: first column
-      if (AT) { r = v / (BM / 8); c = (v % (BM / 8)) * 8; }  // [BK][BM]
-      else { r = v / (BK / 8); c = (v % (BK / 8)) * 8; }     // [BM][BK]
-      const int m = AT ? bm + c : bm + r, k = AT ? kb + r : kb + c;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (m < g.M && k < k1) val = *reinterpret_cast<const uint4*>(AT ? g.A + (long long)k * g.lda + m : g.A + (long long)m * g.lda + k);
-      *reinterpret_cast<uint4*>(sA + r * ((AT ? BM : BK) + PAD) + c) = val;
+  // ---- a K step's A and B tiles (8 bf16 per copy; all extents are multiples of 8)
+  auto stage = [&](int step) {
+    const int kb = k0 + step * BK;
+    bf16 *sA = tA[step % STAGES], *sB = tB[step % STAGES];
+    if (kb < k1) {
+#pragma unroll
+      for (int v = tid; v < BM * BK / 8; v += 128) {
+        int r, c;  // r: row of the staged tile, c: first column
+        if (AT) { r = v / (BM / 8); c = (v % (BM / 8)) * 8; }  // [BK][BM]
+        else { r = v / (BK / 8); c = (v % (BK / 8)) * 8; }     // [BM][BK]
+        const int m = AT ? bm + c : bm + r, k = AT ? kb + r : kb + c;
+        const bool on = m < g.M && k < k1;
+        cp16(sA + r * ((AT ? BM : BK) + PAD) + c,
+             on ? (AT ? g.A + (long long)k * g.lda + m : g.A + (long long)m * g.lda + k) : g.A, on);
+      }
+#pragma unroll
+      for (int v = tid; v < BN * BK / 8; v += 128) {
+        int r, c;
+        if (BT) { r = v / (BK / 8); c = (v % (BK / 8)) * 8; }  // [BN][BK]
+        else { r = v / (BN / 8); c = (v % (BN / 8)) * 8; }     // [BK][BN]
+        const int n = BT ? bn + r : bn + c, k = BT ? kb + c : kb + r;
+        const bool on = n < g.N && k < k1;
+        cp16(sB + r * ((BT ? BK : BN) + PAD) + c,
+             on ? (BT ? g.B + (long long)n * g.ldb + k : g.B + (long long)k * g.ldb + n) : g.B, on);
+      }
     }
-    for (int v = tid; v < BN * BK / 8; v += 128) {
-      int r, c;
-      if (BT) { r = v / (BK / 8); c = (v % (BK / 8)) * 8; }  // [BN][BK]
-      else { r = v / (BN / 8); c = (v % (BN / 8)) * 8; }     // [BK][BN]
-      const int n = BT ? bn + r : bn + c, k = BT ? kb + c : kb + r;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (n < g.N && k < k1) val = *reinterpret_cast<const uint4*>(BT ? g.B + (long long)n * g.ldb + k : g.B + (long long)k * g.ldb + n);
-      *reinterpret_cast<uint4*>(sB + r * ((BT ? BK : BN) + PAD) + c) = val;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const bool sums = EPI == EPI_ATOMIC && blockIdx.y == 0;
+  float cs[4] = {};  // sums over rows 4 i + q of this thread's half of the B tiles' rows
+#pragma unroll
+  for (int i = 0; i < STAGES - 1; ++i) stage(i);
+  for (int step = 0; k0 + step * BK < k1; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();  // the tile is there, and all are done with the one that the next copy replaces
+    stage(step + STAGES - 1);
+    const bf16 *sA = tA[step % STAGES], *sB = tB[step % STAGES];
+    if (sums) {
+#pragma unroll
+      for (int r = 0; r < BK / 2; ++r)
+        cs[r & 3] += __bfloat162float(sB[((tid >> 6) * (BK / 2) + r) * (BN + PAD) + (tid & 63)]);
     }
-    __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 16) {
       uint32_t af[2][4], bfr[4][2];
@@ -117,9 +155,12 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
 #pragma unroll
         for (int ni = 0; ni < 4; ++ni) mma16816(acc[mi][ni], af[mi], bfr[ni][0], bfr[ni][1]);
     }
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   // ---- epilogue
+  if (sums && bn + (tid & 63) < g.N) atomicAdd(g.colsum + bn + (tid & 63), (cs[0] + cs[1]) + (cs[2] + cs[3]));
+  const float scale = EPI == EPI_LOSS ? 1.0f / ((float)g.M * (float)GB_MLP_NOUT) : 0.0f;
+  float part = 0.0f;  // this thread's part of the loss
   const int gq = lane >> 2, tq = lane & 3;
 #pragma unroll
   for (int mi = 0; mi < 2; ++mi)
@@ -131,13 +172,20 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
         const int n = bn + wn * 32 + ni * 8 + 2 * tq;
         if (m >= g.M || n >= g.N) continue;
         const float v0 = acc[mi][ni][2 * h], v1 = acc[mi][ni][2 * h + 1];
-        if (EPI == EPI_F32) {
-          *reinterpret_cast<float2*>(g.C + (long long)m * g.ldc + n) = make_float2(v0, v1);
-        } else if (EPI == EPI_ATOMIC) {
+        if (EPI == EPI_ATOMIC) {
           atomicAdd(g.C + (long long)m * g.ldc + n, v0);
           atomicAdd(g.C + (long long)m * g.ldc + n + 1, v1);
-        } else if (EPI == EPI_BIAS_F32) {
-          *reinterpret_cast<float2*>(g.C + (long long)m * g.ldc + n) = make_float2(v0 + g.bias[n], v1 + g.bias[n + 1]);
+        } else if (EPI == EPI_LOSS) {
+          const float y0 = v0 + g.bias[n], y1 = v1 + g.bias[n + 1];
+          float d0 = 0.0f, d1 = 0.0f;
+          if (n < GB_MLP_NOUT) {  // an even number of outputs: a pair is in or out
+            const float* t = g.t + (long long)m * g.N + n;
+            const float w0 = g.w[n], w1 = g.w[n + 1], e0 = y0 - t[0], e1 = y1 - t[1];
+            d0 = 2.0f * w0 * e0 * scale, d1 = 2.0f * w1 * e1 * scale;
+            part += w0 * e0 * e0 * scale + w1 * e1 * e1 * scale;
+          }
+          if (g.C) *reinterpret_cast<float2*>(g.C + (long long)m * g.ldc + n) = make_float2(y0, y1);
+          *reinterpret_cast<uint32_t*>(g.Z + (long long)m * g.ldz + n) = pack_bf16(d0, d1);
         } else if (EPI == EPI_BIAS_SILU) {
           const float z0 = v0 + g.bias[n], z1 = v1 + g.bias[n + 1];
           *reinterpret_cast<uint32_t*>(g.Z + (long long)m * g.ldz + n) = pack_bf16(z0, z1);
@@ -148,6 +196,13 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
           *reinterpret_cast<uint32_t*>(g.Z + (long long)m * g.ldz + n) = pack_bf16(v0 * dsilu(zf.x), v1 * dsilu(zf.y));
         }
       }
+  if (EPI == EPI_LOSS && g.loss) {
+    __shared__ float red[4];
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) red[warp] = part;
+    __syncthreads();
+    if (tid == 0) atomicAdd(g.loss, (red[0] + red[1]) + (red[2] + red[3]));
+  }
 }
 
 template <bool AT, bool BT, int EPI>
@@ -162,50 +217,6 @@ cudaError_t gemm(const GemmArgs& a0, int splits, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ elementwise
-// dL/dy and the loss of L = sum_j w_j (y_j - t_j)^2 / (rows * 280), j < 280
-__global__ void loss_kernel(long long rows, const float* __restrict__ y, const float* __restrict__ t,
-                            const float* __restrict__ w, bf16* __restrict__ dy, float* __restrict__ loss) {
-  __shared__ float red[32];
-  const long long n = rows * GB_MLP_NOUTP;
-  const float scale = 1.0f / ((float)rows * (float)GB_MLP_NOUT);
-  float part = 0.0f;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(i % GB_MLP_NOUTP);
-    float d = 0.0f;
-    if (j < GB_MLP_NOUT) {
-      const float e = y[i] - t[i];
-      d = 2.0f * w[j] * e * scale;
-      part += w[j] * e * e * scale;
-    }
-    dy[i] = __float2bfloat16_rn(d);
-  }
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0 && loss) atomicAdd(loss, v);
-  }
-}
-
-// out[n] += sum over rows of x[m][n] (bias gradients); one block per 32 columns x 256-row slab
-__global__ void colsum_kernel(long long rows, int N, const bf16* __restrict__ x, float* __restrict__ out) {
-  const int n = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int ry = threadIdx.x >> 5;  // 8 row lanes
-  float s = 0.0f;
-  if (n < N)
-    for (long long m = blockIdx.y * 256 + ry; m < rows && m < (blockIdx.y + 1) * 256LL; m += 8) s += __bfloat162float(x[m * N + n]);
-  __shared__ float red[8][33];
-  red[ry][threadIdx.x & 31] = s;
-  __syncthreads();
-  if (ry == 0 && n < N) {
-    float t = 0.0f;
-    for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x & 31];
-    atomicAdd(out + n, t);
-  }
-}
-
 __global__ void adam_kernel(int n, float* __restrict__ p, const float* __restrict__ grad, float* __restrict__ m,
                             float* __restrict__ v, bf16* __restrict__ p16, float lr, float b1, float b2, float eps,
                             float c1, float c2) {
@@ -447,7 +458,7 @@ cudaError_t gb_mlp_norm_targets(long long rows, const float* d_tau, const float*
 }
 
 cudaError_t gb_mlp_forward_backward(const MlpBuffers& b, long long rows, const bf16* d_x, const float* d_t,
-                                    const float* d_w, float* d_grad, float* d_loss, cudaStream_t st) {
+                                    const float* d_w, float* d_grad, float* d_loss, bool keep_y, cudaStream_t st) {
   const int H = GB_MLP_H, O = GB_MLP_NOUTP;
   const int M = (int)rows;
   cudaError_t e;
@@ -471,13 +482,12 @@ cudaError_t gb_mlp_forward_backward(const MlpBuffers& b, long long rows, const b
   a.M = M; a.N = O; a.K = H;
   a.A = b.act[2]; a.lda = H;
   a.B = W[3]; a.ldb = O;
-  a.C = b.y; a.ldc = O; a.bias = Bs[3];
-  if ((e = gemm<false, false, EPI_BIAS_F32>(a, 1, st)) != cudaSuccess) return e;
-  loss_kernel<<<1024, 256, 0, st>>>(rows, b.y, d_t, d_w, b.dy, d_loss);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  a.C = keep_y ? b.y : nullptr; a.ldc = O; a.bias = Bs[3];
+  a.Z = b.dy; a.ldz = O;
+  a.t = d_t; a.w = d_w; a.loss = d_loss;
+  if ((e = gemm<false, false, EPI_LOSS>(a, 1, st)) != cudaSuccess) return e;
   // backward
   if ((e = cudaMemsetAsync(d_grad, 0, GB_MLP_NPARAM * sizeof(float), st)) != cudaSuccess) return e;
-  const int splits = (int)((rows + 2047) / 2048);
   const bf16* dZ = b.dy;
   int nout = O;
   float* gW[4] = {d_grad + GB_MLP_OFF_W1, d_grad + GB_MLP_OFF_W2, d_grad + GB_MLP_OFF_W3, d_grad + GB_MLP_OFF_W4};
@@ -491,9 +501,11 @@ cudaError_t gb_mlp_forward_backward(const MlpBuffers& b, long long rows, const b
     a.A = Ain; a.lda = kin_l;
     a.B = dZ; a.ldb = nout;
     a.C = gW[l]; a.ldc = nout;
+    a.colsum = gB[l];
+    // about four blocks per SM, of 256 rows or more
+    const int tiles = ((kin_l + BM - 1) / BM) * ((nout + BN - 1) / BN);
+    const int splits = (int)std::min((rows + 255) / 256, (long long)(608 / tiles));
     if ((e = gemm<true, false, EPI_ATOMIC>(a, splits, st)) != cudaSuccess) return e;
-    colsum_kernel<<<dim3((nout + 31) / 32, (unsigned)((rows + 255) / 256)), 256, 0, st>>>(rows, nout, dZ, gB[l]);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (l == 0) break;
     // dZ_{l-1} = (dZ_l W_l^T) * silu'(Z_{l-1})
     a = GemmArgs{};
