@@ -5,15 +5,16 @@
 // or KISS (irng=0) sequence in a fixed loop order and marks sub-column isub
 // of layer ilev cloudy when CDF >= 1 - cldf (:650).  The GPU reproduces the
 // draws bit for bit:
-//   * draw generation -- one thread per column for per-column seeds (the
-//     reference called with ncol = 1 and seed = base + column), or one block
-//     stepping the single sequence 624 words at a time for the reference's
-//     all-columns call (draw order isub, column, layer);
-//   * CDF construction and the cloudy test in double precision, one thread
-//     per (column, sub-column), layers in order (max-random and exponential
-//     overlap carry CDF from one layer to the next).
+//   * draw generation -- per column for per-column seeds (the reference called
+//     with ncol = 1 and seed = base + column), or one block stepping the single
+//     sequence 624 words at a time for the reference's all-columns call (draw
+//     order isub, column, layer);
+//   * CDF construction and the cloudy test in double precision, a thread per
+//     column and pair of sub-columns, layers in order (max-random and
+//     exponential overlap carry CDF from one layer to the next).
 // Draws are kept as doubles exactly as getRandomReal/kissvec return them.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include <mutex>
@@ -32,56 +33,65 @@ __device__ __forceinline__ uint32_t mt_temper(uint32_t y) { return gbmt::temper(
 __device__ __forceinline__ uint32_t mt_twist(uint32_t u, uint32_t v) { return gbmt::twist(u, v); }
 __device__ __forceinline__ double mt_real(uint32_t u) { return gbmt::real(u); }
 
-// Full-state generator for longer per-column sequences.
-struct MtState {
-  uint32_t s[624];
-  int cur;
-};
-__device__ void mt_init(MtState& m, uint32_t seed) {
-  m.s[0] = seed;
-  for (int i = 1; i < 624; ++i) m.s[i] = 1812433253u * (m.s[i - 1] ^ (m.s[i - 1] >> 30)) + (uint32_t)i;
-  m.cur = 624;
-}
-__device__ uint32_t mt_next(MtState& m) {
-  if (m.cur >= 624) {
-    for (int k = 0; k < 227; ++k) m.s[k] = m.s[k + 397] ^ mt_twist(m.s[k], m.s[k + 1]);
-    for (int k = 227; k < 623; ++k) m.s[k] = m.s[k - 227] ^ mt_twist(m.s[k], m.s[k + 1]);
-    m.s[623] = m.s[396] ^ mt_twist(m.s[623], m.s[0]);
-    m.cur = 0;
+// The first n outputs of per-column seeds (column c: seed0 + c), draws[c * n + k].
+// They need the initial state's words 0..n and 397..396+n only (nextState's
+// first loop; n <= 227).  A block has 32 columns: a lane of its first warp walks a
+// column's initialisation, a chain of 536 dependent steps, and leaves those
+// words in shared memory; all threads then temper them and write the rows.
+// The chain bounds it (some 4 us).  One thread per column for both parts took 54 us
+// for 8,192 columns, most of it in fp64 divisions, which also issue one by one
+// (a solver call of 64 columns, draws included: 122 us, now 80 us).
+constexpr int MT_NT = 256;
+constexpr int MT_MAX = 181;  // (2 n + 1) words of 33 columns in 48 KB
+__global__ void __launch_bounds__(MT_NT) mt_percol_kernel(int ncol, uint32_t seed0, int n, double* __restrict__ draws) {
+  extern __shared__ uint32_t word[];  // [2 n + 1][33]
+  const long long c0 = blockIdx.x * 32LL;
+  if (threadIdx.x < 32) {
+    uint32_t s = seed0 + (uint32_t)c0 + threadIdx.x;
+    uint32_t* w = word + threadIdx.x;
+    w[0] = s;
+    auto next = [&](int i) { s = 1812433253u * (s ^ (s >> 30)) + (uint32_t)i; };
+#pragma unroll 8
+    for (int i = 1; i <= n; ++i) {
+      next(i);
+      w[33 * i] = s;
+    }
+#pragma unroll 8
+    for (int i = n + 1; i < 397; ++i) next(i);
+    w += 33 * (n + 1);
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) {
+      next(397 + k);
+      w[33 * k] = s;
+    }
   }
-  return mt_temper(m.s[m.cur++]);
+  __syncthreads();
+  const int nc = (int)min(32LL, ncol - c0);
+  double* out = draws + c0 * n;
+  for (int i = threadIdx.x; i < nc * n; i += MT_NT) {
+    const int c = i / n, k = i - c * n;
+    const uint32_t* w = word + c + 33 * k;
+    out[i] = mt_real(mt_temper(w[33 * (n + 1)] ^ mt_twist(w[0], w[33])));
+  }
 }
 
-// per-column seeds: column c uses seed0 + c; draws[c * ndraw + k]
-__global__ void mt_percol_kernel(int ncol, int seed0, int ndraw, double* __restrict__ draws) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncol) return;
-  double* out = draws + (long long)c * ndraw;
-  uint32_t seed = (uint32_t)(seed0 + c);
-  if (ndraw <= 226) {
-    uint32_t lo[227];
-    gbmt::first_reals(seed, ndraw, lo, out, 1);
-    return;
-  }
-  MtState m;
-  mt_init(m, seed);
-  for (int k = 0; k < ndraw; ++k) out[k] = mt_real(mt_next(m));
-}
-
-// one sequence for the whole call: a single block keeps the 624-word state in
-// shared memory and produces it one twist (624 draws) at a time.
-__global__ void __launch_bounds__(256) mt_stream_kernel(uint32_t seed, long long ndraw, double* __restrict__ draws) {
+// One sequence per block, seeded with seed0 + block: a block keeps the 624-word
+// state in shared memory and produces it one twist (624 draws) at a time.  One
+// block for the reference's own call, else a block per column.
+__global__ void __launch_bounds__(256) mt_stream_kernel(uint32_t seed0, long long ndraw, double* __restrict__ draws) {
   __shared__ uint32_t st[624];
   __shared__ uint32_t nw[624];
   if (threadIdx.x == 0) {
-    uint32_t s = seed;
+    uint32_t s = seed0 + blockIdx.x;
     st[0] = s;
+#pragma unroll 7
     for (int i = 1; i < 624; ++i) {
       s = 1812433253u * (s ^ (s >> 30)) + (uint32_t)i;
       st[i] = s;
     }
   }
   __syncthreads();
+  draws += blockIdx.x * ndraw;
   for (long long base = 0; base < ndraw; base += 624) {
     // nextState (:127-139): words 0..226 from old words, 227..622 from new 0..395, 623 from new 396 and new 0
     for (int k = threadIdx.x; k < 227; k += blockDim.x) nw[k] = st[k + 397] ^ mt_twist(st[k], st[k + 1]);
@@ -164,89 +174,137 @@ __global__ void kiss_percol_kernel(int ncol, long long ld, const double* __restr
 }
 
 // ---------------------------------------------------------------- CDF + outputs
-// One block per column, one thread per sub-column.  `draw(isub, ilev, which)`
-// locates the draw the reference would use for that cell.
-__global__ void mcica_fill_kernel(McicaArgs a, const double* __restrict__ draws) {
-  const int c = blockIdx.x;
-  const int isub = threadIdx.x;
-  if (c >= a.ncol || isub >= a.nsub) return;
-  const int nlay = a.nlay;
+// A block has FILL_C neighbouring columns, whose rows lie side by side in the
+// outputs, and a thread one of their pairs of sub-columns; the layers come in
+// chunks of FILL_L, whose thresholds, water paths and optical properties are
+// staged in shared memory.  `D(ilev, which)` locates the draw the reference would
+// use for a cell.  What bounds it is the write of the sub-column arrays.  The
+// random draws are in [0, 1], so cdf >= 1 - cldf is a comparison of the bit
+// patterns as integers, a negative threshold takes every cell and a NaN none: a
+// double comparison, difference and maximum at 1/64 of the integer rate per cell kept
+// the fp64 pipe half busy (36,000 columns of 45 layers, draws included: 2.54 ms,
+// now 1.22 ms; the writes are 7.3 GB).
+constexpr int FILL_C = 4, FILL_L = 16;
+struct FillCell {
+  long long key;  // 1 - cldf for the integer comparison
+  double omc;     // 1 - cldf
+  double clwp, ciwp;
+};
+
+template <bool RANDOM_MAX>  // icld 3: the same draw in all layers
+__global__ void __launch_bounds__(FILL_C * 70) mcica_fill_kernel(McicaArgs a, const double* __restrict__ draws, bool wide) {
+  __shared__ FillCell cells[FILL_L][FILL_C];
+  extern __shared__ double optics[];  // [1 or 4: tauc, ssac, asmc, fsfc][FILL_L][FILL_C][nbnd]
+  const int np = a.nsub / 2, nt = FILL_C * np, tid = threadIdx.x;
+  const int cc = tid / np, isub = 2 * (tid - cc * np);
+  const long long c0 = (long long)blockIdx.x * FILL_C;
+  const int nc = (int)min((long long)FILL_C, a.ncol - c0);
+  const bool on = cc < nc;
+  const long long c = c0 + (on ? cc : 0);
+  const int nlay = a.nlay, nbnd = a.nbnd;
   const long long ld = a.ld;
-  auto D = [&](int ilev, int which) -> double {
+  const bool sw = a.ssacmcl != nullptr;
+  auto D = [&](int is, int ilev, int which) -> double {
     long long idx;
     if (a.mode == MCICA_STREAM_MT) {
       // one sequence over the call: loop order isub, column, layer (:476-645)
       long long ncol = a.ncol;
-      if (a.icld == 3) idx = (long long)isub * ncol + c;
-      else if (a.icld <= 2) idx = ((long long)isub * ncol + c) * nlay + ilev;
-      else idx = 2 * (((long long)isub * ncol + c) * nlay + ilev) + which;
+      if (RANDOM_MAX) idx = (long long)is * ncol + c;
+      else if (a.icld <= 2) idx = ((long long)is * ncol + c) * nlay + ilev;
+      else idx = 2 * (((long long)is * ncol + c) * nlay + ilev) + which;
       return draws[idx];
     }
     // per-column sequences (MT with per-column seeds, or KISS)
-    long long base = (long long)c * a.ndraw_per_col;
-    if (a.icld == 3) idx = isub;
-    else if (a.icld <= 2) idx = (long long)isub * nlay + ilev;
-    else idx = 2 * ((long long)isub * nlay + ilev) + which;
-    if (a.mode == MCICA_PERCOL_KISS && a.icld <= 2) idx = (long long)isub * nlay + ilev;
+    long long base = c * a.ndraw_per_col;
+    if (RANDOM_MAX) idx = is;
+    else if (a.icld <= 2) idx = (long long)is * nlay + ilev;
+    else idx = 2 * ((long long)is * nlay + ilev) + which;
     return draws[base + idx];
   };
-  auto cldf_at = [&](int ilev) {
-    double v = a.cldfrac[c + ld * ilev];
-    return v < 1.0e-20 ? 0.0 : v;
-  };
-  double cdf_prev = 0.0;
-  for (int ilev = 0; ilev < nlay; ++ilev) {
-    double cdf;
-    if (a.icld == 3) {
-      cdf = D(0, 0);
-    } else if (a.icld <= 2) {
-      cdf = D(ilev, 0);
-      if (a.icld == 2 && ilev > 0) {
-        double cp = cldf_at(ilev - 1);
-        cdf = (cdf_prev > 1.0 - cp) ? cdf_prev : cdf * (1.0 - cp);  // :528-537
-      }
-    } else {
-      cdf = D(ilev, 0);
-      double cdf2 = D(ilev, 1);
-      if (ilev > 0 && cdf2 < a.alpha[c + ld * ilev]) cdf = cdf_prev;  // :626-630, 639-643
-    }
-    cdf_prev = cdf;
-    bool cloudy = cdf >= 1.0 - cldf_at(ilev);
-    long long o = (long long)isub + a.nsub * ((long long)c + ld * ilev);
-    long long oc = c + ld * ilev;
-    // the band of the sub-column's optical properties (mcica_subcol_gen_sw.f90:
-    // n = ngb(isubcol) - ngbm; the longwave one uses ngb itself)
-    const long long ob = (a.ngb[isub] - a.band0 - 1) + (long long)a.nbnd * (c + ld * (long long)ilev);
-    if (cloudy) {
-      a.cldfmcl[o] = 1.0;
-      a.clwpmcl[o] = a.clwp[oc];
-      a.ciwpmcl[o] = a.ciwp[oc];
-      a.taucmcl[o] = a.tauc[ob];
-      if (a.ssacmcl) {
-        a.ssacmcl[o] = a.ssac[ob];
-        a.asmcmcl[o] = a.asmc[ob];
-        a.fsfcmcl[o] = a.fsfc[ob];
-      }
-    } else {
-      a.cldfmcl[o] = 0.0;
-      a.clwpmcl[o] = 0.0;
-      a.ciwpmcl[o] = 0.0;
-      a.taucmcl[o] = 0.0;
-      if (a.ssacmcl) {
-        a.ssacmcl[o] = 1.0;
-        a.asmcmcl[o] = 0.0;
-        a.fsfcmcl[o] = 0.0;
-      }
-    }
-  }
-  // reicmcl / relqmcl copies (:264-265)
-  if (isub == 0) {
-    for (int ilev = 0; ilev < nlay; ++ilev) {
-      long long oc = c + ld * ilev;
-      a.reicmcl[oc] = a.rei[oc];
+  // the band of the sub-column's optical properties (mcica_subcol_gen_sw.f90:
+  // n = ngb(isubcol) - ngbm; the longwave one uses ngb itself)
+  const int b0 = a.ngb[isub] - a.band0 - 1, b1 = a.ngb[isub + 1] - a.band0 - 1;
+  double cdf[2] = {0.0, 0.0}, omp = 0.0;  // the CDF and 1 - cldf of the layer below
+  if (RANDOM_MAX) cdf[0] = D(isub, 0, 0), cdf[1] = D(isub + 1, 0, 0);
+  const long long row = a.nsub * ld;  // of a layer
+  long long o = isub + a.nsub * c;
+  const int nopt = FILL_L * FILL_C * nbnd;
+  for (int l0 = 0; l0 < nlay; l0 += FILL_L) {
+    const int n = min(FILL_L, nlay - l0);
+    __syncthreads();
+    for (int i = tid; i < n * FILL_C; i += nt) {
+      const int l = i / FILL_C, k = i % FILL_C;
+      if (k >= nc) continue;
+      const long long oc = c0 + k + ld * (l0 + l);
+      const double v = a.cldfrac[oc], omc = 1.0 - (v < 1.0e-20 ? 0.0 : v);
+      FillCell& f = cells[l][k];
+      f.key = omc < 0.0 ? LLONG_MIN : (omc == omc ? __double_as_longlong(omc) : LLONG_MAX);
+      f.omc = omc;
+      f.clwp = a.clwp[oc];
+      f.ciwp = a.ciwp[oc];
+      a.reicmcl[oc] = a.rei[oc];  // reicmcl / relqmcl copies (:264-265)
       a.relqmcl[oc] = a.rel[oc];
     }
+    for (int i = tid; i < n * nc * nbnd; i += nt) {
+      const int l = i / (nc * nbnd), r = i - l * (nc * nbnd);  // r: column and band
+      const long long ob = r + nbnd * (c0 + ld * (l0 + l));
+      double* d = optics + l * (FILL_C * nbnd) + r;
+      d[0] = a.tauc[ob];
+      if (sw) d[nopt] = a.ssac[ob], d[2 * nopt] = a.asmc[ob], d[3 * nopt] = a.fsfc[ob];
+    }
+    __syncthreads();
+    if (!on) continue;
+#pragma unroll 4
+    for (int l = 0; l < n; ++l, o += row) {
+      const FillCell& f = cells[l][cc];
+      bool y[2];
+      if (RANDOM_MAX) {
+        y[0] = __double_as_longlong(cdf[0]) >= f.key, y[1] = __double_as_longlong(cdf[1]) >= f.key;
+      } else {
+        const int ilev = l0 + l;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          double v = D(isub + q, ilev, 0);
+          if (a.icld <= 2) {
+            if (a.icld == 2 && ilev > 0) v = (cdf[q] > omp) ? cdf[q] : v * omp;  // :528-537
+          } else {
+            const double v2 = D(isub + q, ilev, 1);
+            if (ilev > 0 && v2 < a.alpha[c + ld * ilev]) v = cdf[q];  // :626-630, 639-643
+          }
+          cdf[q] = v;
+          y[q] = v >= f.omc;
+        }
+        omp = f.omc;
+      }
+      auto put = [&](double* p, double v0, double v1) {
+        if (wide) {
+          *reinterpret_cast<double2*>(p + o) = make_double2(v0, v1);
+        } else {
+          p[o] = v0;
+          p[o + 1] = v1;
+        }
+      };
+      auto sel = [&](double* p, double v0, double v1, double off) { put(p, y[0] ? v0 : off, y[1] ? v1 : off); };
+      const double *t0 = optics + (l * FILL_C + cc) * nbnd + b0, *t1 = t0 + (b1 - b0);
+      sel(a.cldfmcl, 1.0, 1.0, 0.0);
+      sel(a.clwpmcl, f.clwp, f.clwp, 0.0);
+      sel(a.ciwpmcl, f.ciwp, f.ciwp, 0.0);
+      sel(a.taucmcl, t0[0], t1[0], 0.0);
+      if (sw) {
+        sel(a.ssacmcl, t0[nopt], t1[nopt], 1.0);
+        sel(a.asmcmcl, t0[2 * nopt], t1[2 * nopt], 0.0);
+        sel(a.fsfcmcl, t0[3 * nopt], t1[3 * nopt], 0.0);
+      }
+    }
   }
+}
+
+// the Mersenne-twister draws of per-column seeds
+static void percol_mt(int ncol, uint32_t seed0, int ndraw, double* draws, cudaStream_t stream) {
+  if (ndraw <= MT_MAX)
+    mt_percol_kernel<<<(ncol + 31) / 32, MT_NT, (2 * ndraw + 1) * 33 * sizeof(uint32_t), stream>>>(ncol, seed0, ndraw, draws);
+  else
+    mt_stream_kernel<<<ncol, 256, 0, stream>>>(seed0, ndraw, draws);
 }
 
 }  // namespace gbm
@@ -257,7 +315,7 @@ cudaError_t gb_mcica_launch(const McicaArgs& a, double* d_draws, int* d_err, cud
   const int per = a.icld == 3 ? 1 : (a.icld <= 2 ? a.nlay : 2 * a.nlay);
   const int ndraw = a.nsub * per;
   if (a.mode == MCICA_PERCOL_MT) {
-    gbm::mt_percol_kernel<<<(a.ncol + 127) / 128, 128, 0, stream>>>(a.ncol, a.seed, ndraw, d_draws);
+    gbm::percol_mt(a.ncol, (uint32_t)a.seed, ndraw, d_draws, stream);
   } else if (a.mode == MCICA_STREAM_MT) {
     gbm::mt_stream_kernel<<<1, 256, 0, stream>>>((uint32_t)a.seed, (long long)ndraw * a.ncol, d_draws);
   } else {
@@ -269,13 +327,21 @@ cudaError_t gb_mcica_launch(const McicaArgs& a, double* d_draws, int* d_err, cud
   if (e != cudaSuccess) return e;
   McicaArgs b = a;
   b.ndraw_per_col = ndraw;
-  gbm::mcica_fill_kernel<<<a.ncol, 160, 0, stream>>>(b, d_draws);
+  // 16-byte stores where the arrays start on such a boundary (rows are 1,120 or 896 bytes)
+  uintptr_t at = 0;
+  for (const double* p : {b.cldfmcl, b.clwpmcl, b.ciwpmcl, b.taucmcl, b.ssacmcl, b.asmcmcl, b.fsfcmcl}) at |= (uintptr_t)p;
+  const unsigned blocks = (unsigned)((b.ncol + gbm::FILL_C - 1) / gbm::FILL_C), nt = gbm::FILL_C * (b.nsub / 2);
+  const size_t smem = (size_t)(b.ssacmcl ? 4 : 1) * gbm::FILL_L * gbm::FILL_C * b.nbnd * sizeof(double);
+  if (b.icld == 3)
+    gbm::mcica_fill_kernel<true><<<blocks, nt, smem, stream>>>(b, d_draws, (at & 15) == 0);
+  else
+    gbm::mcica_fill_kernel<false><<<blocks, nt, smem, stream>>>(b, d_draws, (at & 15) == 0);
   return cudaGetLastError();
 }
 
 cudaError_t gb_mcica_percol_mt(int ncol, unsigned seed0, int ndraw, double* d_draws, cudaStream_t stream) {
   if (ncol <= 0) return cudaSuccess;
-  gbm::mt_percol_kernel<<<(ncol + 127) / 128, 128, 0, stream>>>(ncol, (int)seed0, ndraw, d_draws);
+  gbm::percol_mt(ncol, seed0, ndraw, d_draws, stream);
   return cudaGetLastError();
 }
 

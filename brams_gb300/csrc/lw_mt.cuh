@@ -15,23 +15,17 @@ __device__ __forceinline__ uint32_t temper(uint32_t y) {
 __device__ __forceinline__ uint32_t twist(uint32_t u, uint32_t v) {
   return (((u & 0x80000000u) | (v & 0x7fffffffu)) >> 1) ^ ((v & 1u) ? 0x9908b0dfu : 0u);
 }
-__device__ __forceinline__ double real(uint32_t u) { return (double)u / 4294967295.0; }
-
-// First n <= 226 outputs of MT(seed) as getRandomReal values.  They need the
-// initial state words 0..n and 397..396+n only (nextState's first loop).
-// lo must hold n+1 words of scratch.
-__device__ inline void first_reals(uint32_t seed, int n, uint32_t* lo, double* out, int stride) {
-  uint32_t s = seed;
-  lo[0] = s;
-  for (int i = 1; i <= n; ++i) {
-    s = 1812433253u * (s ^ (s >> 30)) + (uint32_t)i;
-    lo[i] = s;
-  }
-  for (int i = n + 1; i < 397; ++i) s = 1812433253u * (s ^ (s >> 30)) + (uint32_t)i;
-  for (int k = 0; k < n; ++k) {
-    s = 1812433253u * (s ^ (s >> 30)) + (uint32_t)(397 + k);  // word 397 + k
-    out[(long long)k * stride] = real(temper(s ^ twist(lo[k], lo[k + 1])));
-  }
+// u / (2^32 - 1) rounded to nearest, in integer arithmetic (a conversion and a
+// division in fp64 are some fifteen instructions at 1/64 of the integer rate).
+// In base 2^32 the quotient is 0.uuu..., so its bits from the first set one on are r r r ...
+// with r = u rotated left by its leading zeros z: the significand is the first
+// 53 of them, rounded by the next one (never a tie: the bits go on with another
+// r), and all ones carry over into 1.
+__device__ __forceinline__ double real(uint32_t u) {
+  const int z = __clz(u);
+  const uint32_t r = __funnelshift_l(u, u, z);
+  const unsigned long long m = ((unsigned long long)(r >> 11) << 32 | (r << 21 | r >> 11)) + (r >> 10 & 1u);
+  return u ? __longlong_as_double((long long)(m + ((unsigned long long)(uint32_t)(1021 - z) << 52))) : 0.0;
 }
 
 }  // namespace gbmt
