@@ -18,8 +18,13 @@
 //     another, so that a band's code and tables stay in the SM's caches and
 //     the run's setcoef words in L2.
 //
-// The kernel is bound by its instructions (2,220 multiply-adds and their loads
-// per column and layer) and by the 1,120 bytes it writes per column and layer.
+// What bounds the taumol kernel is the latency and the width of its table loads
+// (a warp's 16-byte load fills registers for four cycles, 2,220 multiply-adds per column
+// and layer, and the L1 pipe is three quarters busy): with 64 registers a thread and 8
+// blocks per SM 16,384 columns of 60 layers take 0.2 ms less than with 128 and 4
+// (transfer included 2.14 ms, now 1.94 ms; 9 or 10 blocks spill more than they
+// hide), of it 0.04 ms from runs of 304 blocks (two per SM) in place of 1,216;
+// with runs of 152 the last wave of each band shows (1.99 ms).
 // Compiled without multiply-add contraction: the prologues and the order of
 // every sum are those of the in-block taumol of lw_solver.cu, bit for bit.
 #include <cuda_runtime.h>
@@ -36,7 +41,7 @@ constexpr int CW = NF + 1;       // words per (column, layer): the LayerFields, 
 constexpr int TILE = 32;         // columns per tile: one per lane
 constexpr int SET_NT = 256;      // setcoef kernel: eight warps, one tile, layers dealt to the warps
 constexpr int TAU_NT = 128;      // taumol kernel: four (tile, layer) units per block
-constexpr int TAU_RUN = 1216;    // blocks of one band before the next band of the same columns
+constexpr int TAU_RUN = 304;     // blocks of one band before the next band of the same columns
 
 static_assert(GB_LW_COEF_WORDS == CW, "setcoef words per column and layer");
 
@@ -171,7 +176,7 @@ __device__ __forceinline__ void taumol_cell(const CoefCell& c, float* row) {
 
 __constant__ unsigned char c_order[16] = {5, 3, 13, 9, 7, 4, 8, 12, 15, 16, 6, 1, 11, 2, 10, 14};  // longest first
 
-__global__ void __launch_bounds__(TAU_NT, 4) lw_taumol_kernel(const __grid_constant__ LwBatch B,
+__global__ void __launch_bounds__(TAU_NT, 8) lw_taumol_kernel(const __grid_constant__ LwBatch B,
                                                               const float* __restrict__ T, long long u0,
                                                               long long nslot, int nblk) {
   // block -> (run of column blocks, band, block within the run)
