@@ -228,7 +228,7 @@ int launch_one(gb_lw_context* ctx, const LwArgs& a, int k, cudaStream_t stream) 
   b.col0[0] = 0;
   b.col0[1] = a.ncol;
   b.g[0] = a;
-  int rc = ensure_buffer(ctx, &ctx->d_gas[k], &ctx->gas_bytes[k], gb_lw_gas_bytes(a.nlay, a.ncol, false),
+  int rc = ensure_buffer(ctx, &ctx->d_gas[k], &ctx->gas_bytes[k], gb_lw_gas_bytes(b, false),
                          gb_lw_gas_min_bytes(a.nlay), stream);
   if (rc) return rc;
   gb_lw_attach_gas(b, ctx->d_gas[k], ctx->gas_bytes[k]);
@@ -332,7 +332,7 @@ int gb_ctx_make_batch(gb_lw_context* ctx, int ngrid, const gb_lw_grid* grids, do
 // hand-over planes for a descriptor's columns from the context's batch buffer
 static int attach_batch_gas(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
   int rc = ensure_buffer(ctx, &ctx->d_bgas, &ctx->bgas_bytes,
-                         gb_lw_gas_bytes(b.nsmax, b.col0[b.ngrid], batch_kind(b) & GB_LW_KIND_LEARNED),
+                         gb_lw_gas_bytes(b, batch_kind(b) & GB_LW_KIND_LEARNED),
                          gb_lw_gas_min_bytes(b.nsmax), stream);
   if (rc) return rc;
   gb_lw_attach_gas(b, ctx->d_bgas, ctx->bgas_bytes);
@@ -1202,7 +1202,7 @@ int gb_rrtmg_lw_batch_graph_create(gb_lw_context* ctx, int ngrid, const gb_lw_gr
   g->ctx = ctx;
   size_t gbytes = 0;
   if ((rc = ensure_buffer(ctx, &g->gas, &gbytes,
-                          gb_lw_gas_bytes(b.nsmax, b.col0[ngrid], batch_kind(b) & GB_LW_KIND_LEARNED),
+                          gb_lw_gas_bytes(b, batch_kind(b) & GB_LW_KIND_LEARNED),
                           gb_lw_gas_min_bytes(b.nsmax), nullptr)) != 0) {
     delete g;
     return rc;

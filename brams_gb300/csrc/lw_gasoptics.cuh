@@ -64,6 +64,16 @@ __host__ __device__ constexpr int g0_const(int b) {
   return m[b];
 }
 
+// the batch column of a slot of units [u0, ..): its grid and its column in it
+// (icol >= ncol where the slot is the missing column of a grid's last unit)
+__device__ __forceinline__ int slot_column(const LwBatch& B, long long u0, long long slot, long long& icol) {
+  const long long u = u0 + slot / B.cpb;
+  int gi = 0;
+  while (gi + 1 < B.ngrid && u >= B.unit0[gi + 1]) ++gi;
+  icol = (u - B.unit0[gi]) * B.cpb + slot % B.cpb;
+  return gi;
+}
+
 // fp64 column amounts of the binary species (inatm :807-867, setcoef.f90:349-362),
 // for decisions near a stencil switch or a truncation that are re-taken in
 // double precision: formed from the inputs where such a decision is met (a few

@@ -341,6 +341,7 @@ __device__ void gas_column(const LwArgs& a, long long icol, const GasSmem& s, co
 // Shared memory of one column: a fixed header, one 384-byte record per
 // layer (so that every per-layer access in the loops is base + layer * 384
 // + a constant), then the per-warp level sums.
+constexpr int CELL_WORDS = GB_LW_CELL_WORDS;
 struct RtHead {
   float misc[64];         // secdiff[16], plankbnd[16], dplankbnd[16], semiss[16]
   float red[2 * RT_NW];   // column sums for pwvcm of 32 layers each
@@ -361,19 +362,16 @@ struct RtLayer {
   // 14 floats (RtSmem::ovl): cldfrac, rtrnmr's upward overlap factors at lev+1
   // (facclr1, facclr2, faccld1, faccld2, faccmb1, faccmb2) and the downward
   // ones at lev-1, in that order
-  unsigned cbits[5];  // per group of 32 g-points: bit l set where g-point 2l of the group is cloudy
+  unsigned cbits[CELL_WORDS];  // the first five: per group of 32 g-points: bit l set where g-point 2l of the group is cloudy
                       // (cldfmc == 1; caller sub-columns: or a fraction, in a layer with a cell
                       // of 1), bit 16 + l where g-point 2l + 1 is
-  int pad0;           // caller sub-columns: five words from here on (RtSmem::fbits), as cbits:
-                      // cldfmcl neither 0 nor 1
-  long long cthr;     // fused clouds: McICA threshold 1 - cldf as double bits
-  long long pad1;
+                      // caller sub-columns: the next five (RtSmem::fbits), as these: cldfmcl neither 0 nor 1
+                      // fused clouds: the McICA threshold 1 - cldf as double bits in words 6 and 7 (RtSmem::cthr)
   float4 lcw;         // (ciwp, clwp, radice, radliq) as floats
 };
 static_assert(sizeof(RtHead) == 320 && sizeof(RtLayer) == 320, "transfer shared-memory records");
-static_assert(offsetof(RtLayer, lcw) + sizeof(float4) - offsetof(RtLayer, cbits) == 14 * sizeof(float),
+static_assert(offsetof(RtLayer, lcw) + sizeof(float4) - offsetof(RtLayer, cbits) == 14 * sizeof(float) && offsetof(RtLayer, cbits) % 8 == 0,
               "band-cloud overlay of the McICA words");
-static_assert(offsetof(RtLayer, lcw) - offsetof(RtLayer, pad0) == 5 * sizeof(unsigned), "fraction bits of caller sub-columns");
 
 struct RtSmem {
   RtHead* h;
@@ -382,7 +380,8 @@ struct RtSmem {
                 // clouds' fractions in fp64
   float* part;  // [RT_NW][nl+1][6] level sums per group of 32 g-points: dn, dn clear, up, up clear, dup/dT,
                 // dup clear/dT (global scratch)
-  __device__ __forceinline__ unsigned* fbits(int lay) const { return reinterpret_cast<unsigned*>(&L[lay].pad0); }
+  __device__ __forceinline__ unsigned* fbits(int lay) const { return L[lay].cbits + 5; }
+  __device__ __forceinline__ long long& cthr(int lay) const { return *reinterpret_cast<long long*>(L[lay].cbits + 6); }
   __device__ __forceinline__ float* ovl(int lay) const { return reinterpret_cast<float*>(L[lay].cbits); }
 };
 
@@ -410,6 +409,8 @@ __device__ inline RtSmem rt_carve(char* p, int nl, float* part) {
 struct GasSrc {
   const float* plane;         // taumol's plane of the column (rows of GB_LW_PROW floats), or NULL
   float* gc;                  // caller sub-columns: the cells' cloud plane [nl][140]
+  const unsigned* cw;         // ... and from lw_cells_kernel the unit's first column's cell bits
+  int cerr;                   // and the column's stop code
   const __half* nt;           // fp16 rows [nl][140] (network), or NULL
   const __half* nf;
   const unsigned char* flag;  // per layer: 1 -> network, 0 -> fp32 planes
@@ -458,15 +459,27 @@ __device__ __forceinline__ void cloud_total(const float2* tt, int itr, float od,
   }
 }
 
+// ciwp + clwp >= 1e-20: on the bit patterns where neither is negative or NaN
+// (the sum is no less than either, and no rounding takes it below 1e-20), in fp64 where that leaves it open
+__device__ __forceinline__ bool has_paths(double ciwp, double clwp) {
+  const long long i = __double_as_longlong(ciwp), l = __double_as_longlong(clwp);
+  const long long kMin = __double_as_longlong(1.0e-20), kInf = 0x7FF0000000000000LL;
+  if (i >= 0 && l >= 0 && i <= kInf && l <= kInf) {
+    if (i >= kMin || l >= kMin) return true;
+    if ((i | l) == 0) return false;
+  }
+  return ciwp + clwp >= 1.e-20;
+}
+
 // a caller sub-column cell's cloud value for the transfer: its cloud optical
 // depth (cldprmc.f90:178-266, rtrnmc.f90:300-312) where cldfmcl = 1,
 // the fraction itself where it is neither 0 nor 1
 __device__ __forceinline__ float cell_value(const LwArgs& a, const RtSmem& S, int lay, int band, bool one,
-                                            double cf, double ciwp, double clwp, double tin,
+                                            double cf, double ciwp, double clwp, bool paths, double tin,
                                             const float* __restrict__ T) {
   if (!one) return (float)cf;
   float tauc = 0.0f;
-  bool from_paths = a.inflag == 2 && ciwp + clwp >= 1.e-20;
+  bool from_paths = a.inflag == 2 && paths;
   if (!from_paths) {
     const long long tb = __double_as_longlong(tin);
     from_paths = a.inflag == 2 && tb >= __double_as_longlong(1.0e-20) && tb <= 0x7FF0000000000000LL;
@@ -803,7 +816,7 @@ struct Passes {
     if (KIND == PK_FUSED) odl = sd * L.rec[band].w;
     if (BAND) odl = L.rec[cband].w;
     if (KIND == PK_FUSED || KIND == PK_RANDOM) efl = 1.0f - __expf(-odl);
-    const unsigned frac = KIND == PK_SUBCOL ? reinterpret_cast<const unsigned*>(&L.pad0)[grp] >> l16 : 0u;
+    const unsigned frac = KIND == PK_SUBCOL ? L.cbits[5 + grp] >> l16 : 0u;
     auto cell = [&](bool cloudy, bool one, float od, float pf, float at, float gs, float tr, float v, float r1, float& A1,
                     float& B1, float& D1, float& cr1, float& kr1, float& rm1) {
       if constexpr (BAND) {
@@ -998,12 +1011,104 @@ __device__ __forceinline__ void rt_passes(const LwArgs& a, const RtSmem& S, cons
     P.template up<false>(ru, rcu, du, dcu);
 }
 
+// a layer's radii as floats and the codes cldprmc's radius checks stop with: bits 0-7 ice, 8-15 liquid
+__device__ __forceinline__ void layer_radii(const LwArgs& a, const RtSmem& S, long long icol, int lay) {
+  const double rice = in2(a.reicmcl, a.ld, icol, lay), rliq = in2(a.relqmcl, a.ld, icol, lay);
+  S.L[lay].lfl = ice_code(a.iceflag, rice) | (liq_code(a.liqflag, rliq) << 8);
+  S.L[lay].lcw = make_float4(0.0f, 0.0f, (float)rice, (float)rliq);
+}
+// the layer's cloudy cells: none where no cell has cldfmcl == 1, else the fractions too
+__device__ __forceinline__ void cloudy_words(const RtSmem& S, int lay) {
+  unsigned* c = S.L[lay].cbits;
+  const unsigned* f = S.fbits(lay);
+  const bool any = (c[0] | c[1] | c[2] | c[3] | c[4]) != 0u;
+  for (int w = 0; w < RT_NW; ++w) c[w] = any ? c[w] | f[w] : 0u;
+}
+// The cells of one of the caller's sub-columns' columns, a pair of g-points per
+// thread (16 lanes of a group of 32 g-points): the layers' cloud bits into their
+// records (RtLayer::cbits, RtSmem::fbits), the cloudy cells' values into the plane
+// gc; returns the largest of the pair's codes that cldprmc stops with (of several
+// going up the column the last).  The layers' radii and their codes (lcw, lfl) are there.
+__device__ __forceinline__ int subcol_cells(const LwArgs& a, const RtSmem& S, long long icol, int nl, bool live, int g,
+                                            int band, int lane, int grp, bool inblk, float* gc,
+                                            const float* __restrict__ T) {
+  const unsigned FULL = 0xffffffffu;
+  const int l16 = lane & 15;
+  // a group's word of a layer from the ballots over the low and the high g-points of its pairs
+  auto word = [&](unsigned lo, unsigned hi) {
+    return lane < 16 ? (lo & 0xffffu) | (hi << 16) : (lo >> 16) | (hi & 0xffff0000u);
+  };
+  // per layer, each group: its 32 cldfmcl values tested on their bit
+  // patterns: == 1, /= 0, >= 1e-20.  A pair is one 16-byte load where the
+  // caller's arrays start on such a boundary (rows are 1,120 bytes).
+  const long long kOne = 0x3FF0000000000000LL, kInf = 0x7FF0000000000000LL;
+  const long long kMin = __double_as_longlong(1.0e-20);
+  const bool wide = (((uintptr_t)a.cldfmcl | (uintptr_t)a.ciwpmcl | (uintptr_t)a.clwpmcl | (uintptr_t)a.taucmcl) & 15) == 0;
+  auto pair = [&](const double* p, long long o) {
+    return wide ? __ldg(reinterpret_cast<const double2*>(p + o)) : make_double2(__ldg(p + o), __ldg(p + o + 1));
+  };
+#pragma unroll 8
+  for (int lay = 0; lay < nl; ++lay) {
+    const double2 cf = pair(a.cldfmcl, g + GB_NGPT * (icol + a.ld * lay));
+    const long long b0 = live ? __double_as_longlong(cf.x) : 0LL, b1 = live ? __double_as_longlong(cf.y) : 0LL;
+    const bool one0 = b0 == kOne, one1 = b1 == kOne;
+    const bool fr0 = !one0 && (b0 << 1) != 0LL, fr1 = !one1 && (b1 << 1) != 0LL;  // neither +-0 nor 1 (NaN included, as /= 0 is)
+    const unsigned m0 = __ballot_sync(FULL, one0), m1 = __ballot_sync(FULL, one1);
+    const unsigned f0 = __ballot_sync(FULL, fr0), f1 = __ballot_sync(FULL, fr1);
+    if (l16 == 0 && inblk) {
+      S.L[lay].cbits[grp] = word(m0, m1);
+      S.fbits(lay)[grp] = word(f0, f1);
+    }
+  }
+  __syncwarp();
+  // then, per pair with a cloud: the water paths for cldprmc's checks and the
+  // cells' optical depths, formed once instead of in both passes.  Two layers'
+  // loads are in flight, and the two cells share one copy of the optics: with
+  // four layers and eight copies the warps waited for instructions
+  int err0 = 0, err1 = 0;
+#pragma unroll 2
+  for (int lay = 0; lay < nl; ++lay) {
+    const unsigned ob = S.L[lay].cbits[grp] >> l16, fb = S.fbits(lay)[grp] >> l16;
+    if (!live || !((ob | fb) & 0x10001u)) continue;
+    const long long o = g + GB_NGPT * (icol + a.ld * lay);
+    const double2 cf = fb & 0x10001u ? pair(a.cldfmcl, o) : make_double2(ob & 1u, ob >> 16 & 1u);
+    const double2 ci = pair(a.ciwpmcl, o), cl = pair(a.clwpmcl, o), ti = pair(a.taucmcl, o);
+    auto cell = [&](bool one, bool cloudy, double cfv, double ciwp, double clwp, double tin, int& err) {
+      if (!cloudy) return 0.0f;
+      const long long cb = __double_as_longlong(cfv);
+      if (!(cb >= kMin && cb <= kInf)) return (float)cfv;  // a fraction below cldmin: cldfmcl itself, no cloud optics
+      const bool paths = has_paths(ciwp, clwp);
+      const float v = cell_value(a, S, lay, band, one, cfv, ciwp, clwp, paths, tin, T);  // cldfmc >= cldmin (cldprmc.f90:178)
+      const long long tb = __double_as_longlong(tin);
+      if (paths || (tb >= kMin && tb <= kInf)) {
+        const int e = S.L[lay].lfl;
+        if (a.inflag == 1) err = GB_COL_INFLAG1;
+        if (a.inflag == 2) {
+          if ((__double_as_longlong(ciwp) << 1) != 0LL && (e & 0xff)) err = e & 0xff;  // ciwp /= 0
+          if ((__double_as_longlong(clwp) << 1) != 0LL && (e >> 8)) err = e >> 8;      // clwp /= 0
+        }
+      }
+      return v;
+    };
+    float v0 = 0.0f, v1 = 0.0f;
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+      const float v = cell(ob >> 16 * k & 1u, (ob | fb) >> 16 * k & 1u, k ? cf.y : cf.x, k ? ci.y : ci.x, k ? cl.y : cl.x,
+                           k ? ti.y : ti.x, k ? err1 : err0);
+      (k ? v1 : v0) = v;
+    }
+    *reinterpret_cast<float2*>(gc + lay * GB_NGPT + g) = make_float2(v0, v1);
+  }
+  return max(err0, err1);
+}
+
 // The transfer of a unit's columns (see the file header); src is that of this
 // thread's column.  RT_NET: a column with any layer off the network is not
 // solved; returns whether this thread's column was solved.  BAND: the non-McICA
 // driver's band clouds (random overlap for icld 1, maximum/random otherwise).
 // Ends with a barrier.
-template <int MODE, bool BAND = false>
+// CELLS: caller sub-columns' cells come from lw_cells_kernel (src.cw).
+template <int MODE, bool BAND = false, bool CELLS = false>
 __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const Cols& C, const GasSrc& src,
                            const float* __restrict__ T) {
   constexpr bool NET = MODE == RT_NET || MODE == RT_NETODD;
@@ -1147,7 +1252,7 @@ __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const
   if constexpr (BAND) {
     band_clouds(a, U, C, nl, clouds);
   } else {
-  for (int i = tid; i < C.n * nl * 5; i += nt) {
+  for (int i = tid; i < C.n * nl * 5 && !(CELLS && clouds && !fused); i += nt) {
     const int r = C.rest(i), l = r / 5, w = r - 5 * l;
     const RtSmem Sc = C.S(C.c(i));
     Sc.L[l].cbits[w] = 0u;
@@ -1168,7 +1273,7 @@ __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const
       // for a threshold >= 0 the integer order is the floating-point order);
       // a negative threshold takes every cell, a NaN none
       const double thr = 1.0 - cf;
-      Sc.L[lay].cthr = thr < 0.0 ? LLONG_MIN : (thr == thr ? __double_as_longlong(thr) : LLONG_MAX);
+      Sc.cthr(lay) = thr < 0.0 ? LLONG_MIN : (thr == thr ? __double_as_longlong(thr) : LLONG_MAX);
       const double ciwp = in2(a.ciwp, a.ld, ic, lay), clwp = in2(a.clwp, a.ld, ic, lay);
       const double rice = in2(a.reicmcl, a.ld, ic, lay), rliq = in2(a.relqmcl, a.ld, ic, lay);
       const int fl = (ciwp != 0.0 ? 1 : 0) | (clwp != 0.0 ? 2 : 0) | (ciwp + clwp >= 1.e-20 ? 4 : 0);
@@ -1192,7 +1297,7 @@ __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const
     // cloudy cells: cdf(g) >= 1 - cldf(lay) (mcica_subcol_gen_lw.f90:650); a
     // layer whose threshold is above every draw of the warp has none there
     for (int lay = 0; lay < nl; ++lay) {
-      const long long tb = S.L[lay].cthr;
+      const long long tb = S.cthr(lay);
       if (__all_sync(FULL, tb > mx)) continue;
       const unsigned m0 = __ballot_sync(FULL, live && d0 >= tb), m1 = __ballot_sync(FULL, live && d1 >= tb);
       if (l16 == 0 && inblk) S.L[lay].cbits[grp] = word(m0, m1);
@@ -1237,79 +1342,20 @@ __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const
       if (err) atomicMax(&Sc.h->iscal[0], err);
     }
   } else if (clouds) {
-    // caller sub-columns: the layer radii as floats and the codes cldprmc's
-    // radius checks stop with: bits 0-7 ice, 8-15 liquid
-    for (int i = tid; i < C.n * nl; i += nt) {
-      const int lay = C.rest(i);
-      const RtSmem Sc = C.S(C.c(i));
-      const long long ic = C.icol(C.c(i));
-      const double rice = in2(a.reicmcl, a.ld, ic, lay), rliq = in2(a.relqmcl, a.ld, ic, lay);
-      Sc.L[lay].lfl = ice_code(a.iceflag, rice) | (liq_code(a.liqflag, rliq) << 8);
-      Sc.L[lay].lcw = make_float4(0.0f, 0.0f, (float)rice, (float)rliq);
-    }
-    U.sync();
-    // per layer, each group: its 32 cldfmcl values tested on their bit
-    // patterns: == 1, /= 0, >= 1e-20.  A pair is one 16-byte load where the
-    // caller's arrays start on such a boundary (rows are 1,120 bytes).
-    const long long kOne = 0x3FF0000000000000LL, kInf = 0x7FF0000000000000LL;
-    const long long kMin = __double_as_longlong(1.0e-20);
-    const bool wide = (((uintptr_t)a.cldfmcl | (uintptr_t)a.ciwpmcl | (uintptr_t)a.clwpmcl | (uintptr_t)a.taucmcl) & 15) == 0;
-    auto pair = [&](const double* p, long long o) {
-      return wide ? __ldg(reinterpret_cast<const double2*>(p + o)) : make_double2(__ldg(p + o), __ldg(p + o + 1));
-    };
-#pragma unroll 8
-    for (int lay = 0; lay < nl; ++lay) {
-      const double2 cf = pair(a.cldfmcl, g + GB_NGPT * (icol + a.ld * lay));
-      const long long b0 = live ? __double_as_longlong(cf.x) : 0LL, b1 = live ? __double_as_longlong(cf.y) : 0LL;
-      const bool one0 = b0 == kOne, one1 = b1 == kOne;
-      const bool fr0 = !one0 && (b0 << 1) != 0LL, fr1 = !one1 && (b1 << 1) != 0LL;  // neither +-0 nor 1 (NaN included, as /= 0 is)
-      const unsigned m0 = __ballot_sync(FULL, one0), m1 = __ballot_sync(FULL, one1);
-      const unsigned f0 = __ballot_sync(FULL, fr0), f1 = __ballot_sync(FULL, fr1);
-      if (l16 == 0 && inblk) {
-        S.L[lay].cbits[grp] = word(m0, m1);
-        S.fbits(lay)[grp] = word(f0, f1);
+    // caller sub-columns
+    if constexpr (CELLS) {
+      for (int i = tid; i < C.n * nl * CELL_WORDS; i += nt) {
+        const int c = C.c(i), r = C.rest(i), lay = r / CELL_WORDS, w = r - CELL_WORDS * lay;
+        C.S(c).L[lay].cbits[w] = src.cw[(size_t)c * C.nlmax * CELL_WORDS + r];
       }
-    }
-    __syncwarp();
-    // then, per pair with a cloud (independent iterations, so that several
-    // pairs' loads are in flight): the water paths for cldprmc's checks and
-    // the cells' optical depths, formed once instead of in both passes
-    int err0 = 0, err1 = 0;
-#pragma unroll 4
-    for (int lay = 0; lay < nl; ++lay) {
-      const unsigned ob = S.L[lay].cbits[grp] >> l16, fb = S.fbits(lay)[grp] >> l16;
-      if (!live || !((ob | fb) & 0x10001u)) continue;
-      const long long o = g + GB_NGPT * (icol + a.ld * lay);
-      const double2 cf = fb & 0x10001u ? pair(a.cldfmcl, o) : make_double2(ob & 1u, ob >> 16 & 1u);
-      const double2 ci = pair(a.ciwpmcl, o), cl = pair(a.clwpmcl, o), ti = pair(a.taucmcl, o);
-      auto cell = [&](bool one, bool cloudy, double cfv, double ciwp, double clwp, double tin, int& err) {
-        if (!cloudy) return 0.0f;
-        const long long cb = __double_as_longlong(cfv);
-        if (!(cb >= kMin && cb <= kInf)) return (float)cfv;  // a fraction below cldmin: cldfmcl itself, no cloud optics
-        const float v = cell_value(a, S, lay, band, one, cfv, ciwp, clwp, tin, T);  // cldfmc >= cldmin (cldprmc.f90:178)
-        const long long tb = __double_as_longlong(tin);
-        if (ciwp + clwp >= 1.e-20 || (tb >= kMin && tb <= kInf)) {
-          const int e = S.L[lay].lfl;
-          if (a.inflag == 1) err = GB_COL_INFLAG1;
-          if (a.inflag == 2) {
-            if ((__double_as_longlong(ciwp) << 1) != 0LL && (e & 0xff)) err = e & 0xff;  // ciwp /= 0
-            if ((__double_as_longlong(clwp) << 1) != 0LL && (e >> 8)) err = e >> 8;      // clwp /= 0
-          }
-        }
-        return v;
-      };
-      const float v0 = cell(ob & 1u, (ob | fb) & 1u, cf.x, ci.x, cl.x, ti.x, err0);
-      const float v1 = cell(ob >> 16 & 1u, (ob | fb) >> 16 & 1u, cf.y, ci.y, cl.y, ti.y, err1);
-      *reinterpret_cast<float2*>(src.gc + lay * GB_NGPT + g) = make_float2(v0, v1);
-    }
-    if (err0 || err1) atomicMax(&S.h->iscal[0], max(err0, err1));
+      if (t == 0 && inblk) S.h->iscal[0] = src.cerr;
+    } else {
+    for (int i = tid; i < C.n * nl; i += nt) layer_radii(a, C.S(C.c(i)), C.icol(C.c(i)), C.rest(i));
     U.sync();
-    for (int i = tid; i < C.n * nl; i += nt) {
-      const RtSmem Sc = C.S(C.c(i));
-      unsigned* c = Sc.L[C.rest(i)].cbits;
-      const unsigned* f = Sc.fbits(C.rest(i));
-      const bool any = (c[0] | c[1] | c[2] | c[3] | c[4]) != 0u;
-      for (int w = 0; w < RT_NW; ++w) c[w] = any ? c[w] | f[w] : 0u;
+    const int err = subcol_cells(a, S, icol, nl, live, g, band, lane, grp, inblk, src.gc, T);
+    if (err) atomicMax(&S.h->iscal[0], err);
+    U.sync();
+    for (int i = tid; i < C.n * nl; i += nt) cloudy_words(C.S(C.c(i)), C.rest(i));
     }
   } else {
     for (int i = tid; i < C.n * nl; i += nt) C.S(C.c(i)).L[C.rest(i)].cldlay = 0;
@@ -1507,11 +1553,58 @@ __global__ void __launch_bounds__(RT_NT * MAXU, 1) lw_rt_kernel(const __grid_con
       src.plane = B.plane + ((u - u0) * B.cpb + col) * B.nsmax * GB_LW_PROW;
     else if (a.sur_flag)
       src = net_source(a, C.icol(col));
-    if (!BAND) src.gc = B.gcld + ((long long)slot * B.cpb + col) * B.nsmax * GB_NGPT;
-    const bool done = (MODE == RT_GAS || a.sur_flag) && rt_columns<MODE, BAND>(a, U, C, src, T);
+    constexpr bool CELLS = MODE == RT_GAS && !BAND;
+    if constexpr (CELLS) {
+      if (B.cellw) {
+        const long long ps = (u - u0) * B.cpb;
+        src.gc = B.gcld + (ps + col) * B.nsmax * GB_NGPT;
+        src.cw = B.cellw + ps * B.nsmax * CELL_WORDS;
+        src.cerr = __ldg(B.cellerr + ps + col);
+      }
+    } else if (!BAND) {
+      src.gc = B.gcld + ((long long)slot * B.cpb + col) * B.nsmax * GB_NGPT;
+    }
+    const bool done = (MODE == RT_GAS || a.sur_flag) && rt_columns<MODE, BAND, CELLS>(a, U, C, src, T);
     if (MODE != RT_GAS && !done && U.tid == half * RT_CT && half < B.cpb && C.col0 + col <= C.last)
       B.fall[atomicAdd(B.nfall, 1u)] = B.col0[gi] + C.col0 + col;
   }
+}
+
+// The cells of caller sub-columns for the column slots of units [u0, ..): each
+// column's cloud bits, the cloudy cells' values and its stop code, a block per
+// column.  The arrays are read once, so what bounds it is latency: it has 39 warps
+// of an SM in flight, the transfer kernel 20, where this took as long as the
+// passes (32,768 columns of 45 layers, all kernels: 4.45 ms there, 3.78 ms as
+// a kernel of its own, 3.45 ms with two layers unrolled in place of four and without a
+// sum in fp64 per cell).
+constexpr int CELL_NT = 96;
+__global__ void __launch_bounds__(CELL_NT, 13) lw_cells_kernel(const __grid_constant__ LwBatch B,
+                                                           const float* __restrict__ T, long long u0) {
+  extern __shared__ __align__(16) char smem_raw[];
+  const long long slot = blockIdx.x;
+  long long icol;
+  const LwArgs& a = B.g[slot_column(B, u0, slot, icol)];
+  const bool none = icol >= a.ncol || a.cloud_mode != LW_CLOUD_SUBCOL || a.icld < 1;
+  if (none) {
+    if (threadIdx.x == 0) B.cellerr[slot] = 0;
+    return;
+  }
+  const int t = threadIdx.x, lane = t & 31, nl = a.nlay;
+  const RtSmem S = rt_carve(smem_raw, nl, nullptr);
+  const bool inblk = t < RT_CT, live = t < GB_NGPT / 2;
+  const int g = live ? 2 * t : GB_NGPT - 2;
+  const int band = __float_as_int(__ldg(T + c_T.gpt_band + g));
+  if (t == 0) S.h->iscal[0] = 0;
+  for (int lay = t; lay < nl; lay += CELL_NT) layer_radii(a, S, icol, lay);
+  __syncthreads();
+  const int err = subcol_cells(a, S, icol, nl, live, g, band, lane, t >> 4, inblk, B.gcld + slot * B.nsmax * GB_NGPT, T);
+  if (err) atomicMax(&S.h->iscal[0], err);
+  __syncthreads();
+  for (int lay = t; lay < nl; lay += CELL_NT) cloudy_words(S, lay);
+  if (t == 0) B.cellerr[slot] = S.h->iscal[0];
+  __syncthreads();
+  unsigned* out = B.cellw + slot * B.nsmax * CELL_WORDS;
+  for (int i = t; i < nl * CELL_WORDS; i += CELL_NT) out[i] = S.L[i / CELL_WORDS].cbits[i % CELL_WORDS];
 }
 
 // The columns handed over by the network's transfer kernel (B.fall), one per
@@ -1710,6 +1803,16 @@ int gb_lw_slots(int nlay, int variant, bool lean) {
 namespace {
 // plane bytes of one column slot: its rows, setcoef's words, laytrop
 size_t slot_bytes(int nlay) { return (size_t)nlay * (GB_LW_PROW + GB_LW_COEF_WORDS) * 4 + sizeof(int); }
+// ... and of a batch with caller sub-columns: the cells' values and bits, the stop code
+size_t cell_bytes(int nlay) { return (size_t)nlay * (GB_NGPT + GB_LW_CELL_WORDS) * 4 + sizeof(int); }
+bool has_cells(const LwBatch& b) {
+  bool any = false;
+  for (int i = 0; i < b.ngrid; ++i) {
+    if (b.g[i].sur_flag) return false;  // learned gas optics take their cells in the transfer kernel
+    any |= b.g[i].cloud_mode == LW_CLOUD_SUBCOL && b.g[i].icld >= 1;
+  }
+  return any;
+}
 // per resident column: the cloud plane of caller sub-columns, the level sums
 size_t resident_cols() { return (size_t)device_sms() * kMaxPerSm * 2; }
 size_t resident_bytes(int nlay) {
@@ -1722,24 +1825,31 @@ size_t round_slots(size_t n) { return (n + 31) & ~size_t(31); }
 constexpr size_t kPlaneBytes = size_t(1536) << 20;
 }  // namespace
 
-size_t gb_lw_gas_bytes(int nlay, long long ncols, bool learned) {
-  const size_t room = std::max<size_t>(kPlaneBytes / slot_bytes(nlay) & ~size_t(31), 32);
-  const size_t want = learned ? 0 : round_slots((size_t)ncols + GB_LW_MAX_GRIDS);  // a column may be missing per grid
-  const size_t slots = std::max(std::min(want, room), round_slots((size_t)gb_lw_list_slots()));
-  return resident_bytes(nlay) + slots * slot_bytes(nlay);
+size_t gb_lw_gas_min_bytes(int nlay) {
+  return resident_bytes(nlay) + round_slots((size_t)gb_lw_list_slots()) * slot_bytes(nlay);
 }
 
-size_t gb_lw_gas_min_bytes(int nlay) { return gb_lw_gas_bytes(nlay, 0, true); }
+size_t gb_lw_gas_bytes(const LwBatch& b, bool learned) {
+  const size_t per = slot_bytes(b.nsmax) + (has_cells(b) ? cell_bytes(b.nsmax) : 0);
+  const size_t room = std::max<size_t>(kPlaneBytes / per & ~size_t(31), 32);
+  const size_t want = learned ? 0 : round_slots((size_t)b.col0[b.ngrid] + GB_LW_MAX_GRIDS);  // a column may be missing per grid
+  return std::max(resident_bytes(b.nsmax) + std::min(want, room) * per, gb_lw_gas_min_bytes(b.nsmax));
+}
 
 void gb_lw_attach_gas(LwBatch& b, void* buf, size_t bytes) {
   const size_t res = resident_bytes(b.nsmax);
+  const bool cells = has_cells(b);
+  const size_t per = slot_bytes(b.nsmax) + (cells ? cell_bytes(b.nsmax) : 0);
   b.rcols = (long long)resident_cols();
-  b.pslots = bytes > res ? (long long)((bytes - res) / slot_bytes(b.nsmax) & ~size_t(31)) : 0;
+  b.pslots = bytes > res ? (long long)((bytes - res) / per & ~size_t(31)) : 0;
+  const size_t rows = (size_t)b.pslots * b.nsmax;
   b.plane = static_cast<float*>(buf);  // the rows first: each on a 32-byte boundary
-  b.coef = b.plane + (size_t)b.pslots * b.nsmax * GB_LW_PROW;
-  b.gcld = b.coef + (size_t)b.pslots * b.nsmax * GB_LW_COEF_WORDS;
-  b.part = b.gcld + (size_t)b.rcols * b.nsmax * GB_NGPT;
+  b.coef = b.plane + rows * GB_LW_PROW;
+  b.gcld = b.coef + rows * GB_LW_COEF_WORDS;
+  b.part = b.gcld + std::max(cells ? rows : 0, (size_t)b.rcols * b.nsmax) * GB_NGPT;
   b.laytrop = reinterpret_cast<int*>(b.part + (size_t)b.rcols * gb::rt_part_floats(b.nsmax));
+  b.cellerr = cells ? b.laytrop + b.pslots : nullptr;
+  b.cellw = cells ? reinterpret_cast<unsigned*>(b.cellerr + b.pslots) : nullptr;
 }
 
 long long gb_lw_list_slots() { return (long long)device_sms() * gb::LIST_PER_SM; }
@@ -1784,12 +1894,21 @@ cudaError_t gb_lw_launch_batch(const LwBatch& bin, const float* d_tables, int va
     return v.launch(b, d_tables, u0, u1, blocks, nunit * unit_threads(b.cpb), nunit, smem, stream);
   };
   if (!b.fall || !b.nfall) {
-    // pass by pass: taumol into the planes, then the transfer
+    // pass by pass: taumol into the planes, caller sub-columns' cells, then the transfer
+    for (int i = 0; i < b.ngrid; ++i)
+      if (b.g[i].cloud_mode == LW_CLOUD_SUBCOL && b.g[i].icld >= 1 && !b.cellw) return cudaErrorInvalidValue;
     if (nband && nband != b.ngrid) return cudaErrorInvalidValue;  // band clouds: every grid in that mode
     const long long room = b.pslots / b.cpb, passes = (units + room - 1) / room, step = (units + passes - 1) / passes;
     for (long long u0 = 0; u0 < units; u0 += step) {
       const long long u1 = std::min(u0 + step, units);
       cudaError_t e = gb_lw_launch_taumol(b, d_tables, u0, u1, stream);
+      if (e == cudaSuccess && b.cellw) {
+        const size_t smem = gb::rt_smem_bytes(b.nsmax);
+        e = cudaFuncSetAttribute((const void*)gb::lw_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        gb::lw_cells_kernel<<<(unsigned)((u1 - u0) * b.cpb), gb::CELL_NT, smem, stream>>>(b, d_tables, u0);
+        e = cudaGetLastError();
+      }
       if (e == cudaSuccess) e = transfer(nband ? kBand : info(variant, false), u0, u1);
       if (e != cudaSuccess) return e;
     }

@@ -74,6 +74,7 @@ struct LwArgs {
 // gtau and gfrac ([slot][layer][140] planes, gstride floats per slot) are the
 // outputs of the taumol-only launch (training samples, diagnostics).
 constexpr int GB_LW_PROW = 304;        // floats per plane row: 76 pair positions
+constexpr int GB_LW_CELL_WORDS = 10;   // cell bits of a layer (140 cloudy, 140 fractional, in groups of 32)
 constexpr int GB_LW_COEF_WORDS = 26;   // setcoef words per column and layer
 // first pair position of band b (1..16) in a plane row
 __host__ __device__ constexpr int gb_pair0(int b) {
@@ -91,7 +92,10 @@ struct LwBatch {
   int* laytrop = nullptr;                 // per slot
   long long pslots = 0;                   // plane slots available (a multiple of 32)
   float* gcld = nullptr;                  // caller sub-columns: each cloudy cell's optical depth (or
-                                          // fractional cldfmcl), [nsmax][140] per resident column
+                                          // fractional cldfmcl), [nsmax][140] per slot (learned gas
+                                          // optics: per resident column)
+  unsigned* cellw = nullptr;              // and per slot and layer the cells' bits: GB_LW_CELL_WORDS words
+  int* cellerr = nullptr;                 // and the columns' stop codes
   float* part = nullptr;                  // level sums per resident column
   long long rcols = 0;                    // resident columns there is room for
   float* gtau = nullptr;                  // taumol-only launch (see above)
@@ -121,9 +125,9 @@ int gb_lw_default_variant(int nlay);
 size_t gb_lw_smem_bytes(int nlay);
 // column blocks of `variant` resident on the device at once for this nlay
 int gb_lw_slots(int nlay, int variant = 0, bool lean = false);
-// bytes of the hand-over buffer a batch of `ncols` columns is solved with
+// bytes of the hand-over buffer a batch (its grids set) is solved with
 // (learned: only the hand-over kernel's planes), and the least it runs with
-size_t gb_lw_gas_bytes(int nlay, long long ncols, bool learned);
+size_t gb_lw_gas_bytes(const LwBatch& b, bool learned);
 size_t gb_lw_gas_min_bytes(int nlay);
 // points a descriptor at a hand-over buffer of `bytes`
 void gb_lw_attach_gas(LwBatch& b, void* buf, size_t bytes);

@@ -82,16 +82,6 @@ struct RegTerms {
   }
 };
 
-// the batch column of a slot of units [u0, ..): its grid and its column in it
-// (icol >= ncol where the slot is the missing column of a grid's last unit)
-__device__ __forceinline__ int slot_column(const LwBatch& B, long long u0, long long slot, long long& icol) {
-  const long long u = u0 + slot / B.cpb;
-  int gi = 0;
-  while (gi + 1 < B.ngrid && u >= B.unit0[gi + 1]) ++gi;
-  icol = (u - B.unit0[gi]) * B.cpb + slot % B.cpb;
-  return gi;
-}
-
 __global__ void __launch_bounds__(SET_NT) lw_setcoef_kernel(const __grid_constant__ LwBatch B,
                                                             const float* __restrict__ T, long long u0, long long nslot) {
   __shared__ int lt[TILE];
