@@ -49,3 +49,17 @@ def test_several_passes_repeat_their_columns(swctx, bits):
     for k in ("swuflx", "swdflx", "swhr", "swuflxc", "swdflxc", "swhrc"):
         v = one[k]
         assert np.array_equal(many[k].reshape(115, 131, -1), np.broadcast_to(v, (115,) + v.shape)), k
+
+
+def test_fractions_that_are_no_numbers_stay_in_their_column(swctx):
+    """A column whose surface albedo is not a number gets no numbers, its neighbours the clean call's bits."""
+    st = sw_state(ncol=9, nlay=38, seed=21)
+    clean = _solve(swctx, 32, st, None, icld=0, iaer=0)
+    bad = {k: np.array(v, order="F", copy=True) if isinstance(v, np.ndarray) else v for k, v in st.items()}
+    for k in ("asdir", "asdif", "aldir", "aldif"):
+        bad[k][4] = np.nan
+    out = _solve(swctx, 32, bad, None, icld=0, iaer=0)
+    keep = np.arange(9) != 4
+    for k in ("swuflx", "swdflx", "swuflxc", "swdflxc"):
+        assert np.isnan(out[k][4]).all(), k
+        assert np.array_equal(out[k][keep], clean[k][keep]), k
