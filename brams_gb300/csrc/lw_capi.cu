@@ -1080,7 +1080,11 @@ int gb_rrtmg_lw_tuning_set(gb_lw_context* ctx, int nlay, int kind, const gb_lw_t
   cudaSetDevice(ctx->device);
   const bool lean = kind & GB_LW_KIND_LEARNED;
   const int occ = gb_lw_slots(nlay, shape->variant, lean) / std::max(1, ctx->num_sms);
-  if (shape->blocks_per_sm < 1 || shape->blocks_per_sm > occ) {
+  // shapes saved when a block was one column (6, 7, 5 and 4 of an SM at most, of
+  // 816 + 504.5 nlay bytes) are taken too, and run with as many units as fit
+  const int column_blocks[] = {6, 7, 5, 4};
+  const int old = shape->variant < 4 ? std::min(column_blocks[shape->variant], 233472 / (1840 + 505 * nlay)) : 0;
+  if (shape->blocks_per_sm < 1 || shape->blocks_per_sm > std::max(occ, old)) {
     ctx->last_error = "blocks_per_sm exceeds what fits on an SM for this nlay and variant";
     return GB_LW_E_ARGS;
   }
@@ -1088,7 +1092,7 @@ int gb_rrtmg_lw_tuning_set(gb_lw_context* ctx, int nlay, int kind, const gb_lw_t
   t.variant = shape->variant;
   t.threads = gb_lw_variant(t.variant, lean).threads;
   t.min_blocks = gb_lw_variant(t.variant, lean).min_blocks;
-  t.blocks_per_sm = shape->blocks_per_sm;
+  t.blocks_per_sm = std::min(shape->blocks_per_sm, occ);
   t.blocks = t.blocks_per_sm * ctx->num_sms;
   t.ms = shape->ms;
   store_tuning(ctx, nlay, kind, t);

@@ -98,3 +98,20 @@ def test_network_rows_on_any_address(ctx, ncol):
     for k in OUTS:
         assert np.array_equal(got[0][k], got[1][k]), k
     mlp.close()
+
+
+@pytest.mark.parametrize("nlay,variant,blocks,ok", [(45, 0, 6, True), (60, 0, 6, True), (60, 1, 7, True), (38, 3, 4, True),
+                                                    (45, 0, 8, False), (45, 0, 0, False), (60, 3, 5, False)])
+def test_shapes_pinned_in_column_blocks(ctx, nlay, variant, blocks, ok):
+    """Shapes saved when a block was one column are taken, and run with as many units as fit."""
+    saved = ctx.tuning(nlay, kind=R.KIND_FUSED)
+    try:
+        if not ok:
+            with pytest.raises(R.RrtmgLwError):
+                ctx.set_tuning(nlay, variant, blocks, kind=R.KIND_FUSED)
+            return
+        ctx.set_tuning(nlay, variant, blocks, kind=R.KIND_FUSED)
+        got = ctx.tuning(nlay, kind=R.KIND_FUSED)
+        assert got["variant"] == variant and 1 <= got["blocks_per_sm"] <= blocks
+    finally:
+        ctx.set_tuning(nlay, saved["variant"], saved["blocks_per_sm"], kind=R.KIND_FUSED)
