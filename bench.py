@@ -27,7 +27,7 @@ transfer with FP64 heating rates.  One step solves every column once by:
                   copy counts for its phases (inatm, cldprmc, rtrnmc)
   batched      -- three nested grids (200x180x45, 150x150x45, 97x97x38) x 8
                   ensemble members with perturbed T and H2O, all in one
-                  persistent launch captured in a CUDA graph (taumol, fused
+                  call captured in a CUDA graph (taumol, fused
                   clouds), with HBM and FP32 rooflines and an oracle check
   eval         -- the learned gas optics on 512x512x45 columns: columns/s
                   and heating-rate RMSE against the FP64 oracle, beside the
@@ -808,7 +808,7 @@ def _errors(got, ref, n):
 
 
 def batched_block(ctx, dev, stream, args, hbm):
-    """Three nested grids x 8 members in one persistent launch captured in a CUDA graph."""
+    """Three nested grids x 8 members in one call captured in a CUDA graph."""
     import torch
 
     from brams_gb300 import surrogate as S
@@ -867,7 +867,7 @@ def batched_block(ctx, dev, stream, args, hbm):
     flops = sum((fl38 if g.nlay == 38 else fl45)["total"] * g.ncol for g in grids)
     tf = flops / t / 1e12
     return {"workload": "batched uneven grids 200x180x45 + 150x150x45 + 97x97x38, x 8 members (T + N(0,1 K), "
-                        "H2O x lognormal(0,0.2)), one persistent launch of taumol + transfer captured in a CUDA graph; "
+                        "H2O x lognormal(0,0.2)), one call (taumol + transfer) captured in a CUDA graph; "
                         "McICA clouds in the kernel; autotuned launch shape",
             "columns": ncols, "value": ncols / t, "unit": "columns/s", "ms_per_step": t * 1e3,
             "launch_shape": {k: best[k] for k in ("threads", "min_blocks", "blocks_per_sm")},
@@ -1215,7 +1215,7 @@ def abi_block(ctx, dev, stream, args, rank, world, hbm):
                         + ("360x300 columns x 45 layers" if ncol == NCOL else f"{ncol} columns x 45 layers"),
             "value": world * ncol / t_dev, "unit": "columns/s", "ms_per_step": t_dev * 1e3,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                         "traffic": traffic_from_profiles("lw_full_kernel_drop_in_traffic.txt"), "alg_bytes_per_launch": alg},
+                         "traffic": traffic_from_profiles("lw_drop_in_traffic.txt"), "alg_bytes_per_launch": alg},
             "e2e": {"value": world * ncol / t_e2e, "unit": "columns/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "host_path_matches_device_path": same},
             "launch_shape": ({k: shape[k] for k in ("threads", "min_blocks", "blocks_per_sm")} if shape

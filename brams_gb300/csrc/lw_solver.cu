@@ -5,7 +5,7 @@
 // 160 threads solves two neighbouring columns, 80 threads a column, each
 // standing for a pair of g-points of one band (70 live); an SM holds up to four units, which
 // walk the columns of a batch of grids.  Nothing per cell goes to global scratch
-// but the clouds of caller sub-columns:
+// but the planes between the kernels:
 //
 //   taumol -- of a batch, by kernels of its own (lw_taumol.cu), into a plane
 //     per column that the transfer reads; the batch goes through in passes of
@@ -21,9 +21,10 @@
 //     the layer's term list (lw_gasoptics.cuh) and one thread per (layer, g)
 //     cell gathers taug = sum w * table[row + g].
 //
-//   transfer (rt_column) -- inatm's column amounts, the laytrop and value
+//   transfer (rt_columns) -- inatm's column amounts, the laytrop and value
 //     checks, Planck interpolation per (layer, band) and the surface source,
-//     the McICA cloud bits and cldprmc's optical depths, then rtrnmc: a
+//     the McICA cloud bits and cldprmc's optical depths (caller sub-columns:
+//     lw_cells_kernel), then rtrnmc: a
 //     downward pass from the model top and an upward pass from the surface.
 //     Each pass evaluates a cell's transmittance and sources in registers from
 //     taug, the Planck fraction, the layer's Planck values and rtrnmc's
@@ -45,7 +46,7 @@
 //
 // Kernels: lw_rt_kernel (the transfer, on taumol's planes or on the network's
 // fp16 taug and Planck fractions; there, columns with a layer off the network
-// are handed over), lw_list_kernel (taumol and the transfer of the columns
+// are handed over), lw_cells_kernel (caller sub-columns' cells), lw_list_kernel (taumol and the transfer of the columns
 // handed over), lw_gas_kernel (taumol alone, for the network's training
 // samples and the gas-optics diagnostics).
 //

@@ -475,7 +475,7 @@ class Context:
         return n, arr
 
     def rrtmg_lw_batch_device(self, grids, stream=None) -> None:
-        """All grids (GridDesc list) in one persistent launch on `stream`."""
+        """All grids (GridDesc list) in one call on `stream`."""
         n, arr = self._grids(grids)
         _check(self.L, self.h, self.L.gb_rrtmg_lw_batch_device(self.h, _ptr(stream or 0), n, arr))
 

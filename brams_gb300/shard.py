@@ -79,7 +79,7 @@ def shard_grids(grids, world: int, rank: int) -> list[tuple[int, R.GridDesc]]:
 def solve_shard(ctx: R.Context, grids, world: int | None = None, rank: int | None = None, stream=None,
                 mlp: R.Mlp | None = None) -> list[tuple[int, R.GridDesc]]:
     """One rank's part of a batched call: its slices of `grids` in one
-    persistent launch on this process's device (rank and world default to
+    call on this process's device (rank and world default to
     torch.distributed's).  With `mlp` the slices run on the learned gas
     optics (gb_rrtmg_lw_batch_surrogate).  Returns the slices solved."""
     if world is None or rank is None:

@@ -297,7 +297,8 @@ int gb_mcica_subcol_lw_noalloc(void* stream, int ncol, int nlay, int icld, int p
  * Batched calls (no counterpart in the reference, which BRAMS calls once per
  * grid and MPI rank, rtm_driver.f90:1313): several grids -- nested grids,
  * ensemble members -- with their own column and layer counts are solved in
- * ONE persistent kernel launch.  Each grid is described by device arrays in
+ * one call, pass by pass of columns (gas optics, then the transfer's persistent
+ * kernel).  Each grid is described by device arrays in
  * the layouts of gb_rrtmg_lw_device.
  *
  * cloud_mode GB_LW_CLOUD_SUBCOL: McICA sub-column arrays as for
@@ -335,14 +336,14 @@ typedef struct gb_lw_grid {
   const uint8_t* sur_flag;
 } gb_lw_grid;
 
-/* Launch shape of the batched kernel: compiled variant (threads per column
- * block, register budget) and resident blocks per SM of the persistent grid. */
+/* Launch shape of the transfer kernel: compiled variant (threads per unit of
+ * two columns, register budget: min_blocks units an SM) and units per SM. */
 typedef struct gb_lw_tuning {
   int variant, threads, min_blocks, blocks_per_sm, blocks;
   double ms; /* measured time of the tuned shape on the sample batch (autotune only) */
 } gb_lw_tuning;
 
-/* All grids in one launch on `stream` (ngrid <= GB_LW_MAX_GRIDS), with the
+/* All grids, in order on `stream` (ngrid <= GB_LW_MAX_GRIDS), with the
  * shape the context's autotuner chose for this batch (largest nlay), or the
  * default shape.  Same status handling as gb_rrtmg_lw_device. */
 int gb_rrtmg_lw_batch_device(gb_lw_context* ctx, void* stream, int ngrid, const gb_lw_grid* grids);
@@ -366,8 +367,8 @@ int gb_rrtmg_lw_autotune_report(gb_lw_context* ctx, gb_lw_tuning* out, int max);
  * gb_rrtmg_lw_batch_device would use (tuned, pinned or the default); _set
  * pins one (variant and blocks_per_sm are used, the rest is derived).  For
  * the GB_LW_KIND_LEARNED kinds the variant is one of the learned-only
- * kernel's shapes (that kernel solves the columns wholly on the network; the
- * full kernel, in a second launch, the rest). */
+ * kernel's shapes (that kernel solves the columns wholly on the network; a
+ * hand-over kernel, in a second launch, the rest). */
 #define GB_LW_KIND_FUSED 1
 #define GB_LW_KIND_LEARNED 2
 int gb_rrtmg_lw_tuning_get(gb_lw_context* ctx, int nlay, int kind, gb_lw_tuning* out);
@@ -378,8 +379,7 @@ int gb_rrtmg_lw_num_variants(void);
 /* CUDA graph of one batched launch: the descriptor and the gas-optics
  * hand-over buffer owned by the graph are fixed at creation, so the caller
  * updates the input arrays in place between replays (a time-stepping model's
- * resident state).  The graph holds the batch's kernels (one persistent
- * launch for taumol batches). */
+ * resident state).  The graph holds the batch's kernels. */
 typedef struct gb_lw_graph gb_lw_graph;
 int gb_rrtmg_lw_batch_graph_create(gb_lw_context* ctx, int ngrid, const gb_lw_grid* grids,
                                    gb_lw_graph** graph);
