@@ -166,7 +166,9 @@ __device__ __forceinline__ void taumol_cell(const CoefCell& c, float* row) {
 
 __constant__ unsigned char c_order[16] = {5, 3, 13, 9, 7, 4, 8, 12, 15, 16, 6, 1, 11, 2, 10, 14};  // longest first
 
-__global__ void __launch_bounds__(TAU_NT, 8) lw_taumol_kernel(const __grid_constant__ LwBatch B,
+// PER_SM: blocks an SM the register allocation is sized for
+template <int PER_SM>
+__global__ void __launch_bounds__(TAU_NT, PER_SM) lw_taumol_kernel(const __grid_constant__ LwBatch B,
                                                               const float* __restrict__ T, long long u0,
                                                               long long nslot, int nblk) {
   // block -> (run of column blocks, band, block within the run)
@@ -216,6 +218,15 @@ cudaError_t gb_lw_launch_taumol(const LwBatch& b, const float* d_tables, long lo
   if (e != cudaSuccess) return e;
   const int per = gb::TAU_NT / 32;
   const int nblk = (int)((tiles * b.nsmax + per - 1) / per);
-  gb::lw_taumol_kernel<<<(unsigned)nblk * 16u, gb::TAU_NT, 0, stream>>>(b, d_tables, u0, nslot, nblk);
+  int dev = 0, nsm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // where every block is resident at four an SM, the more loads a warp has in
+  // flight at 128 registers count, not the warps (64 columns of 38 layers: 84 us
+  // a call at 64 registers, 82 at 128)
+  if (nblk * 16LL <= 4LL * nsm)
+    gb::lw_taumol_kernel<4><<<(unsigned)nblk * 16u, gb::TAU_NT, 0, stream>>>(b, d_tables, u0, nslot, nblk);
+  else
+    gb::lw_taumol_kernel<8><<<(unsigned)nblk * 16u, gb::TAU_NT, 0, stream>>>(b, d_tables, u0, nslot, nblk);
   return cudaGetLastError();
 }

@@ -115,3 +115,23 @@ def test_shapes_pinned_in_column_blocks(ctx, nlay, variant, blocks, ok):
         assert got["variant"] == variant and 1 <= got["blocks_per_sm"] <= blocks
     finally:
         ctx.set_tuning(nlay, saved["variant"], saved["blocks_per_sm"], kind=R.KIND_FUSED)
+
+
+def test_small_calls_equal_their_columns_in_a_large_one(ctx):
+    """taumol's two register allocations (few blocks, many) give a column the same bits."""
+    import torch
+
+    from brams_gb300.shard import slice_grid
+
+    st = make_state(ProfileSpec(ncol=1000, nlay=38, seed=17, t_noise=4.0, h2o_sigma=0.5))
+    g = S.DeviceGrid(st, pyoracle.cldprop_columns(st))
+    whole = _solve(ctx, [g], [5])[0]
+    for k in OUTS:
+        g.d[k].zero_()
+    d = g.desc(seed0=5)
+    for c0 in range(0, 1000, 40):
+        ctx.rrtmg_lw_batch_device([slice_grid(d, c0, c0 + 40)])
+    torch.cuda.synchronize()
+    got = g.outputs()
+    for k in OUTS:
+        assert np.array_equal(got[k], whole[k]), k
