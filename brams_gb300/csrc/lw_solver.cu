@@ -67,10 +67,10 @@
 #include "lw_common.h"
 #include "lw_solver.h"
 #include "lw_gasoptics.cuh"
+#include "lw_table.cuh"
 
 namespace gb {
 
-constexpr float BPADE = 1.0f / 0.278f;
 constexpr float REC_6 = 0.166667f;
 constexpr int TGROUP = MAXT_ALL;  // term slots per layer of a band's term list
 constexpr int RT_NT = 160;        // threads per block of two columns; virtual threads per column in the
@@ -171,30 +171,6 @@ __device__ __forceinline__ float sum8(float2 v0, float2 v1, float2 v2, float2 v3
   k += __shfl_xor_sync(0xffffffffu, f ? k0 : k1, 4);
   k += __shfl_xor_sync(0xffffffffu, k, 8);
   return k;
-}
-
-// od / (bpade + od) as __fdividef forms it (a divisor above 2^126 gives 0), without its scaling of
-// subnormal divisors, which bpade + od is not
-__device__ __forceinline__ float tbl_quotient(float od) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(BPADE + od));
-  return od * r;
-}
-// rtrnmc's table index of an optical depth (rrtmg_lw_rtrnmc.f90:385-388):
-// itr = int(tblint * od / (bpade + od) + 0.5), within 0 .. ntbl (od >= 0, and
-// a quotient that is not a number converts to 0)
-__device__ __forceinline__ int tbl_index(float od) {
-  const float tblind = __fdividef(od, BPADE + od);
-  const int itr = (int)fmaf(10000.0f, tblind, 0.5f);
-  return itr < 0 ? 0 : (itr > 10000 ? 10000 : itr);
-}
-// tau_tbl at an index formed in registers, bpade * t / (1 - t) at t = itr /
-// 10000 (1e10 at the last entry; rrtmg_lw_init.f90:120-142), instead of a
-// table load that depends on the clear cell's lookup (fp32 arithmetic: within
-// a few units in the last place of the fp64-built table's float)
-__device__ __forceinline__ float tbl_tau(int itr) {
-  const float t = (float)itr * 1.0e-4f;
-  return itr >= 10000 ? 1.0e10f : BPADE * t / (1.0f - t);
 }
 
 // cldprmc's optical depth ciwp*abscoice + clwp*abscoliq of one cell
