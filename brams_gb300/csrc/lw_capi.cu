@@ -33,18 +33,36 @@ struct gb_lw_graph {
   gb_lw_context* ctx = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  float* gas = nullptr;      // taumol hand-over planes
+  GbScratch gas;             // taumol hand-over planes
   double* draws = nullptr;  // McICA draws of the fused-cloud grids
   long long* fall = nullptr;  // hand-over list of a batch with learned gas optics
   unsigned* nfall = nullptr;
 };
 
-bool gb_capturing(cudaStream_t s) {
+namespace {
+// whether the stream is being captured (nothing can be allocated then)
+bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
   cudaGetLastError();
   return false;
 }
+void* device_get(size_t bytes) {
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+void device_put(void* p) { cudaFree(p); }
+const GbAlloc kDevice = {device_get, device_put};
+}  // namespace
+
+int gb_ctx_scratch(gb_lw_context* ctx, GbScratch& b, size_t want, size_t least, cudaStream_t s, const char* what) {
+  if (b.ensure(want, least, capturing(s), kDevice)) return 0;
+  ctx->last_error = std::string("device allocation failed: ") + what;
+  return GB_LW_E_NOMEM;
+}
+void gb_scratch_close(GbScratch& b) { b.close(kDevice); }
 
 int gb_ctx_fail(gb_lw_context* c, cudaError_t e, const char* where) {
   if (c) c->last_error = std::string(where) + ": " + cudaGetErrorString(e);
@@ -147,28 +165,6 @@ cudaError_t copy2d(double* dst, size_t dpitch, const double* src, size_t spitch,
   return cudaMemcpy2DAsync(dst, dpitch * 8, src, spitch * 8, width * 8, rows, kind, s);
 }
 
-// a gas-optics hand-over buffer of about `bytes` (grown on demand).  A buffer of
-// at least `least` bytes also does, with more passes per call: it is kept
-// under stream capture, where nothing can be allocated, and taken in place of
-// a larger one that does not fit on the device.
-int ensure_buffer(gb_lw_context* ctx, float** buf, size_t* have, size_t bytes, size_t least, cudaStream_t stream) {
-  if (*buf && (*have >= bytes || (*have >= least && gb_capturing(stream)))) return 0;
-  cudaFree(*buf);
-  *buf = nullptr;
-  *have = 0;
-  for (size_t n = bytes;; n = std::max(n / 2, least)) {
-    if (cudaMalloc(buf, n) == cudaSuccess) {
-      *have = n;
-      return 0;
-    }
-    cudaGetLastError();
-    *buf = nullptr;
-    if (n <= least) break;
-  }
-  ctx->last_error = "device allocation of the gas-optics hand-over planes failed";
-  return GB_LW_E_NOMEM;
-}
-
 bool flags_ok(int idrv, int inflglw, int iceflglw, int liqflglw) {
   return (idrv == 0 || idrv == 1) && inflglw >= 0 && inflglw <= 2 && iceflglw >= 0 && iceflglw <= 3 &&
          liqflglw >= 0 && liqflglw <= 1;
@@ -228,10 +224,10 @@ int launch_one(gb_lw_context* ctx, const LwArgs& a, int k, cudaStream_t stream) 
   b.col0[0] = 0;
   b.col0[1] = a.ncol;
   b.g[0] = a;
-  int rc = ensure_buffer(ctx, &ctx->d_gas[k], &ctx->gas_bytes[k], gb_lw_gas_bytes(b, false),
-                         gb_lw_gas_min_bytes(a.nlay), stream);
+  GbScratch& gas = ctx->gas[k];
+  int rc = gb_ctx_scratch(ctx, gas, gb_lw_gas_bytes(b, false), gb_lw_gas_min_bytes(a.nlay), stream, "gas-optics planes");
   if (rc) return rc;
-  gb_lw_attach_gas(b, ctx->d_gas[k], ctx->gas_bytes[k]);
+  gb_lw_attach_gas(b, gas.p, gas.bytes);
   const gb_lw_tuning t = tuning_for(ctx, a.nlay, batch_kind(b));
   cudaError_t e = gb_lw_launch_batch(b, ctx->d_tables, t.variant, t.blocks, stream);
   return e == cudaSuccess ? GB_LW_OK : gb_ctx_fail(ctx, e, "column kernels");
@@ -239,29 +235,20 @@ int launch_one(gb_lw_context* ctx, const LwArgs& a, int k, cudaStream_t stream) 
 
 // A batch with learned gas optics gets the context's hand-over list (room
 // for every column of the batch); other batches run the full kernel alone.
-int attach_fall(gb_lw_context* ctx, LwBatch& b) {
+int attach_fall(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
   b.fall = nullptr;
   b.nfall = nullptr;
   if (!(batch_kind(b) & GB_LW_KIND_LEARNED)) return 0;
-  const size_t need = (size_t)b.col0[b.ngrid];
-  if (need > ctx->fall_elems || !ctx->d_nfall) {
-    cudaFree(ctx->d_fall);
-    ctx->d_fall = nullptr;
-    ctx->fall_elems = 0;
-    if (!ctx->d_nfall && cudaMalloc(&ctx->d_nfall, sizeof(unsigned)) != cudaSuccess) {
-      cudaGetLastError();
-      ctx->d_nfall = nullptr;
-      ctx->last_error = "device allocation of the hand-over list failed";
-      return GB_LW_E_NOMEM;
-    }
-    if (cudaMalloc(&ctx->d_fall, need * sizeof(long long)) != cudaSuccess) {
-      cudaGetLastError();
-      ctx->last_error = "device allocation of the hand-over list failed";
-      return GB_LW_E_NOMEM;
-    }
-    ctx->fall_elems = need;
+  const size_t need = (size_t)b.col0[b.ngrid] * sizeof(long long);
+  int rc = gb_ctx_scratch(ctx, ctx->fall, need, need, stream, "hand-over list");
+  if (rc) return rc;
+  if (!ctx->d_nfall && cudaMalloc(&ctx->d_nfall, sizeof(unsigned)) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->d_nfall = nullptr;
+    ctx->last_error = "device allocation failed: hand-over list";
+    return GB_LW_E_NOMEM;
   }
-  b.fall = ctx->d_fall;
+  b.fall = static_cast<long long*>(ctx->fall.p);
   b.nfall = ctx->d_nfall;
   return 0;
 }
@@ -331,14 +318,12 @@ int gb_ctx_make_batch(gb_lw_context* ctx, int ngrid, const gb_lw_grid* grids, do
 
 // hand-over planes for a descriptor's columns from the context's batch buffer
 static int attach_batch_gas(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
-  int rc = ensure_buffer(ctx, &ctx->d_bgas, &ctx->bgas_bytes,
-                         gb_lw_gas_bytes(b, batch_kind(b) & GB_LW_KIND_LEARNED),
-                         gb_lw_gas_min_bytes(b.nsmax), stream);
+  int rc = gb_ctx_scratch(ctx, ctx->bgas, gb_lw_gas_bytes(b, batch_kind(b) & GB_LW_KIND_LEARNED),
+                          gb_lw_gas_min_bytes(b.nsmax), stream, "gas-optics planes");
   if (rc) return rc;
-  gb_lw_attach_gas(b, ctx->d_bgas, ctx->bgas_bytes);
+  gb_lw_attach_gas(b, ctx->bgas.p, ctx->bgas.bytes);
   return 0;
 }
-
 
 size_t gb_ctx_fused_draws(const LwBatch& b) {
   size_t n = 0;
@@ -360,29 +345,22 @@ int gb_ctx_make_draws(gb_lw_context* ctx, LwBatch& b, double* buf, cudaStream_t 
   return GB_LW_OK;
 }
 
+// the draws of a descriptor's fused-cloud grids, into the context's buffer
+static int context_draws(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
+  const size_t need = gb_ctx_fused_draws(b) * sizeof(double);
+  if (!need) return 0;
+  int rc = gb_ctx_scratch(ctx, ctx->fdraws, need, need, stream, "McICA draws");
+  return rc ? rc : gb_ctx_make_draws(ctx, b, static_cast<double*>(ctx->fdraws.p), stream);
+}
+
 int gb_ctx_launch_batch(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
   if (b.col0[b.ngrid] == 0) return GB_LW_OK;
   cudaSetDevice(ctx->device);
   const gb_lw_tuning t = tuning_for(ctx, b.nsmax, batch_kind(b));
   int rc = attach_batch_gas(ctx, b, stream);
   if (rc) return rc;
-  const size_t nd = gb_ctx_fused_draws(b);
-  if (nd > ctx->fdraws_elems) {
-    cudaFree(ctx->d_fdraws);
-    ctx->d_fdraws = nullptr;
-    ctx->fdraws_elems = 0;
-    if (cudaMalloc(&ctx->d_fdraws, nd * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      ctx->last_error = "device allocation of the McICA draws failed";
-      return GB_LW_E_NOMEM;
-    }
-    ctx->fdraws_elems = nd;
-  }
-  if (nd) {
-    rc = gb_ctx_make_draws(ctx, b, ctx->d_fdraws, stream);
-    if (rc) return rc;
-  }
-  if ((rc = attach_fall(ctx, b)) != 0) return rc;
+  if ((rc = context_draws(ctx, b, stream)) != 0) return rc;
+  if ((rc = attach_fall(ctx, b, stream)) != 0) return rc;
   cudaError_t e = gb_lw_launch_batch(b, ctx->d_tables, t.variant, t.blocks, stream);
   if (e != cudaSuccess) return gb_ctx_fail(ctx, e, "batched launch");
   return GB_LW_OK;
@@ -486,20 +464,13 @@ int gb_rrtmg_lw_free(gb_lw_context* ctx) {
     if (s) cudaStreamDestroy(s);
   cudaFree(ctx->d_tables);
   cudaFree(ctx->d_err);
-  cudaFree(ctx->d_draws);
-  for (auto& p : ctx->d_gas) cudaFree(p);
-  cudaFree(ctx->d_bgas);
-  cudaFree(ctx->d_sur);
-  cudaFree(ctx->d_sur_flag);
-  cudaFree(ctx->d_fdraws);
-  cudaFree(ctx->d_fall);
+  for (GbScratch* b : {&ctx->draws, &ctx->gas[0], &ctx->gas[1], &ctx->bgas, &ctx->sur, &ctx->sur_flag, &ctx->fdraws,
+                       &ctx->fall, &ctx->band, &ctx->ncb, &ctx->sw_scratch})
+    gb_scratch_close(*b);
   cudaFree(ctx->d_nfall);
   cudaFree(ctx->d_cloud64);
-  cudaFree(ctx->d_band);
-  cudaFree(ctx->d_ncb);
   cudaFree(ctx->d_sw_tables);
   cudaFree(ctx->d_sw_tables_f);
-  cudaFree(ctx->d_sw_scratch);
   if (ctx->lw_const_held) gb_const_release(GB_CONST_LW, ctx->device);
   if (ctx->sw_const_held) gb_const_release(GB_CONST_SW, ctx->device);
   delete ctx;
@@ -670,22 +641,6 @@ int gb_rrtmg_lw(gb_lw_context* ctx, int ncol, int nlay, int* icld, int idrv, con
 
 namespace {
 
-// grows a device array of the context to at least `n` elements of `size` bytes
-int ensure_elems(gb_lw_context* ctx, void** p, size_t* have, size_t n, size_t size, const char* what) {
-  if (*p && *have >= n) return 0;
-  cudaFree(*p);
-  *p = nullptr;
-  *have = 0;
-  if (cudaMalloc(p, n * size) != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
-    ctx->last_error = std::string("device allocation failed: ") + what;
-    return GB_LW_E_NOMEM;
-  }
-  *have = n;
-  return 0;
-}
-
 // argument checks shared by the non-McICA entry points
 int nomcica_check(gb_lw_context* ctx, int ncol, int nlay, int* icld, int idrv, int inflglw, int iceflglw,
                   int liqflglw, int64_t ld_in, int64_t ld_out) {
@@ -706,18 +661,18 @@ int nomcica_launch(gb_lw_context* ctx, LwArgs a, const double* cldfr, const doub
                    const double* cliqwp, const double* reice, const double* reliq, int k, cudaStream_t stream) {
   a.cloud_mode = LW_CLOUD_BAND;
   if (a.icld >= 1) {
-    int rc = ensure_elems(ctx, reinterpret_cast<void**>(&ctx->d_band), &ctx->band_elems, (size_t)16 * a.ld * a.nlay,
-                          sizeof(double), "band cloud depths");
-    if (!rc)
-      rc = ensure_elems(ctx, reinterpret_cast<void**>(&ctx->d_ncb), &ctx->ncb_elems, (size_t)a.ld, sizeof(int),
-                        "cloud-band counts");
+    const size_t nband = (size_t)16 * a.ld * a.nlay * sizeof(double), nncb = (size_t)a.ld * sizeof(int);
+    int rc = gb_ctx_scratch(ctx, ctx->band, nband, nband, stream, "band cloud depths");
+    if (!rc) rc = gb_ctx_scratch(ctx, ctx->ncb, nncb, nncb, stream, "cloud-band counts");
+    double* band = static_cast<double*>(ctx->band.p);
+    int* ncb = static_cast<int*>(ctx->ncb.p);
     if (!rc)
       rc = gb_ctx_cldprop(ctx, stream, a.ncol, a.nlay, a.inflag, a.iceflag, a.liqflag, cldfr, taucld, cicewp, cliqwp,
-                          reice, reliq, ctx->d_band, a.ld, a.col_err, ctx->d_ncb, a.err_flag);
+                          reice, reliq, band, a.ld, a.col_err, ncb, a.err_flag);
     if (rc) return rc;
     a.cldfrac = cldfr;
-    a.tauc = ctx->d_band;
-    a.ncbands = ctx->d_ncb;
+    a.tauc = band;
+    a.ncbands = ncb;
   } else if (a.col_err) {
     CK(cudaMemsetAsync(a.col_err, 0, sizeof(int) * (size_t)a.ncol, stream));
   }
@@ -892,17 +847,9 @@ int gb_mcica_subcol_lw_device(gb_lw_context* ctx, void* stream, int ncol, int nl
   if (*irng == 0 && nlay < 4) return GB_LW_E_ARGS;
   if (ncol == 0) return GB_LW_OK;
   cudaSetDevice(ctx->device);
-  size_t need = gb_mcica_draw_count(ncol, nlay, icld);
-  if (need > ctx->draws_elems) {
-    cudaFree(ctx->d_draws);
-    ctx->d_draws = nullptr;
-    ctx->draws_elems = 0;
-    if (cudaMalloc(&ctx->d_draws, need * 8) != cudaSuccess) {
-      cudaGetLastError();
-      return GB_LW_E_NOMEM;
-    }
-    ctx->draws_elems = need;
-  }
+  const size_t need = gb_mcica_draw_count(ncol, nlay, icld) * sizeof(double);
+  int rc = gb_ctx_scratch(ctx, ctx->draws, need, need, (cudaStream_t)stream, "McICA draws");
+  if (rc) return rc;
   McicaArgs a{};
   a.mode = *irng == 0 ? MCICA_PERCOL_KISS : (seed_per_column ? MCICA_PERCOL_MT : MCICA_STREAM_MT);
   a.ncol = ncol;
@@ -916,7 +863,7 @@ int gb_mcica_subcol_lw_device(gb_lw_context* ctx, void* stream, int ncol, int nl
   a.cldfmcl = cldfmcl; a.ciwpmcl = ciwpmcl; a.clwpmcl = clwpmcl; a.taucmcl = taucmcl;
   a.reicmcl = reicmcl; a.relqmcl = relqmcl;
   for (int g = 0; g < GB_NGPT; ++g) a.ngb[g] = ctx->tabs.ngb[g];
-  CK(gb_mcica_launch(a, ctx->d_draws, ctx->d_err, (cudaStream_t)stream, seed_per_column != 0));
+  CK(gb_mcica_launch(a, static_cast<double*>(ctx->draws.p), ctx->d_err, (cudaStream_t)stream, seed_per_column != 0));
   return GB_LW_OK;
 }
 
@@ -1129,20 +1076,9 @@ int gb_rrtmg_lw_autotune(gb_lw_context* ctx, void* stream, int ngrid, const gb_l
   if (cands.empty()) return GB_LW_E_ARGS;
   (void)max_blocks;
   if ((rc = attach_batch_gas(ctx, b, st)) != 0) return rc;
-  if ((rc = attach_fall(ctx, b)) != 0) return rc;
+  if ((rc = attach_fall(ctx, b, st)) != 0) return rc;
   // the fused-cloud draws are made once: every candidate times the column kernel alone
-  const size_t nd = gb_ctx_fused_draws(b);
-  if (nd > ctx->fdraws_elems) {
-    cudaFree(ctx->d_fdraws);
-    ctx->d_fdraws = nullptr;
-    ctx->fdraws_elems = 0;
-    if (cudaMalloc(&ctx->d_fdraws, nd * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      return GB_LW_E_NOMEM;
-    }
-    ctx->fdraws_elems = nd;
-  }
-  if (nd && (rc = gb_ctx_make_draws(ctx, b, ctx->d_fdraws, st)) != 0) return rc;
+  if ((rc = context_draws(ctx, b, st)) != 0) return rc;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -1204,14 +1140,12 @@ int gb_rrtmg_lw_batch_graph_create(gb_lw_context* ctx, int ngrid, const gb_lw_gr
   const gb_lw_tuning t = tuning_for(ctx, b.nsmax, batch_kind(b));
   gb_lw_graph* g = new gb_lw_graph();
   g->ctx = ctx;
-  size_t gbytes = 0;
-  if ((rc = ensure_buffer(ctx, &g->gas, &gbytes,
-                          gb_lw_gas_bytes(b, batch_kind(b) & GB_LW_KIND_LEARNED),
-                          gb_lw_gas_min_bytes(b.nsmax), nullptr)) != 0) {
+  if ((rc = gb_ctx_scratch(ctx, g->gas, gb_lw_gas_bytes(b, batch_kind(b) & GB_LW_KIND_LEARNED),
+                           gb_lw_gas_min_bytes(b.nsmax), nullptr, "gas-optics planes")) != 0) {
     delete g;
     return rc;
   }
-  gb_lw_attach_gas(b, g->gas, gbytes);
+  gb_lw_attach_gas(b, g->gas.p, g->gas.bytes);
   const size_t nd = gb_ctx_fused_draws(b);
   if (nd && cudaMalloc(&g->draws, nd * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
@@ -1259,7 +1193,7 @@ int gb_rrtmg_lw_graph_destroy(gb_lw_graph* g) {
   cudaSetDevice(g->ctx->device);
   if (g->exec) cudaGraphExecDestroy(g->exec);
   if (g->graph) cudaGraphDestroy(g->graph);
-  cudaFree(g->gas);
+  gb_scratch_close(g->gas);
   cudaFree(g->draws);
   cudaFree(g->fall);
   cudaFree(g->nfall);

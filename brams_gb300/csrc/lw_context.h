@@ -7,6 +7,7 @@
 
 #include "../../include/gb_rrtmg_lw.h"
 #include "lw_common.h"
+#include "lw_scratch.h"
 #include "lw_solver.h"
 
 struct ChunkBufs {
@@ -26,37 +27,25 @@ struct gb_lw_context {
   cudaStream_t streams[2] = {nullptr, nullptr};
   ChunkBufs bufs[2];
   int chunk_cols = 0, chunk_nlay = 0;
-  double* d_draws = nullptr;
-  size_t draws_elems = 0;
-  // taumol hand-over planes of the single-grid calls (one buffer per chunk stream)
-  float* d_gas[2] = {nullptr, nullptr};
-  size_t gas_bytes[2] = {0, 0};
+  GbScratch draws;   // the sub-column generators' random draws
+  GbScratch gas[2];  // taumol hand-over planes of the single-grid calls (one buffer per chunk stream)
   std::string last_error;
   size_t max_smem = 0;
   int num_sms = 0;
-  float* d_bgas = nullptr;  // taumol hand-over planes of batched launches
-  size_t bgas_bytes = 0;
+  GbScratch bgas;  // taumol hand-over planes of batched launches
   std::vector<gb_lw_tuning> tuned;  // autotuned shapes, parallel to tuned_nlay (largest nlay of the batch)
   std::vector<int> tuned_nlay;
   std::vector<gb_lw_tuning> last_tune;  // every candidate of the last autotune call
-  // McICA draws of fused-cloud grids in batched calls (grown on demand)
-  double* d_fdraws = nullptr;
-  size_t fdraws_elems = 0;
+  GbScratch fdraws;  // McICA draws of fused-cloud grids in batched calls
   // columns the learned-only kernel hands over to the full kernel, and their
-  // count (batches with learned gas optics; grown on demand)
-  long long* d_fall = nullptr;
+  // count (batches with learned gas optics)
+  GbScratch fall;
   unsigned* d_nfall = nullptr;
-  size_t fall_elems = 0;
-  // surrogate outputs of batched calls with a network (grown on demand)
-  uint16_t* d_sur = nullptr;  // fp16 taug and Planck fractions
-  unsigned char* d_sur_flag = nullptr;
-  size_t sur_rows = 0;
+  // surrogate outputs of batched calls with a network: fp16 taug and Planck fractions, the layers' flags
+  GbScratch sur, sur_flag;
   // band clouds of the non-McICA calls: cldprop's optical depths (16, ncol,
-  // nlay) and cloud-band counts (ncol) (grown on demand)
-  double* d_band = nullptr;
-  size_t band_elems = 0;
-  int* d_ncb = nullptr;
-  size_t ncb_elems = 0;
+  // nlay) and cloud-band counts (ncol)
+  GbScratch band, ncb;
   // RRTMG_SW: tables (fp64 and fp32 blobs, loaded by gb_rrtmg_sw_ini), the
   // precision of the column kernel (gb_rrtmg_sw_set_precision) and the
   // column blocks' scratch slots
@@ -66,8 +55,7 @@ struct gb_lw_context {
   bool sw_ready = false;
   int sw_bits = 32;
   double sw_scon = 0.0;  // rrsw_scon of the tables (parrrsw.f90)
-  void* d_sw_scratch = nullptr;
-  size_t sw_scratch_bytes = 0;
+  GbScratch sw_scratch;
   // this context's hold on its device's constant table blocks (see below)
   bool lw_const_held = false, sw_const_held = false;
 };
@@ -83,8 +71,10 @@ enum GbConstKind { GB_CONST_LW = 0, GB_CONST_SW = 1 };
 bool gb_const_acquire(int kind, int device, const void* bytes, size_t n, bool* upload);
 void gb_const_release(int kind, int device);
 
-// whether the stream is being captured (nothing can be allocated then)
-bool gb_capturing(cudaStream_t s);
+// a context's scratch of `want` bytes, or at least `least`, for a call on stream s (GbScratch::ensure);
+// GB_LW_E_NOMEM, with `what` in the last error, where there is none
+int gb_ctx_scratch(gb_lw_context* ctx, GbScratch& b, size_t want, size_t least, cudaStream_t s, const char* what);
+void gb_scratch_close(GbScratch& b);
 // records a CUDA error on the context; returns GB_LW_E_CUDA
 int gb_ctx_fail(gb_lw_context* c, cudaError_t e, const char* where);
 // validates a batched call's grids and fills the launch descriptor (frac < 1: sample of each grid)

@@ -454,37 +454,26 @@ int gb_rrtmg_lw_batch_surrogate(gb_lw_context* ctx, void* stream, int ngrid, con
   cudaSetDevice(ctx->device);
   size_t rows = 0;
   for (int i = 0; i < ngrid; ++i) rows += (size_t)std::max(grids[i].ncol, 0) * std::max(grids[i].nlay, 0);
-  if (rows > ctx->sur_rows) {
-    cudaFree(ctx->d_sur);
-    cudaFree(ctx->d_sur_flag);
-    ctx->d_sur = nullptr;
-    ctx->d_sur_flag = nullptr;
-    ctx->sur_rows = 0;
-    if (cudaMalloc(&ctx->d_sur, rows * 2 * GB_NGPT_MLP * sizeof(uint16_t)) != cudaSuccess ||
-        cudaMalloc(&ctx->d_sur_flag, rows) != cudaSuccess) {
-      cudaGetLastError();
-      ctx->last_error = "device allocation of the learned gas-optics buffers failed";
-      return GB_LW_E_NOMEM;
-    }
-    ctx->sur_rows = rows;
-  }
+  const size_t nsur = rows * 2 * GB_NGPT_MLP * sizeof(uint16_t);
+  int rc = 0;
+  if (rows) rc = gb_ctx_scratch(ctx, ctx->sur, nsur, nsur, (cudaStream_t)stream, "learned gas-optics values");
+  if (rows && !rc) rc = gb_ctx_scratch(ctx, ctx->sur_flag, rows, rows, (cudaStream_t)stream, "learned gas-optics flags");
+  if (rc) return rc;
   std::vector<gb_lw_grid> g(grids, grids + ngrid);
   size_t off = 0;
   for (int i = 0; i < ngrid; ++i) {
     const size_t r = (size_t)std::max(g[i].ncol, 0) * std::max(g[i].nlay, 0);
-    uint16_t* tau = ctx->d_sur + off * 2 * GB_NGPT_MLP;
+    uint16_t* tau = static_cast<uint16_t*>(ctx->sur.p) + off * 2 * GB_NGPT_MLP;
     uint16_t* frac = tau + r * GB_NGPT_MLP;
-    uint8_t* flag = ctx->d_sur_flag + off;
-    int rc = gb_lw_mlp_infer(m, stream, &g[i], tau, frac, flag);
-    if (rc) return rc;
+    uint8_t* flag = static_cast<uint8_t*>(ctx->sur_flag.p) + off;
+    if ((rc = gb_lw_mlp_infer(m, stream, &g[i], tau, frac, flag)) != 0) return rc;
     g[i].sur_tau = tau;
     g[i].sur_frac = frac;
     g[i].sur_flag = flag;
     off += r;
   }
   LwBatch b;
-  int rc = gb_ctx_make_batch(ctx, ngrid, g.data(), 1.0, b);
-  if (rc) return rc;
+  if ((rc = gb_ctx_make_batch(ctx, ngrid, g.data(), 1.0, b)) != 0) return rc;
   return gb_ctx_launch_batch(ctx, b, (cudaStream_t)stream);
 }
 

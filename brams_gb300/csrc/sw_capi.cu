@@ -66,27 +66,11 @@ int launch(gb_lw_context* ctx, const SwArgs& a, cudaStream_t stream) {
   const int bits = ctx->sw_bits;
   const long long slots = gb_sw_slots(ctx->num_sms, bits);
   const size_t need = gb_sw_scratch_bytes(a.nlay, bits, slots, a.ncol), least = gb_sw_scratch_bytes(a.nlay, bits, slots, 1);
-  // grown on demand; a smaller buffer, with more passes, is kept under stream
-  // capture and taken where the wanted one does not fit on the device
-  if (need > ctx->sw_scratch_bytes && !(least <= ctx->sw_scratch_bytes && gb_capturing(stream))) {
-    cudaFree(ctx->d_sw_scratch);
-    ctx->d_sw_scratch = nullptr;
-    ctx->sw_scratch_bytes = 0;
-    for (size_t n = need;; n = std::max(n / 2, least)) {
-      if (cudaMalloc(&ctx->d_sw_scratch, n) == cudaSuccess) {
-        ctx->sw_scratch_bytes = n;
-        break;
-      }
-      cudaGetLastError();
-      ctx->d_sw_scratch = nullptr;
-      if (n <= least) {
-        ctx->last_error = "device allocation of the SW scratch slots failed";
-        return GB_LW_E_NOMEM;
-      }
-    }
-  }
+  GbScratch& scr = ctx->sw_scratch;
+  int rc = gb_ctx_scratch(ctx, scr, need, least, stream, "SW scratch slots");
+  if (rc) return rc;
   const void* tables = bits == 32 ? (const void*)ctx->d_sw_tables_f : (const void*)ctx->d_sw_tables;
-  cudaError_t e = gb_sw_launch(a, bits, tables, ctx->d_sw_scratch, ctx->sw_scratch_bytes, slots, stream);
+  cudaError_t e = gb_sw_launch(a, bits, tables, scr.p, scr.bytes, slots, stream);
   return e == cudaSuccess ? GB_LW_OK : gb_ctx_fail(ctx, e, "SW column kernel");
 }
 
@@ -288,17 +272,9 @@ int gb_mcica_subcol_sw_device(gb_lw_context* ctx, void* stream, int ncol, int nl
     if (!p) return GB_LW_E_ARGS;
   if (ncol == 0) return GB_LW_OK;
   cudaSetDevice(ctx->device);
-  const size_t need = gb_mcica_draw_count(ncol, nlay, icld, SW_NGPT);
-  if (need > ctx->draws_elems) {
-    cudaFree(ctx->d_draws);
-    ctx->d_draws = nullptr;
-    ctx->draws_elems = 0;
-    if (cudaMalloc(&ctx->d_draws, need * 8) != cudaSuccess) {
-      cudaGetLastError();
-      return GB_LW_E_NOMEM;
-    }
-    ctx->draws_elems = need;
-  }
+  const size_t need = gb_mcica_draw_count(ncol, nlay, icld, SW_NGPT) * sizeof(double);
+  int rc = gb_ctx_scratch(ctx, ctx->draws, need, need, (cudaStream_t)stream, "McICA draws");
+  if (rc) return rc;
   McicaArgs a{};
   a.mode = *irng == 0 ? MCICA_PERCOL_KISS : (seed_per_column ? MCICA_PERCOL_MT : MCICA_STREAM_MT);
   a.ncol = ncol;
@@ -317,7 +293,7 @@ int gb_mcica_subcol_sw_device(gb_lw_context* ctx, void* stream, int ncol, int nl
   a.ssac = ssac; a.asmc = asmc; a.fsfc = fsfc;
   a.ssacmcl = ssacmcl; a.asmcmcl = asmcmcl; a.fsfcmcl = fsfcmcl;
   sw_ngb(a.ngb);
-  CKS(gb_mcica_launch(a, ctx->d_draws, ctx->d_err, (cudaStream_t)stream, seed_per_column != 0));
+  CKS(gb_mcica_launch(a, static_cast<double*>(ctx->draws.p), ctx->d_err, (cudaStream_t)stream, seed_per_column != 0));
   return GB_LW_OK;
 }
 
