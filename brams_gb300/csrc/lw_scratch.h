@@ -6,6 +6,10 @@
 // sets it aside.  A new one in its place is at least twice as large (and half
 // of what a call wants does where it is enough to run with), so all that are
 // set aside are together smaller than the one in use.
+//
+// Where the device has no room for what a call wants, the call runs with less,
+// and that size is not asked for again: calls of its size and above keep the
+// buffer they have, without an allocation (and its synchronisation) each.
 #pragma once
 #include <algorithm>
 #include <cstddef>
@@ -25,8 +29,9 @@ class GbScratch {
   // (a solver call then makes more passes).  Under stream capture, where
   // nothing can be allocated, `least` does.  False: there is none.
   bool ensure(size_t want, size_t least, bool capturing, const GbAlloc& a) {
-    const bool does = p && bytes >= least && (bytes >= want || capturing || (captured && bytes >= want / 2));
-    if (!does && !grow(captured ? std::max(want, 2 * bytes) : want, least, capturing, a)) return false;
+    const bool runs = p && bytes >= least;
+    const bool does = runs && (bytes >= want || capturing || want >= refused || (captured && bytes >= want / 2));
+    if (!does && !grow(want, least, capturing, a)) return false;
     captured |= capturing;
     return true;
   }
@@ -39,25 +44,40 @@ class GbScratch {
   }
 
  private:
-  bool captured = false;      // a captured call has used p
-  std::vector<void*> aside;   // outgrown, still held by graphs
+  bool captured = false;       // a captured call has used p
+  size_t refused = ~size_t(0);  // the least wanted that the device had no room for
+  std::vector<void*> aside;    // outgrown, still held by graphs
 
+  // the largest of want, want / 2, .. least above `over` that can be had
+  static void* most(size_t want, size_t least, size_t over, const GbAlloc& a, size_t* n) {
+    for (*n = want; *n > over; *n = std::max(*n / 2, least)) {
+      if (void* q = a.get(*n)) return q;
+      if (*n <= least) break;
+    }
+    return nullptr;
+  }
   bool grow(size_t want, size_t least, bool capturing, const GbAlloc& a) {
-    if (p) {
-      if (captured || capturing)
-        aside.push_back(p);
-      else
-        a.put(p);
+    const bool runs = p && bytes >= least, held = captured || capturing;
+    // the new buffer before the present one goes, which does where there is no room for a larger one
+    size_t n = 2 * bytes;
+    void* q = captured && n > want ? a.get(n) : nullptr;
+    if (!q) q = most(want, least, runs ? bytes : 0, a, &n);
+    if (!q && !runs && p && !held) {
+      a.put(p);
+      p = nullptr;
+      bytes = 0;
+      q = most(want, least, 0, a, &n);
     }
-    p = nullptr;
-    bytes = 0;
+    if (!capturing && (!q || n < want)) refused = std::min(refused, want);
+    if (!q) return runs;
+    if (p && held)
+      aside.push_back(p);
+    else if (p)
+      a.put(p);
+    p = q;
+    bytes = n;
     captured = false;
-    for (size_t n = want;; n = std::max(n / 2, least)) {
-      if ((p = a.get(n)) != nullptr) {
-        bytes = n;
-        return true;
-      }
-      if (n <= least) return false;
-    }
+    if (n >= refused) refused = ~size_t(0);
+    return true;
   }
 };

@@ -103,3 +103,56 @@ def test_less_is_taken_where_less_is_free(tmp_path):
   CHECK(!t.ensure(1000, 500, false, A) && t.p == nullptr);
   s.close(A);
 """)
+
+
+def test_a_size_that_did_not_fit_is_not_asked_for_again(tmp_path):
+    _run(tmp_path, """
+  limit = 300;
+  GbScratch s;
+  CHECK(s.ensure(1000, 100, false, A));       // 250 of it
+  void* p = s.p;
+  const size_t n = s.bytes;
+  const int g = gets, f = puts_;
+  for (int k = 0; k < 5; ++k) {
+    CHECK(s.ensure(1000, 100, false, A));
+    CHECK(s.ensure(4000, 200, false, A));
+    CHECK(s.ensure(90, 10, false, A));
+  }
+  CHECK(s.p == p && s.bytes == n && gets == g && puts_ == f);
+  limit = 1000;                               // a smaller size is still tried
+  CHECK(s.ensure(600, 100, false, A) && s.bytes == 600 && live.size() == 1);
+  CHECK(s.ensure(1000, 100, false, A) && s.bytes == 600);
+  CHECK(!s.ensure(1001, 1001, false, A));     // too little to run with, nothing larger
+  limit = 5000;
+  CHECK(s.ensure(2000, 2000, false, A) && s.bytes == 2000 && live.size() == 1);
+  s.close(A);
+  CHECK(live.empty());
+""")
+
+
+def test_a_buffer_that_does_is_not_given_up_for_a_larger_one(tmp_path):
+    _run(tmp_path, """
+  GbScratch s;
+  CHECK(s.ensure(300, 100, false, A));
+  void* p = s.p;
+  limit = 400;                                // no room for a larger one beside it
+  CHECK(s.ensure(5000, 100, false, A) && s.p == p && live.count(p));
+  CHECK(s.ensure(5000, 100, false, A) && s.p == p && puts_ == 0);
+  CHECK(s.ensure(350, 350, false, A) && s.bytes == 350 && live.size() == 1);  // needed: the old one makes room
+  s.close(A);
+  CHECK(live.empty());
+""")
+
+
+def test_nothing_is_freed_under_capture(tmp_path):
+    _run(tmp_path, """
+  GbScratch s;
+  CHECK(s.ensure(300, 100, false, A));
+  void* p = s.p;
+  limit = 300;
+  CHECK(!s.ensure(1000, 500, true, A));       // the call fails, the buffer stays
+  CHECK(live.count(p) && puts_ == 0 && s.p == p && s.bytes == 300);
+  limit = 2000;
+  CHECK(s.ensure(1000, 500, false, A) && s.bytes == 1000);  // and the size is tried again afterwards
+  s.close(A);
+""")
