@@ -17,6 +17,18 @@ __host__ __device__
 #endif
 constexpr int gb_pitch(int ng) { return ng <= 2 ? ng : (ng + 3) / 4 * 4; }
 
+#ifdef __CUDACC__
+// Lets a kernel be launched with any dynamic shared memory a block can have.
+// The attribute is the process's, and host threads with a context each launch
+// the same kernel with different amounts: it is only ever set to this one value.
+inline cudaError_t gb_allow_smem(const void* kernel) {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+}
+#endif
+
 // Offsets (in floats) of every band table inside the device table blob.
 // Layouts are g-fastest, rows of p = gb_pitch(ng) floats, every table on a
 // 16-byte boundary, so that a row's g-points are read by vector loads:

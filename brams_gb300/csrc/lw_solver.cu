@@ -1692,9 +1692,9 @@ cudaError_t set_carveout(const void* fn, size_t smem, int per) {
   return cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 
-// resident blocks per SM of `fn` with `threads` and `smem` (after allowing that much shared memory)
+// resident blocks per SM of `fn` with `threads` and `smem`
 cudaError_t occupancy(const void* fn, int threads, size_t smem, int* per) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = gb_allow_smem(fn);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, fn, threads, smem);
@@ -1866,7 +1866,7 @@ cudaError_t gb_lw_launch_batch(const LwBatch& bin, const float* d_tables, int va
     const int nunit = (int)std::min<long long>((want + nsm - 1) / nsm, units_per_sm(b.nsmax, b.cpb, v));
     const int blocks = (int)std::min<long long>((want + nunit - 1) / nunit, nsm);
     const size_t smem = block_smem(b.nsmax, b.cpb, nunit);
-    const cudaError_t e = cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = gb_allow_smem(v.fn);
     if (e != cudaSuccess) return e;
     return v.launch(b, d_tables, u0, u1, blocks, nunit * unit_threads(b.cpb), nunit, smem, stream);
   };
@@ -1881,7 +1881,7 @@ cudaError_t gb_lw_launch_batch(const LwBatch& bin, const float* d_tables, int va
       cudaError_t e = gb_lw_launch_taumol(b, d_tables, u0, u1, stream);
       if (e == cudaSuccess && b.cellw) {
         const size_t smem = gb::rt_smem_bytes(b.nsmax);
-        e = cudaFuncSetAttribute((const void*)gb::lw_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = gb_allow_smem((const void*)gb::lw_cells_kernel);
         if (e != cudaSuccess) return e;
         gb::lw_cells_kernel<<<(unsigned)((u1 - u0) * b.cpb), gb::CELL_NT, smem, stream>>>(b, d_tables, u0);
         e = cudaGetLastError();
