@@ -1027,12 +1027,13 @@ int gb_rrtmg_lw_tuning_set(gb_lw_context* ctx, int nlay, int kind, const gb_lw_t
   cudaSetDevice(ctx->device);
   const bool lean = kind & GB_LW_KIND_LEARNED;
   const int occ = gb_lw_slots(nlay, shape->variant, lean) / std::max(1, ctx->num_sms);
-  // shapes saved when a block was one column (6, 7, 5 and 4 of an SM at most, of
-  // 816 + 504.5 nlay bytes) are taken too, and run with as many units as fit
-  const int column_blocks[] = {6, 7, 5, 4};
-  const int old = shape->variant < 4 ? std::min(column_blocks[shape->variant], 233472 / (1840 + 505 * nlay)) : 0;
-  if (shape->blocks_per_sm < 1 || shape->blocks_per_sm > std::max(occ, old)) {
-    ctx->last_error = "blocks_per_sm exceeds what fits on an SM for this nlay and variant";
+  // What is taken is part of the interface, since programs keep shapes in
+  // files: 6, 7, 5 and 4 blocks of the variants at most, and as many as fit in
+  // an SM's 228 KB at 1,876 + 504 nlay bytes each (a block of one column; a
+  // unit of two needs less than two of these).  They run with as many units as fit.
+  const int most[] = {6, 7, 5, 4};
+  if (shape->blocks_per_sm < 1 || shape->blocks_per_sm > std::min(most[shape->variant], 233472 / (1876 + 504 * nlay))) {
+    ctx->last_error = "blocks_per_sm exceeds what is taken for this nlay and variant";
     return GB_LW_E_ARGS;
   }
   gb_lw_tuning t{};

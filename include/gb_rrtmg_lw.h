@@ -372,7 +372,9 @@ int gb_rrtmg_lw_autotune_report(gb_lw_context* ctx, gb_lw_tuning* out, int max);
  * if any grid generates its McICA clouds in the kernel, | GB_LW_KIND_LEARNED
  * if any grid uses learned gas optics.  _get returns the shape
  * gb_rrtmg_lw_batch_device would use (tuned, pinned or the default); _set
- * pins one (variant and blocks_per_sm are used, the rest is derived).  For
+ * pins one (variant and blocks_per_sm are used, the rest is derived;
+ * blocks_per_sm up to 6, 7, 5 and 4 of the variants and up to
+ * 233,472 / (1,876 + 504 nlay), run with as many as fit).  For
  * the GB_LW_KIND_LEARNED kinds the variant is one of the learned-only
  * kernel's shapes (that kernel solves the columns wholly on the network; a
  * hand-over kernel, in a second launch, the rest). */

@@ -16,6 +16,13 @@ FLUX_TOL, HR_TOL = 0.05, 0.01  # the solver's parity tolerances (W m-2, K/day)
 OUTS = ("uflx", "dflx", "hr", "uflxc", "dflxc", "hrc", "duflx_dt", "duflxc_dt")
 
 
+@pytest.fixture
+def own():
+    c = R.Context()
+    yield c
+    c.close()
+
+
 def _solve(ctx, grids, seeds):
     import torch
 
@@ -115,6 +122,27 @@ def test_shapes_pinned_in_column_blocks(ctx, nlay, variant, blocks, ok):
         assert got["variant"] == variant and 1 <= got["blocks_per_sm"] <= blocks
     finally:
         ctx.set_tuning(nlay, saved["variant"], saved["blocks_per_sm"], kind=R.KIND_FUSED)
+
+
+# the largest nlay at which 7, 6, .. 1 blocks per SM have been taken since shapes can be kept
+TAKEN = {7: 62, 6: 73, 5: 88, 4: 112, 3: 150, 2: 227, 1: 256}
+
+
+@pytest.mark.parametrize("kind", [R.KIND_FUSED, R.KIND_FUSED | R.KIND_LEARNED])
+@pytest.mark.parametrize("variant,most", enumerate((6, 7, 5, 4)))
+def test_which_shapes_are_taken(own, variant, most, kind):
+    def taken(nlay, blocks):
+        try:
+            own.set_tuning(nlay, variant, blocks, kind=kind)
+        except R.RrtmgLwError:
+            return False
+        return own.tuning(nlay, kind=kind)["blocks_per_sm"] <= blocks
+
+    for blocks, nlay in TAKEN.items():
+        for n in (nlay, nlay + 1):
+            if n <= 256:
+                assert taken(n, blocks) == (blocks <= most and n <= nlay), (blocks, n)
+    assert not taken(38, 0) and not taken(38, most + 1)
 
 
 def test_small_calls_equal_their_columns_in_a_large_one(ctx):
