@@ -129,7 +129,7 @@ TAKEN = {7: 62, 6: 73, 5: 88, 4: 112, 3: 150, 2: 227, 1: 256}
 
 
 @pytest.mark.parametrize("kind", [R.KIND_FUSED, R.KIND_FUSED | R.KIND_LEARNED])
-@pytest.mark.parametrize("variant,most", enumerate((6, 7, 5, 4)))
+@pytest.mark.parametrize("variant,most", [(0, 6), (1, 7), (2, 5), (3, 4)])
 def test_which_shapes_are_taken(own, variant, most, kind):
     def taken(nlay, blocks):
         try:
