@@ -36,7 +36,8 @@ cudaError_t gb_mlp_norm_targets(long long rows, const float* d_tau, const float*
 // forward + backward of one batch: gradients of the loss w.r.t. all parameters into d_grad (fp32, blob order); the
 // outputs stay in b.y where keep_y is true
 cudaError_t gb_mlp_forward_backward(const MlpBuffers& b, long long rows, const __nv_bfloat16* d_x, const float* d_t,
-                                    const float* d_w, float* d_grad, float* d_loss, bool keep_y, cudaStream_t st);
+                                    const float* d_w, float* d_grad, float* d_loss, bool keep_y, int num_sms,
+                                    cudaStream_t st);
 cudaError_t gb_mlp_adam(const MlpBuffers& b, const float* d_grad, float lr, int step, cudaStream_t st);
 cudaError_t gb_mlp_sync_bf16(const MlpBuffers& b, cudaStream_t st);
 // surrogate taug [(icol*nlay + lay)*140 + g], Planck fractions (same layout), both fp16 (taug clamped to

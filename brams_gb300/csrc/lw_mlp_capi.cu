@@ -378,7 +378,7 @@ int gb_lw_mlp_gradients(gb_lw_mlp* m, void* stream, int64_t rows, const void* d_
   cudaStream_t st = (cudaStream_t)stream;
   if (d_loss) cudaMemsetAsync(d_loss, 0, 4, st);
   cudaError_t e = gb_mlp_forward_backward(m->b, rows, (const __nv_bfloat16*)d_x, d_t, m->d_w,
-                                          d_grad ? d_grad : m->d_grad, d_loss, false, st);
+                                          d_grad ? d_grad : m->d_grad, d_loss, false, m->ctx->num_sms, st);
   return e == cudaSuccess ? GB_LW_OK : fail(m->ctx, e, "forward/backward");
 }
 
@@ -406,7 +406,8 @@ int gb_lw_mlp_forward(gb_lw_mlp* m, void* stream, int64_t rows, const void* d_x,
     return GB_LW_E_NOMEM;
   }
   cudaMemsetAsync(d_t, 0, (size_t)rows * GB_MLP_NOUTP * 4, st);
-  cudaError_t e = gb_mlp_forward_backward(m->b, rows, (const __nv_bfloat16*)d_x, d_t, m->d_w, m->d_grad, nullptr, true, st);
+  cudaError_t e = gb_mlp_forward_backward(m->b, rows, (const __nv_bfloat16*)d_x, d_t, m->d_w, m->d_grad, nullptr, true,
+                                          m->ctx->num_sms, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_y, m->b.y, (size_t)rows * GB_MLP_NOUTP * 4, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(d_t);
