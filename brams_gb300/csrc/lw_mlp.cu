@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const bool sums = EPI == EPI_ATOMIC && blockIdx.y == 0;
-  float cs[4] = {};  // sums over rows 4 i + q of this thread's half of the B tiles' rows
+  float cs = 0.0f;  // sum over this thread's half of the B tiles' rows
 #pragma unroll
   for (int i = 0; i < STAGES - 1; ++i) stage(i);
   for (int step = 0; k0 + step * BK < k1; ++step) {
@@ -121,9 +121,11 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
     stage(step + STAGES - 1);
     const bf16 *sA = tA[step % STAGES], *sB = tB[step % STAGES];
     if (sums) {
+      float v[4] = {};
 #pragma unroll
       for (int r = 0; r < BK / 2; ++r)
-        cs[r & 3] += __bfloat162float(sB[((tid >> 6) * (BK / 2) + r) * (BN + PAD) + (tid & 63)]);
+        v[r & 3] += __bfloat162float(sB[((tid >> 6) * (BK / 2) + r) * (BN + PAD) + (tid & 63)]);
+      cs += (v[0] + v[1]) + (v[2] + v[3]);
     }
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 16) {
@@ -158,7 +160,12 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   // ---- epilogue
-  if (sums && bn + (tid & 63) < g.N) atomicAdd(g.colsum + bn + (tid & 63), (cs[0] + cs[1]) + (cs[2] + cs[3]));
+  if (sums) {  // one sum per block and column: each that is added to the total is rounded at the total's size
+    __shared__ float half[64];
+    if (tid >= 64) half[tid - 64] = cs;
+    __syncthreads();
+    if (tid < 64 && bn + tid < g.N) atomicAdd(g.colsum + bn + tid, cs + half[tid]);
+  }
   const float scale = EPI == EPI_LOSS ? 1.0f / ((float)g.M * (float)GB_MLP_NOUT) : 0.0f;
   float part = 0.0f;  // this thread's part of the loss
   const int gq = lane >> 2, tq = lane & 3;

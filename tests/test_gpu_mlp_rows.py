@@ -58,3 +58,55 @@ def test_one_accumulator_adds_at_most_2048_rows(ctx):
     exact = big + rows - 1
     for got in (G["b4"][:280] / unit, G["W4"][:, :280] / (32.0 * unit)):
         assert np.abs(got - exact).max() <= 2047 + 8 * 200, np.abs(got - exact).max()
+
+
+def _known_sums(ctx, rows, seed, mean):
+    """A batch whose dL/dy are known to the bit (no weights, so y = 0): the
+    gradients, the loss, dL/dy and the targets."""
+    import torch
+
+    mlp = R.Mlp(ctx, seed=11)
+    mlp.set_params(np.zeros(R.MLP_NPARAM, dtype=np.float32))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    t = torch.zeros((rows, 288), device="cuda")
+    t[:, :280] = torch.randn((rows, 280), generator=g, device="cuda") + mean
+    x = torch.zeros((rows, 16), dtype=torch.bfloat16, device="cuda")
+    grad = torch.zeros(R.MLP_NPARAM, dtype=torch.float32, device="cuda")
+    loss = torch.zeros(1, dtype=torch.float32, device="cuda")
+    mlp.gradients(rows, x, t, grad, loss)
+    scale = torch.tensor(1.0, device="cuda") / (torch.tensor(float(rows), device="cuda") * torch.tensor(280.0, device="cuda"))
+    dy = ((2.0 * (0.0 - t[:, :280])) * scale).to(torch.bfloat16).to(torch.float32)
+    torch.cuda.synchronize()
+    mlp.close()
+    return M.unpack(grad.cpu().numpy().astype(np.float64)), loss.double().item(), dy, t[:, :280]
+
+
+def _rms(a, ref):
+    return float(np.sqrt(((a - ref) ** 2).sum() / (ref ** 2).sum()))
+
+
+@pytest.mark.parametrize("rows", [4096, 16384, 65536])
+def test_bias_sums_are_as_exact_as_sums_of_256_row_slabs(ctx, rows):
+    """Against fp64: the rms error over eight batches is at most a tenth above that
+    of fp32 sums over slabs of 256 rows (eight lanes of 32 rows, the lanes in turn)
+    added to the total one after another."""
+    err, ref = [], []
+    for seed in range(8):
+        G, _, dy, _ = _known_sums(ctx, rows, seed, float(seed & 1))
+        exact = dy.double().sum(0).cpu().numpy()
+        v = dy.reshape(rows // 256, 32, 8, 280)
+        lanes = v[:, 0].clone()
+        for i in range(1, 32):
+            lanes += v[:, i]
+        slabs = lanes[:, 0].clone()
+        for i in range(1, 8):
+            slabs += lanes[:, i]
+        slabs = slabs.cpu().numpy()
+        total = np.zeros(280, dtype=np.float32)
+        for s in slabs:
+            total = total + s
+        err.append(_rms(G["b4"][:280], exact))
+        ref.append(_rms(total.astype(np.float64), exact))
+    rms = lambda e: np.sqrt(np.mean(np.square(e)))
+    assert rms(err) <= 1.1 * rms(ref), (rms(err), rms(ref))
