@@ -47,7 +47,10 @@ struct GemmArgs {
   const bf16* Zin;
   float* colsum;  // EPI_ATOMIC: += the column sums of B over this block's rows
   const float *t, *w;
-  float* loss;    // EPI_LOSS: L = sum_j w_j (y_j - t_j)^2 / (rows * 280) over j < 280, added to loss where not NULL
+  // L = sum_j w_j (y_j - t_j)^2 / (rows * 280) over j < 280.  EPI_LOSS: each block's part of it into part, where not
+  // NULL; EPI_DSILU: the first block adds nparts of them up into loss, where not NULL
+  float *part, *loss;
+  int nparts;
 };
 
 constexpr int BM = 64, BN = 64, BK = 32, PAD = 8;
@@ -203,12 +206,27 @@ __global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g) {
           *reinterpret_cast<uint32_t*>(g.Z + (long long)m * g.ldz + n) = pack_bf16(v0 * dsilu(zf.x), v1 * dsilu(zf.y));
         }
       }
-  if (EPI == EPI_LOSS && g.loss) {
+  const bool last = EPI == EPI_DSILU && g.loss && blockIdx.x == 0 && blockIdx.y == 0;
+  if ((EPI == EPI_LOSS && g.part) || last) {
     __shared__ float red[4];
+    if (last) {  // eight sums a thread, as the parts' number is large where their rounding counts
+      float v[8] = {};
+      for (int i = tid; i < g.nparts; i += 8 * 128)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (i + 128 * k < g.nparts) v[k] += g.part[i + 128 * k];
+      part = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     if (lane == 0) red[warp] = part;
     __syncthreads();
-    if (tid == 0) atomicAdd(g.loss, (red[0] + red[1]) + (red[2] + red[3]));
+    if (tid == 0) {
+      const float s = (red[0] + red[1]) + (red[2] + red[3]);
+      if (last)
+        *g.loss = s;
+      else
+        g.part[blockIdx.y * gridDim.x + blockIdx.x] = s;
+    }
   }
 }
 
@@ -464,6 +482,9 @@ cudaError_t gb_mlp_norm_targets(long long rows, const float* d_tau, const float*
   return cudaGetLastError();
 }
 
+// parts of the loss: blocks of the output layer
+int gb_mlp_loss_parts(long long rows) { return (int)((rows + BM - 1) / BM) * ((GB_MLP_NOUTP + BN - 1) / BN); }
+
 cudaError_t gb_mlp_forward_backward(const MlpBuffers& b, long long rows, const bf16* d_x, const float* d_t,
                                     const float* d_w, float* d_grad, float* d_loss, bool keep_y, int num_sms,
                                     cudaStream_t st) {
@@ -492,7 +513,7 @@ cudaError_t gb_mlp_forward_backward(const MlpBuffers& b, long long rows, const b
   a.B = W[3]; a.ldb = O;
   a.C = keep_y ? b.y : nullptr; a.ldc = O; a.bias = Bs[3];
   a.Z = b.dy; a.ldz = O;
-  a.t = d_t; a.w = d_w; a.loss = d_loss;
+  a.t = d_t; a.w = d_w; a.part = d_loss ? b.part : nullptr;
   if ((e = gemm<false, false, EPI_LOSS>(a, 1, st)) != cudaSuccess) return e;
   // backward
   if ((e = cudaMemsetAsync(d_grad, 0, GB_MLP_NPARAM * sizeof(float), st)) != cudaSuccess) return e;
@@ -523,6 +544,7 @@ cudaError_t gb_mlp_forward_backward(const MlpBuffers& b, long long rows, const b
     a.A = dZ; a.lda = nout;
     a.B = W[l]; a.ldb = nout;  // W_l is [in][out]: as B^T with B[n][k] = W[n][k]
     a.Z = b.dz[l - 1]; a.ldz = H; a.Zin = b.z[l - 1];
+    if (l == 3) a.part = b.part, a.nparts = gb_mlp_loss_parts(rows), a.loss = d_loss;
     if ((e = gemm<false, true, EPI_DSILU>(a, 1, st)) != cudaSuccess) return e;
     dZ = b.dz[l - 1];
     nout = H;

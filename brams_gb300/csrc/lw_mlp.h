@@ -24,10 +24,12 @@ struct MlpBuffers {
   __nv_bfloat16* p16;
   __nv_bfloat16 *z[3], *act[3], *dz[3], *dy;
   float* y;
+  float* part;  // the output layer's blocks' parts of the loss (gb_mlp_loss_parts)
   long long rows;
 };
 
 size_t gb_mlp_infer_smem();
+int gb_mlp_loss_parts(long long rows);
 cudaError_t gb_mlp_features(const GbMlpGridIn& g, double grav, double avogad, float* d_feat, cudaStream_t st);
 cudaError_t gb_mlp_norm_inputs(long long rows, const float* d_feat, const GbMlpNorm& nm, __nv_bfloat16* d_x,
                                cudaStream_t st);

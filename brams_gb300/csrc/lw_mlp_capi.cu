@@ -45,8 +45,10 @@ void free_rows(MlpBuffers& b) {
   }
   cudaFree(b.dy);
   cudaFree(b.y);
+  cudaFree(b.part);
   b.dy = nullptr;
   b.y = nullptr;
+  b.part = nullptr;
   b.rows = 0;
 }
 
@@ -62,6 +64,7 @@ int ensure_rows(gb_lw_mlp* m, long long rows) {
   }
   ok = ok && cudaMalloc(&m->b.dy, rows * O * 2) == cudaSuccess;
   ok = ok && cudaMalloc(&m->b.y, rows * O * 4) == cudaSuccess;
+  ok = ok && cudaMalloc(&m->b.part, gb_mlp_loss_parts(rows) * sizeof(float)) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     free_rows(m->b);
@@ -376,7 +379,6 @@ int gb_lw_mlp_gradients(gb_lw_mlp* m, void* stream, int64_t rows, const void* d_
   int rc = ensure_rows(m, rows);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  if (d_loss) cudaMemsetAsync(d_loss, 0, 4, st);
   cudaError_t e = gb_mlp_forward_backward(m->b, rows, (const __nv_bfloat16*)d_x, d_t, m->d_w,
                                           d_grad ? d_grad : m->d_grad, d_loss, false, m->ctx->num_sms, st);
   return e == cudaSuccess ? GB_LW_OK : fail(m->ctx, e, "forward/backward");

@@ -110,3 +110,17 @@ def test_bias_sums_are_as_exact_as_sums_of_256_row_slabs(ctx, rows):
         ref.append(_rms(total.astype(np.float64), exact))
     rms = lambda e: np.sqrt(np.mean(np.square(e)))
     assert rms(err) <= 1.1 * rms(ref), (rms(err), rms(ref))
+
+
+@pytest.mark.parametrize("rows", [8, 72, 4104, 65536, 262144])
+def test_loss_of_large_batches(ctx, rows):
+    """Against fp64 from the same targets: 2^-24 a rounding, at most 16 sums of a
+    thread, 12 of a block and its parts' 20 + 10 (20,480 parts, eight sums of 128
+    threads) one after another, all of one sign; and the same in a second call."""
+    for seed in range(4):
+        _, loss, _, t = _known_sums(ctx, rows, seed, 0.5 * seed)
+        exact = (t.double() ** 2).sum().item() / (rows * 280.0)
+        # each term w e e scale: three roundings, and that of the scale
+        assert abs(loss - exact) <= (16 + 12 + 30 + 4) * 2.0 ** -24 * exact, (loss, exact)
+        assert abs(loss - exact) <= 6e-7 * exact, (loss, exact)  # ten roundings: what such sums are off in practice
+        assert _known_sums(ctx, rows, seed, 0.5 * seed)[1] == loss
