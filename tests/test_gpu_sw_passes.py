@@ -63,3 +63,21 @@ def test_fractions_that_are_no_numbers_stay_in_their_column(swctx):
     for k in ("swuflx", "swdflx", "swuflxc", "swdflxc"):
         assert np.isnan(out[k][4]).all(), k
         assert np.array_equal(out[k][keep], clean[k][keep]), k
+
+
+# the largest and the rms difference from the oracle (W m-2, K/day) on the columns below, with IEEE division throughout
+FP32_ERRORS = {"swuflx": (9.5e-4, 5.0e-5), "swdflx": (1.96e-3, 5.5e-5), "swhr": (4.6e-4, 2.7e-5),
+               "swuflxc": (3.6e-4, 2.0e-5), "swdflxc": (9.1e-4, 2.7e-5), "swhrc": (3.1e-4, 2.0e-5)}
+
+
+def test_fp32_errors_stay_what_they_were(swctx):
+    """A quarter above the errors first measured on these columns: far below the
+    parity tolerances, within which approximate divisions would pass."""
+    st = sw_state(ncol=512, nlay=45, seed=731, cloud_prob=0.5)
+    mc = sw_mcica(st, seed=7)
+    ref = pyoracle.rrtmg_sw(st, mc, icld=3, iaer=10, nthreads=8)
+    out = _solve(swctx, 32, st, mc, icld=3, iaer=10)
+    for k, (top, rms) in FP32_ERRORS.items():
+        d = out[k] - ref[k]
+        assert np.abs(d).max() <= 1.25 * top, (k, np.abs(d).max())
+        assert np.sqrt((d * d).mean()) <= 1.25 * rms, (k, np.sqrt((d * d).mean()))
