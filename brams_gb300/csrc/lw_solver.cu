@@ -503,7 +503,7 @@ __device__ __forceinline__ int liq_code(int liqflag, double rliq) {
 // a unit of a block: the threads that solve a unit's columns, with a barrier of their own
 struct Unit {
   int tid, nt, bar;
-  const float2* tt;  // rtrnmc's (exp_tbl, tfn_tbl), in shared memory
+  const float2* tt;  // rtrnmc's (exp_tbl, tfn_tbl), in shared memory (hand-over kernel: in global)
   __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory"); }
 };
 // the columns of a unit: n (1 or 2) neighbouring columns of one grid from
@@ -736,7 +736,7 @@ struct Passes {
   };
   const GasSrc& src;
   const RtLayer* L0;
-  const float2* tt;  // (exp_tbl, tfn_tbl), in shared memory
+  const float2* tt;  // (exp_tbl, tfn_tbl)
   const float* gc;
   float* part;
   float sd;
@@ -1590,14 +1590,17 @@ __global__ void __launch_bounds__(CELL_NT, 13) lw_cells_kernel(const __grid_cons
 
 // The columns handed over by the network's transfer kernel (B.fall), one per
 // block: taumol into the block's plane slot, then the transfer with each
-// layer's gas optics from the network or from taumol.
+// layer's gas optics from the network or from taumol.  rtrnmc's table is read
+// through L1: with a copy of it in shared memory a second block fitted up to 96
+// layers only (3,000 columns handed over: of 128 layers 3.74 ms, 2.45 ms with the
+// table in L1; 8,192 columns of 45 and of 60 layers 3.23 and 3.86 ms, 3.23 and 3.57 ms).
 __global__ void __launch_bounds__(RT_NT, LIST_PER_SM) lw_list_kernel(const __grid_constant__ LwBatch B,
                                                                      const float* __restrict__ T) {
   extern __shared__ __align__(16) char smem_raw[];
   const long long n = (long long)*B.nfall;
   if (blockIdx.x >= n) return;
-  const Unit U{(int)threadIdx.x, RT_NT, 1, stage_table(T, smem_raw)};
-  char* smem = smem_raw + TABLE_BYTES;
+  const Unit U{(int)threadIdx.x, RT_NT, 1, reinterpret_cast<const float2*>(T + c_T.tbl_tt)};
+  char* smem = smem_raw;
   const GasSmem gs = gas_carve(smem + ARGS_BYTES, B.nsmax);  // the transfer uses the same memory afterwards
   float* plane = B.plane + (long long)blockIdx.x * B.nsmax * GB_LW_PROW;
   for (long long i = blockIdx.x; i < n; i += gridDim.x) {
@@ -1679,7 +1682,7 @@ size_t block_smem(int nlay, int cpb, int units) {
   return gb::TABLE_BYTES + units * (gb::ARGS_BYTES + cpb * gb::rt_smem_bytes(nlay));
 }
 size_t list_smem(int nlay) {
-  return gb::TABLE_BYTES + gb::ARGS_BYTES + std::max(gb::rt_smem_bytes(nlay), gb::gas_smem_bytes(nlay));
+  return gb::ARGS_BYTES + std::max(gb::rt_smem_bytes(nlay), gb::gas_smem_bytes(nlay));
 }
 
 // Shared-memory carve-out for `per` resident blocks of `smem` bytes: just what
@@ -1742,7 +1745,7 @@ LwVariant gb_lw_variant(int v, bool lean) {
   return LwVariant{gb::RT_NT, info(v, lean).max_units};
 }
 
-size_t gb_lw_smem_bytes(int nlay) { return list_smem(nlay); }
+size_t gb_lw_smem_bytes(int nlay) { return std::max(block_smem(nlay, 1, 1), list_smem(nlay)); }
 
 cudaError_t gb_lw_set_tables(const GbTables& T) {
   const cudaError_t e = cudaMemcpyToSymbol(gb::c_T, &T, sizeof(GbTables));

@@ -163,3 +163,24 @@ def test_small_calls_equal_their_columns_in_a_large_one(ctx):
     got = g.outputs()
     for k in OUTS:
         assert np.array_equal(got[k], whole[k]), k
+
+
+@pytest.mark.parametrize("ncol,nlay", [(5, 96), (340, 97), (5, 207), (3, 256)])
+def test_deep_columns_off_the_network(own, ncol, nlay):
+    """Columns whose layers are all off the network have the plain path's bits, with
+    one and several columns per hand-over block."""
+    import torch
+
+    g = S.DeviceGrid(make_state(ProfileSpec(ncol=ncol, nlay=nlay, seed=5, t_noise=4.0)))
+    g.d["tauc"] = torch.full((nlay, ncol, 16), 3.0, dtype=torch.float64, device="cuda")
+    g.d["tlay"] += 200.0
+    ref = _solve(own, [g], [11])[0]
+    for k in OUTS:
+        g.d[k].zero_()
+    net = S.load(own)
+    net.batch([g.desc(seed0=11)])
+    torch.cuda.synchronize()
+    got = g.outputs()
+    for k in OUTS:
+        assert np.array_equal(got[k], ref[k]), k
+    net.close()
