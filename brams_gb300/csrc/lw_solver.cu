@@ -333,7 +333,9 @@ struct RtLayer {
   float4 rec[16];     // per band: Planck value of the layer, that of the level above it, aerosol optical
                       // depth, cloud optical depth (fused clouds; band clouds: secdiff(ib) * taucloud
                       // per cloud band ib, rtrn's odcld).  The record before layer 0 has the
-                      // Planck value of the lowest level.
+                      // Planck value of the lowest level.  In the first phase the fourth words of
+                      // the record before a layer hold the Planck-table row and fraction of the
+                      // level below it (words 0 and 1) and of the layer (2 and 3).
   int cldlay;         // 1: a cell of the layer has cldfmc == 1 (rtrnmc's icldlyr), or band
                       // clouds: cldfrac >= 1e-6; in the first phase: 1 where the layer is in
                       // the lower atmosphere
@@ -357,8 +359,7 @@ static_assert(offsetof(RtLayer, lcw) + sizeof(float4) - offsetof(RtLayer, cbits)
 struct RtSmem {
   RtHead* h;
   RtLayer* L;   // [-1 .. nl-1]; in the last phase: fp64 net fluxes [nl+1][2]
-  float4* prow; // [nl+1] first phase: the Planck-table row and fraction of tlev and tlay; then band
-                // clouds' fractions in fp64
+  double* cf;   // [nl] band clouds' fractions
   float* part;  // [RT_NW][nl+1][6] level sums per group of 32 g-points: dn, dn clear, up, up clear, dup/dT,
                 // dup clear/dT (global scratch)
   __device__ __forceinline__ unsigned* fbits(int lay) const { return L[lay].cbits + 5; }
@@ -370,7 +371,7 @@ __host__ __device__ inline size_t rt_layers_bytes(int nl) {
   return (size_t)(nl + 1) * sizeof(RtLayer);
 }
 __host__ __device__ inline size_t rt_smem_bytes(int nl) {
-  return sizeof(RtHead) + rt_layers_bytes(nl) + align16((size_t)(nl + 1) * 24);
+  return sizeof(RtHead) + rt_layers_bytes(nl) + align16((size_t)nl * sizeof(double));
 }
 // floats of a column's level sums
 __host__ __device__ inline size_t rt_part_floats(int nl) { return (size_t)RT_NW * (nl + 1) * 6; }
@@ -381,7 +382,7 @@ __device__ inline RtSmem rt_carve(char* p, int nl, float* part) {
   p += sizeof(RtHead);
   s.L = (RtLayer*)p + 1;
   p += rt_layers_bytes(nl);
-  s.prow = (float4*)p;
+  s.cf = (double*)p;
   s.part = part;
   return s;
 }
@@ -523,8 +524,6 @@ struct Cols {
   }
   __device__ __forceinline__ long long icol(int c) const { return col0 + c < last ? col0 + c : last; }
 };
-// fp64 fractions for the overlap factors, after the Planck-table rows of the first phase
-__device__ __forceinline__ double* band_cf64(const RtSmem& S, int nl) { return reinterpret_cast<double*>(S.prow + nl + 1); }
 
 // rtrnmr's maximum/random overlap factors (rrtmg_lw_rtrnmr.f90:345-514), by
 // one thread in fp64 from the layer fractions cf[0 .. nl-1]; lev is the
@@ -683,9 +682,10 @@ __device__ __forceinline__ void band_clouds(const LwArgs& a, const Unit& U, cons
     ov[0] = (float)cf;
 #pragma unroll
     for (int k = 1; k < 14; ++k) ov[k] = 0.0f;
-    band_cf64(S, nl)[lay] = cf;
+    S.cf[lay] = cf;
     if (lay == 0) S.h->iscal[2] = __ldg(a.ncbands + C.icol(c));
   }
+  U.sync();  // the records' fourth words are the Planck-table rows until here
   for (int it = tid; it < C.n * nl * 16; it += nt) {
     const int c = C.c(it), lay = C.rest(it) >> 4, ib = C.rest(it) & 15;
     const RtSmem S = C.S(c);
@@ -697,7 +697,7 @@ __device__ __forceinline__ void band_clouds(const LwArgs& a, const Unit& U, cons
     U.sync();
     if (tid % RT_CT == 0 && tid / RT_CT < C.n) {
       const RtSmem S = C.S(tid / RT_CT);
-      band_overlap(S, band_cf64(S, nl), nl);
+      band_overlap(S, S.cf, nl);
     }
   }
 }
@@ -1133,7 +1133,6 @@ __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const
     const int c = C.c(i), vw = C.rest(i);
     const RtSmem Sc = C.S(c);
     const long long ic = C.icol(c);
-    float4* prow = Sc.prow;
     float amttl = 0.0f, wvttl = 0.0f;
     int bad = 0;
     for (int lay = vw * 32 + lane; lay < nl; lay += RT_NT) {
@@ -1155,11 +1154,14 @@ __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const
       // Planck-table rows of the level below and of the layer (setcoef.f90:173-269)
       const int ind = clampi((int)(tz - 159.0f), 1, 180);
       const int il = clampi((int)(tavel - 159.0f), 1, 180);
-      prow[lay] = make_float4(__int_as_float(ind), tz - 159.0f - (float)ind, __int_as_float(il), tavel - 159.0f - (float)il);
+      float4* r = Sc.L[lay - 1].rec;
+      r[0].w = __int_as_float(ind), r[1].w = tz - 159.0f - (float)ind;
+      r[2].w = __int_as_float(il), r[3].w = tavel - 159.0f - (float)il;
       if (lay == nl - 1) {
         const float tt = (float)in2(a.tlev, a.ld, ic, nl);
         const int it = clampi((int)(tt - 159.0f), 1, 180);
-        prow[nl] = make_float4(__int_as_float(it), tt - 159.0f - (float)it, 0.0f, 0.0f);
+        float4* t = Sc.L[lay].rec;
+        t[0].w = __int_as_float(it), t[1].w = tt - 159.0f - (float)it;
       }
     }
 #pragma unroll
@@ -1216,13 +1218,12 @@ __device__ __forceinline__ bool rt_columns(const LwArgs& a, const Unit& U, const
   for (int i = tid; i < C.n * nl * 16; i += nt) {
     const int lay = C.rest(i) >> 4, ib = C.rest(i) & 15;
     const RtSmem Sc = C.S(C.c(i));
-    const float4* prow = Sc.prow;
     const float* tp = T + c_T.totplnk + ib * 181;
-    const float4 r0 = prow[lay], r1 = prow[lay + 1];
-    const int i0 = __float_as_int(r0.x), il = __float_as_int(r0.z), i1 = __float_as_int(r1.x);
-    const float pdn = tp[i0 - 1] + r0.y * (tp[i0] - tp[i0 - 1]);
-    const float pup = tp[i1 - 1] + r1.y * (tp[i1] - tp[i1 - 1]);
-    const float blay = tp[il - 1] + r0.w * (tp[il] - tp[il - 1]);
+    const float4 *r0 = Sc.L[lay - 1].rec, *r1 = Sc.L[lay].rec;  // their fourth words (see the phase above)
+    const int i0 = __float_as_int(r0[0].w), il = __float_as_int(r0[2].w), i1 = __float_as_int(r1[0].w);
+    const float pdn = tp[i0 - 1] + r0[1].w * (tp[i0] - tp[i0 - 1]);
+    const float pup = tp[i1 - 1] + r1[1].w * (tp[i1] - tp[i1 - 1]);
+    const float blay = tp[il - 1] + r0[3].w * (tp[il] - tp[il - 1]);
     const float taua = (float)__ldg(a.tauaer + C.icol(C.c(i)) + a.ld * (lay + (long long)nl * ib));
     float4& r = Sc.L[lay].rec[ib];  // its w is the clouds'
     *reinterpret_cast<float2*>(&r) = make_float2(blay, pup);
@@ -1754,7 +1755,8 @@ cudaError_t gb_lw_set_tables(const GbTables& T) {
 
 namespace {
 // Columns per unit: two, a thread per pair of g-points (80 a column), where
-// two columns fit in a block's shared memory, and where the batch has more
+// two columns fit in a block's shared memory (up to 229 layers; 3,000 columns of 227
+// layers with maximum/random overlap take 3.00 ms so, 4.69 ms one by one), and where the batch has more
 // columns than the device has SMs: of fewer, each gets an SM to itself.
 int cols_per_unit(int nlay, long long ncols) {
   return ncols > device_sms() && block_smem(nlay, 2, 1) <= device_smem() ? 2 : 1;

@@ -184,3 +184,19 @@ def test_deep_columns_off_the_network(own, ncol, nlay):
     for k in OUTS:
         assert np.array_equal(got[k], ref[k]), k
     net.close()
+
+
+@pytest.mark.parametrize("icld", [1, 2])
+@pytest.mark.parametrize("nlay", [208, 229, 230])
+def test_deep_band_clouds(own, nlay, icld):
+    """Two columns a unit up to 229 layers, one above: the first columns of a call of
+    155 against the oracle, and with the bits of a call of their own (a column a unit)."""
+    st = make_state(ProfileSpec(ncol=155, nlay=nlay, seed=17, t_noise=3.0, cloud_prob=0.6))
+    got = own.rrtmg_lw_nomcica(st, icld=icld)
+    few = {k: np.asfortranarray(v[:4]) if getattr(v, "shape", (0,))[:1] == (155,) else v for k, v in st.items()}
+    one = own.rrtmg_lw_nomcica(few, icld=icld)
+    ref = pyoracle.rrtmg_lw_nomcica(few, icld=icld)
+    for k in OUTS:
+        assert np.array_equal(got[k][:4], one[k]), k
+        tol = HR_TOL if k.startswith("hr") else 1e-3 if k.startswith("du") else FLUX_TOL
+        assert np.abs(one[k] - ref[k]).max() <= tol, k
