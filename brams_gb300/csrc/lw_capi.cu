@@ -234,7 +234,7 @@ int launch_one(gb_lw_context* ctx, const LwArgs& a, int k, cudaStream_t stream) 
 }
 
 // A batch with learned gas optics gets the context's hand-over list (room
-// for every column of the batch); other batches run the full kernel alone.
+// for every column of the batch); other batches have none.
 int attach_fall(gb_lw_context* ctx, LwBatch& b, cudaStream_t stream) {
   b.fall = nullptr;
   b.nfall = nullptr;

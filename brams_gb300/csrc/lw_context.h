@@ -37,8 +37,8 @@ struct gb_lw_context {
   std::vector<int> tuned_nlay;
   std::vector<gb_lw_tuning> last_tune;  // every candidate of the last autotune call
   GbScratch fdraws;  // McICA draws of fused-cloud grids in batched calls
-  // columns the learned-only kernel hands over to the full kernel, and their
-  // count (batches with learned gas optics)
+  // columns off the network, which the transfer kernel hands over to
+  // lw_list_kernel, and their count (batches with learned gas optics)
   GbScratch fall;
   unsigned* d_nfall = nullptr;
   // surrogate outputs of batched calls with a network: fp16 taug and Planck fractions, the layers' flags

@@ -319,9 +319,10 @@ __device__ void gas_column(const LwArgs& a, long long icol, const GasSmem& s, co
 }
 
 // ================================================================== transfer
-// Shared memory of one column: a fixed header, one 384-byte record per
-// layer (so that every per-layer access in the loops is base + layer * 384
-// + a constant), then the per-warp level sums.
+// Shared memory of one column: a fixed header, one 320-byte record per
+// layer (so that every per-layer access in the loops is base + layer * 320
+// + a constant), then band clouds' fractions.  The level sums are in global
+// scratch (LwBatch::part).
 constexpr int CELL_WORDS = GB_LW_CELL_WORDS;
 struct RtHead {
   float misc[64];         // secdiff[16], plankbnd[16], dplankbnd[16], semiss[16]

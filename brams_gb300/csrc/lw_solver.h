@@ -120,8 +120,9 @@ LwVariant gb_lw_variant(int v, bool lean = false);
 // the variant sized for the units (column blocks) that fit on an SM at this nlay
 int gb_lw_default_variant(int nlay);
 
-// shared memory one block needs at this nlay (one column's taumol or
-// transfer area); a launch is possible iff this fits in one block
+// the most shared memory a block needs at this nlay at least (a unit of one
+// column beside rtrnmc's table, or the hand-over kernel's taumol area); a
+// launch is possible iff this fits in one block
 size_t gb_lw_smem_bytes(int nlay);
 // column blocks of `variant` resident on the device at once for this nlay
 int gb_lw_slots(int nlay, int variant = 0, bool lean = false);

@@ -222,8 +222,9 @@ cudaError_t gb_lw_launch_taumol(const LwBatch& b, const float* d_tables, long lo
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   // where every block is resident at four an SM, the more loads a warp has in
-  // flight at 128 registers count, not the warps (64 columns of 38 layers: 84 us
-  // a call at 64 registers, 82 at 128)
+  // flight at 128 registers count, not the warps (calls of 1x38, 32x60, 64x38, 96x45
+  // and 128x38 columns and layers: 72.0, 97.6, 84.0, 92.3 and 84.2 us at 64 registers,
+  // 69.8, 94.6, 80.1, 90.3 and 82.1 at 128; 16x45 83.2 either way)
   if (nblk * 16LL <= 4LL * nsm)
     gb::lw_taumol_kernel<4><<<(unsigned)nblk * 16u, gb::TAU_NT, 0, stream>>>(b, d_tables, u0, nslot, nblk);
   else

@@ -20,8 +20,8 @@
  * on one stream, or order the streams (events).  Separate contexts run
  * concurrently.
  *
- * Graphs: the solvers' and the generators' *_device calls may be captured in a
- * CUDA graph of the caller's, once a call of the same size (or for
+ * Graphs: the solvers' and the generators' calls on device arrays may be
+ * captured in a CUDA graph of the caller's, once a call of the same size (for
  * gb_rrtmg_lw_device and gb_rrtmg_sw_device one of any size at the same nlay and
  * precision) has sized the scratch.  Scratch that a captured call uses is kept
  * until the context is freed, also when later calls outgrow it (what is kept so
