@@ -15,7 +15,9 @@
  *
  * Threading: a context may be used by one host thread at a time, and its
  * calls share the context's device scratch (taumol hand-over planes, McICA
- * draws, the shortwave kernel's slot records, grown on demand), so the
+ * draws, the shortwave kernel's slot records, grown with the columns of a
+ * call: up to about 1.5 GiB each for single-grid calls, batches, a batch graph
+ * and the shortwave, less where less is free), so the
  * *_device calls of one context must not overlap on the device: issue them
  * on one stream, or order the streams (events).  Separate contexts run
  * concurrently.
